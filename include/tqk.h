@@ -307,17 +307,22 @@ int tqk_block_unbuild(const tqk_block_desc* blocks, int nblocks, int max_batch,
                       const tqk_block_op* ops, void* stream);
 
 /* ---------------------------------------------------------------------------------
- * Staged low-qubit runs (plain method).  Upstream applies every gate as its own
- * permute + bmm pass (functional/gate_wrapper.py:96-140); tqk_staged_apply applies a run
- * of up to TQK_STAGED_MAX_OPS consecutive ops whose targets lie in the lowest tile_bits
- * bits of the amplitude index (wires n - tile_bits .. n - 1) in ONE pass: each CTA loads
- * contiguous tiles of 2^tile_bits amplitudes of a batch row into shared memory (128-bit
- * loads), applies the ops in order there, and writes the tiles back.  Controls, phase
- * wires and diagonal wires may be anywhere.  tqk_staged_adjoint is the matching reverse
- * step of the adjoint method on (psi, lam): ops in reverse order, psi <- U^H psi,
- * lam <- U^H lam, and for every op with a grad slot the operand cotangent
- * sum lam_in conj(psi_out) added in float64 (as tqk_adjoint_matrix / _phase / _diagonal
- * do for one op).  Ops whose uncompute is not U^H (non-unitary) must not be staged. */
+ * Shared passes of the plain method.  Upstream applies every gate as its own permute + bmm
+ * pass (functional/gate_wrapper.py:96-140); here a run of up to TQK_STAGED_MAX_OPS ops whose
+ * targets lie in one set of index bits (the tile bits) is ONE pass: each CTA takes tiles of
+ * a batch row (every value of the tile bits, the other bits fixed) on chip, applies the ops
+ * there and writes the tiles back.  Controls, phase wires and diagonal wires may be anywhere.
+ *   tqk_staged_apply / _adjoint  tiles of the lowest tile_bits bits (wires n - tile_bits ..
+ *                                n - 1), the ops in order; targets must lie there;
+ *   tqk_tiled_apply / _adjoint   tiles of the index bits in tile_mask: min(n,
+ *                                TQK_STAGED_MAX_TILE_BITS) of them, bit 0 included (the lowest
+ *                                four keep memory accesses to whole 128-byte lines), n >= 9;
+ *                                ops on disjoint wires may trade places.
+ * The adjoint entry points are the matching reverse step of the adjoint method on (psi,
+ * lam): ops in reverse order, psi <- U^H psi, lam <- U^H lam, and for every op with a grad
+ * slot the operand cotangent sum lam_in conj(psi_out) added in float64 (as
+ * tqk_adjoint_matrix / _phase / _diagonal do for one op).  Ops whose uncompute is not U^H
+ * (non-unitary) must not be in a run. */
 enum { TQK_S_DENSE1 = 0, TQK_S_X = 1, TQK_S_PHASE = 2, TQK_S_DIAG = 3 };
 enum { TQK_STAGED_MAX_OPS = 64, TQK_STAGED_MAX_TILE_BITS = 12, TQK_STAGED_MAX_WIRES = 8 };
 
@@ -336,12 +341,16 @@ typedef struct {
                           as the operand), or NULL */
 } tqk_staged_op; /* 72 bytes */
 
-/* status: device int; TQK_TIMEOUT is written there if a tile's bulk load (TMA) did not
- * complete within ~2 s (the pass then stops early). */
+/* status: device int; the staged passes write TQK_TIMEOUT there if a tile's bulk load (TMA)
+ * did not complete within ~2 s (the pass then stops early); the tiled passes leave it. */
 int tqk_staged_apply(void* state, int64_t bsz, int n, const tqk_staged_op* ops, int nops, int tile_bits,
                      int* status, void* stream);
 int tqk_staged_adjoint(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* ops, int nops,
                        int tile_bits, int* status, void* stream);
+int tqk_tiled_apply(void* state, int64_t bsz, int n, const tqk_staged_op* ops, int nops, uint64_t tile_mask,
+                    int* status, void* stream);
+int tqk_tiled_adjoint(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* ops, int nops,
+                      uint64_t tile_mask, int* status, void* stream);
 
 /* ---------------------------------------------------------------- persistent circuit batches
  * Many independent circuits of different sizes (n <= 24) in one launch.  tqk_batch_plan
@@ -449,8 +458,9 @@ enum {
   TQK_X_STAGED = 6,      /* staged run: `staged[0..nstaged)` in one shared-memory pass */
   TQK_X_BLOCK_TC = 7,    /* fused 6-wire block on the tensor cores: image / image_h */
   TQK_X_BLOCK_DENSE = 8, /* fused block on the CUDA cores: operand = U (complex64) */
-  TQK_X_BLOCK_ZERO = 9   /* fused 6-wire block applied to |0...0> (tqk_fused_zero_input, u = U):
+  TQK_X_BLOCK_ZERO = 9,  /* fused 6-wire block applied to |0...0> (tqk_fused_zero_input, u = U):
                             forward only; in the reverse table it must carry skip_reverse */
+  TQK_X_TILED = 10       /* staged run on the tile bits in `batch` (tqk_tiled_apply / _adjoint) */
 };
 typedef struct {
   int32_t kind;            /* TQK_X_* */
@@ -458,7 +468,7 @@ typedef struct {
   int32_t nctrl;
   int32_t ctrl_val;
   int32_t wires[TQK_MAX_OP_WIRES];
-  int64_t batch;           /* operand / block batch: 1 or bsz */
+  int64_t batch;           /* operand / block batch: 1 or bsz; TILED: the tile mask */
   const void* operand;     /* complex64 operand (DENSE, CTRL, PHASE, DIAG, BLOCK_DENSE) */
   const void* uncompute;   /* DENSE / CTRL: exact inverse for psi (non-unitary gates), or NULL */
   const void* image;       /* BLOCK_TC forward image (tqk_fused_prepare of U) */
@@ -472,7 +482,7 @@ typedef struct {
   double* mr;              /* BLOCK_TC reverse with grad: cross-term buffer [batch][128][128] float64,
                               zeroed; a stored-input step leaves M there (add it with
                               tqk_fused_cross_add_many), an in-place step adds M U to grad */
-  const tqk_staged_op* staged; /* STAGED: the run's ops (their grad slots are used in reverse) */
+  const tqk_staged_op* staged; /* STAGED, TILED: the run's ops (their grad slots are used in reverse) */
   int32_t nstaged;
   int32_t tile_bits;       /* STAGED */
   int32_t skip_reverse;    /* the reverse sweep stops before this op (it must be op 0: a first block

@@ -67,6 +67,8 @@ _SIGS = {
     "tqk_sample": (_int, [_vp, _i64, _int, _vp, _i64, _vp, _vp, _i64, _vp]),
     "tqk_staged_apply": (_int, [_vp, _i64, _int, _vp, _int, _int, _vp, _vp]),
     "tqk_staged_adjoint": (_int, [_vp, _vp, _i64, _int, _vp, _int, _int, _vp, _vp]),
+    "tqk_tiled_apply": (_int, [_vp, _i64, _int, _vp, _int, ctypes.c_uint64, _vp, _vp]),
+    "tqk_tiled_adjoint": (_int, [_vp, _vp, _i64, _int, _vp, _int, ctypes.c_uint64, _vp, _vp]),
     "tqk_batch_plan": (_int, [_vp, _int, _vp, _int, _vp, _vp, _int, _int]),
     "tqk_batch_items": (_i64, [_vp, _int, _vp, _vp, _i64]),
     "tqk_batch_run": (_int, [_vp, _int, _vp, _vp, _vp, _i64, _vp, _vp, _int, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
@@ -345,6 +347,7 @@ class StagedOp(ctypes.Structure):
 assert ctypes.sizeof(StagedOp) == 72
 S_DENSE1, S_X, S_PHASE, S_DIAG = 0, 1, 2, 3
 STAGED_MAX_OPS, STAGED_MAX_TILE_BITS, STAGED_MAX_WIRES = 64, 12, 8
+TILED_MIN_WIRES = 9
 
 
 # ------------------------------------------------------------------ compiled segments
@@ -360,7 +363,7 @@ class ExecOp(ctypes.Structure):
 
 
 assert ctypes.sizeof(ExecOp) == 184
-X_DENSE, X_CTRL, X_MCX, X_PHASE, X_DIAG, X_SWAP, X_STAGED, X_BLOCK_TC, X_BLOCK_DENSE, X_BLOCK_ZERO = range(10)
+X_DENSE, X_CTRL, X_MCX, X_PHASE, X_DIAG, X_SWAP, X_STAGED, X_BLOCK_TC, X_BLOCK_DENSE, X_BLOCK_ZERO, X_TILED = range(11)
 # Optional Python callables (exec record, after) the runners call around each op's
 # launches, per direction (bench.py installs one to time the dominant kernel's launches
 # inside a step).
@@ -401,15 +404,25 @@ def segment_backward(psi_end, lam, work, n, table, nops) -> int:
 
 
 def staged_apply(state, n, ops, tile_bits):
-    """Apply a run of ``StagedOp`` (sequence) in one shared-memory pass."""
+    """Apply a run of ``StagedOp`` (sequence) in one pass through tiles: ``tile_bits`` is the
+    number of lowest index bits a tile spans, or (above 64) the mask of its index bits."""
     arr = (StagedOp * max(1, len(ops)))(*ops)
+    if tile_bits > 64:
+        _check(load().tqk_tiled_apply(state.data_ptr(), state.shape[0], n, arr, len(ops), tile_bits,
+                                      status_word(state.device).data_ptr(), _stream(state)))
+        return
     _check(load().tqk_staged_apply(state.data_ptr(), state.shape[0], n, arr, len(ops), tile_bits,
                                    status_word(state.device).data_ptr(), _stream(state)))
 
 
 def staged_adjoint(psi, lam, n, ops, tile_bits):
-    """Reverse step of a staged run on (psi, lam); ops carry their cotangent slots."""
+    """Reverse step of a staged run on (psi, lam); ops carry their cotangent slots;
+    ``tile_bits`` as in ``staged_apply``."""
     arr = (StagedOp * max(1, len(ops)))(*ops)
+    if tile_bits > 64:
+        _check(load().tqk_tiled_adjoint(psi.data_ptr(), lam.data_ptr(), psi.shape[0], n, arr, len(ops), tile_bits,
+                                        status_word(psi.device).data_ptr(), _stream(psi)))
+        return
     _check(load().tqk_staged_adjoint(psi.data_ptr(), lam.data_ptr(), psi.shape[0], n, arr, len(ops), tile_bits,
                                      status_word(psi.device).data_ptr(), _stream(psi)))
 

@@ -44,6 +44,7 @@ int check_op(const tqk_exec_op& op, int i, const char* what) {
     return fail(TQK_BAD_SHAPE, "%s: op %d has nw=%d, nctrl=%d", what, i, op.nw, op.nctrl);
   switch (op.kind) {
     case TQK_X_STAGED:
+    case TQK_X_TILED:
       if (op.staged == nullptr || op.nstaged <= 0) return fail(TQK_BAD_POINTER, "%s: op %d: empty staged run", what, i);
       return TQK_OK;
     case TQK_X_BLOCK_TC:
@@ -115,6 +116,9 @@ extern "C" int tqk_segment_forward(void* state, int64_t bsz, int n, const tqk_ex
         break;
       case TQK_X_STAGED:
         rc = tqk_staged_apply(cur, bsz, n, op.staged, op.nstaged, op.tile_bits, status, stream);
+        break;
+      case TQK_X_TILED:
+        rc = tqk_tiled_apply(cur, bsz, n, op.staged, op.nstaged, static_cast<uint64_t>(op.batch), status, stream);
         break;
       case TQK_X_BLOCK_TC:
         if (op.out != nullptr) {
@@ -209,6 +213,10 @@ extern "C" int tqk_segment_backward(const void* psi_end, void* lam, void* work, 
         break;
       case TQK_X_STAGED:
         rc = tqk_staged_adjoint(p, lam, bsz, n, op.staged, op.nstaged, op.tile_bits, status, stream);
+        break;
+      case TQK_X_TILED:
+        rc = tqk_tiled_adjoint(p, lam, bsz, n, op.staged, op.nstaged, static_cast<uint64_t>(op.batch), status,
+                               stream);
         break;
       case TQK_X_BLOCK_TC: {
         double* mr = op.grad ? op.mr : nullptr;

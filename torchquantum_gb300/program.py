@@ -233,7 +233,7 @@ class Segment:
             self.exec_ops = exec_ops
             self._build_blocks()
         else:
-            self.exec_ops = stage_runs(ops, n) if getattr(qdev, "stage_low", True) else ops
+            self.exec_ops = tile_runs(ops, n, self.bsz) if getattr(qdev, "stage_low", True) else ops
         # ---- differentiable inputs
         self.bases: Dict[int, tuple] = {}
         for g in natives:
@@ -619,7 +619,11 @@ def _staged_record(run, descs, keep: list) -> "_lib.ExecOp":
     arr = (_lib.StagedOp * len(descs))(*descs)
     keep.append(arr)  # alive until the runner returns (it reads the table on the host)
     r = _lib.ExecOp()
-    r.kind, r.staged, r.nstaged, r.tile_bits = _lib.X_STAGED, ctypes.addressof(arr), len(descs), run.tile_bits
+    r.staged, r.nstaged = ctypes.addressof(arr), len(descs)
+    if run.tile_bits > 64:
+        r.kind, r.batch = _lib.X_TILED, run.tile_bits
+    else:
+        r.kind, r.tile_bits = _lib.X_STAGED, run.tile_bits
     return r
 
 
@@ -659,10 +663,11 @@ def _new_state(like: torch.Tensor) -> Optional[torch.Tensor]:
         return None
 
 
-# ---------------------------------------------------------------- staged low-qubit runs
+# ---------------------------------------------------------------- staged runs
 class StagedRun:
-    """Consecutive ops whose targets lie in the lowest ``tile_bits`` index bits, applied
-    in one shared-memory pass (``tqk_staged_apply``) and reversed in one adjoint pass."""
+    """Ops applied in one pass through tiles held on chip and reversed in one adjoint pass.
+    ``tile_bits``: the number of lowest index bits a tile spans (``tqk_staged_apply``), or,
+    above 64, the mask of its index bits (``tqk_tiled_apply``)."""
 
     def __init__(self, ops, tile_bits):
         self.ops = ops
@@ -764,6 +769,91 @@ def stage_runs(ops, n: int, min_run: int = 2):
             out.append(op)
     close()
     return out
+
+
+# A tile pass moves the state once (2 S bytes forward, 4 S in reverse).  On a state larger
+# than this its ops must together cost at least that on their own kernels to share a pass;
+# a smaller state stays in L2, where launches cost more than bytes.
+TILE_L2_BYTES = 32 << 20
+# Rows of at most 2^12 amplitudes are one tile either way.  Up to 2^21 amplitudes in all the
+# run keeps the op-by-op kernels of staged.cu, whose order of operations its results are
+# known by: there a step is host bound (n = 10, bsz = 256, 100 gates: 162 us of 3.3 ms in
+# these kernels, 128 us in the tiled ones).  Above, the tiled kernels' rate counts.
+TILE_SHORT_ROW_AMPS = 1 << 22
+_TILE_PLANS: dict = {}
+
+
+def _pass_share(op) -> float:
+    """Share of a pass over the state (2 S forward, 4 S reverse) of an op's own kernel."""
+    if op.kind in (engine.KIND_CTRL, engine.KIND_X):
+        return 0.5 ** len(op.controls)
+    if op.kind == engine.KIND_PHASE:
+        return 0.5 ** len(op.wires)
+    return 1.0
+
+
+def plan_tiles(ops, n: int, small: bool) -> List[tuple]:
+    """Cut the ops into passes: (op indices, tile mask), mask 0 for an op on its own kernel.
+
+    A pass starts from the lowest four index bits (whole 128-byte lines) and walks the
+    pending ops in order: an op joins when no wire of it was touched by an op left out and
+    its target (if any) is or fits among the tile's bits; ops on disjoint wires commute, so
+    the passes apply an equivalent order.  Free bits are filled from the lowest."""
+    tb = min(n, _lib.STAGED_MAX_TILE_BITS)
+    pending, out = list(range(len(ops))), []
+    while pending:
+        mask, free, blocked = 15, tb - 4, 0
+        take, rest = [], []
+        for i in pending:
+            op = ops[i]
+            wires = 0
+            for w in op.wires:
+                wires |= 1 << (n - 1 - w)
+            if not (wires & blocked) and len(take) < _lib.STAGED_MAX_OPS and stageable(op, n, n):
+                tgt = 0
+                if op.kind not in (engine.KIND_PHASE, engine.KIND_DIAG):
+                    tgt = 1 << (n - 1 - (op.targets[0] if op.kind != engine.KIND_DENSE else op.wires[0]))
+                if not tgt & ~mask:
+                    take.append(i)
+                    continue
+                if free:
+                    mask |= tgt
+                    free -= 1
+                    take.append(i)
+                    continue
+            blocked |= wires if wires else (1 << n) - 1
+            rest.append(i)
+        if not take:  # the first op is not one a tile pass can hold
+            out.append(([pending[0]], 0))
+            pending = pending[1:]
+            continue
+        if len(take) < 2 or not (small or sum(_pass_share(ops[i]) for i in take) >= 1.0):
+            out.extend(([i], 0) for i in take)
+        else:
+            for b in range(n):
+                if free and not (mask >> b) & 1:
+                    mask |= 1 << b
+                    free -= 1
+            out.append((take, mask))
+        pending = rest
+    return out
+
+
+def tile_runs(ops, n: int, bsz: int):
+    """The plain method's execution list: ``StagedRun`` passes and ops on their own kernels.
+    Short rows take ``stage_runs``; the others are cut by ``plan_tiles``, memoised on the
+    circuit's structure."""
+    if n < _lib.TILED_MIN_WIRES or (n <= _lib.STAGED_MAX_TILE_BITS and (bsz << n) < TILE_SHORT_ROW_AMPS):
+        return stage_runs(ops, n)
+    small = (bsz << (n + 3)) <= TILE_L2_BYTES
+    key = (n, small, tuple((op.kind, tuple(op.wires), len(op.controls), stageable(op, n, n)) for op in ops))
+    plan = _TILE_PLANS.get(key)
+    if plan is None:
+        if len(_TILE_PLANS) > 256:
+            _TILE_PLANS.clear()
+        plan = plan_tiles(ops, n, small)
+        _TILE_PLANS[key] = plan
+    return [StagedRun([ops[i] for i in idx], mask) if mask else ops[idx[0]] for idx, mask in plan]
 
 
 def _operand_shape(r: NativeGate, sz: int):
