@@ -10,10 +10,13 @@ This module depends only on ctypes, torch and the C ABI (``include/tqk.h``), lik
 binding a maintainer would add to upstream.  It keeps upstream's semantics
 (``gate_wrapper.py:96-140``): out of place, the input state is never written, and the
 result is differentiable with respect to both ``state`` and ``mat`` through a
-``torch.autograd.Function`` whose backward is one adjoint step of the engine
-(``tqk_adjoint_matrix``): the state cotangent ``U^H g`` and the matrix cotangent
-``sum g x^H`` over the batch (per row for a per-row matrix), as torch's own ``bmm``
-backward gives them.
+``torch.autograd.Function`` whose backward is one adjoint step of the engine against the
+saved input: the state cotangent ``U^H g`` and the matrix cotangent ``sum g x^H`` over the
+batch (per row for a per-row matrix), as torch's own ``bmm`` backward gives them.
+
+Gates on one or two wires read the caller's state and write the result (``tqk_apply_matrix_to``,
+``tqk_adjoint_matrix_stored``: 2 and 3 transfers of the state); wider ones run the in-place
+kernels on copies.
 """
 from __future__ import annotations
 
@@ -39,6 +42,10 @@ def _load():
         lib.tqk_apply_matrix.argtypes = [vp, i64, c_int, i32p, c_int, vp, i64, vp]
         lib.tqk_adjoint_matrix.restype = c_int
         lib.tqk_adjoint_matrix.argtypes = [vp, vp, i64, c_int, i32p, c_int, vp, i64, vp, vp, vp]
+        lib.tqk_apply_matrix_to.restype = c_int
+        lib.tqk_apply_matrix_to.argtypes = [vp, vp, i64, c_int, i32p, c_int, vp, i64, vp]
+        lib.tqk_adjoint_matrix_stored.restype = c_int
+        lib.tqk_adjoint_matrix_stored.argtypes = [vp, vp, vp, i64, c_int, i32p, c_int, vp, i64, vp, vp]
         _lib = lib
     return _lib
 
@@ -52,6 +59,21 @@ def _wires(wires) -> List[int]:
     return [int(wires)] if isinstance(wires, int) else [int(w) for w in wires]
 
 
+def _readable(t: torch.Tensor, bsz: int) -> torch.Tensor:
+    """``t``'s values as bsz rows of complex64 that a kernel can read: no lazy conjugation or
+    negation, contiguous, 16-byte aligned (``t`` itself where it already is)."""
+    if t.dtype is torch.complex64 and t.is_contiguous() and not t.is_conj() and not t.is_neg():
+        x = t
+    else:
+        x = t.detach().reshape(bsz, -1).to(torch.complex64).resolve_conj().resolve_neg().contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
+def _out_of_place(x: torch.Tensor, bsz: int, n: int, k: int) -> bool:
+    """Whether the kernels that read one state and write another take this gate."""
+    return k <= 2 and x.numel() == bsz << n
+
+
 class _ApplyUnitary(torch.autograd.Function):
     @staticmethod
     def forward(ctx, state: torch.Tensor, mat: torch.Tensor, wires: List[int]):
@@ -59,13 +81,18 @@ class _ApplyUnitary(torch.autograd.Function):
         bsz, n, k = state.shape[0], state.dim() - 1, len(wires)
         if state.device.type != "cuda":
             raise ValueError("apply_unitary_bmm (libtqk): the state must be a CUDA tensor")
-        x = state.detach().reshape(bsz, -1).to(torch.complex64).contiguous()
+        x = _readable(state, bsz)
         m = mat.detach().to(x.device, torch.complex64)
         m3 = (m if m.dim() == 3 else m.unsqueeze(0)).resolve_conj().resolve_neg().contiguous()
-        out = x.clone()
         w = (ctypes.c_int32 * k)(*wires)
         stream = torch.cuda.current_stream(x.device).cuda_stream
-        _check(lib.tqk_apply_matrix(out.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0], stream))
+        if _out_of_place(x, bsz, n, k):
+            out = torch.empty_like(x)
+            _check(lib.tqk_apply_matrix_to(x.data_ptr(), out.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0],
+                                           stream))
+        else:
+            out = x.clone()
+            _check(lib.tqk_apply_matrix(out.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0], stream))
         ctx.save_for_backward(x, m3)
         ctx.wires, ctx.shape = wires, state.shape
         ctx.mat_shape, ctx.mat_dtype, ctx.mat_device = mat.shape, mat.dtype, mat.device
@@ -75,20 +102,27 @@ class _ApplyUnitary(torch.autograd.Function):
     def backward(ctx, grad_out: torch.Tensor):
         lib = _load()
         x, m3 = ctx.saved_tensors
-        bsz, n, k = x.shape[0], len(ctx.shape) - 1, len(ctx.wires)
+        bsz, n, k = ctx.shape[0], len(ctx.shape) - 1, len(ctx.wires)
         d = 1 << k
-        # one adjoint step: lam <- U^H g, cotangent of U += g x^H; the stored input x is
-        # recovered with an identity "uncompute" (exact, also for matrices that are not
-        # unitary), on a copy so the saved tensor is never written
-        psi = x.clone()
-        lam = grad_out.reshape(bsz, -1).to(torch.complex64).resolve_conj().resolve_neg().contiguous().clone()
-        eye = torch.eye(d, dtype=torch.complex64, device=x.device).expand(m3.shape[0], d, d).contiguous()
         need_mat = ctx.needs_input_grad[1]
         grad = torch.zeros(m3.shape[0] * d * d * 2, dtype=torch.float64, device=x.device) if need_mat else None
         w = (ctypes.c_int32 * k)(*ctx.wires)
         stream = torch.cuda.current_stream(x.device).cuda_stream
-        _check(lib.tqk_adjoint_matrix(psi.data_ptr(), lam.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0],
-                                      eye.data_ptr(), None if grad is None else grad.data_ptr(), stream))
+        if _out_of_place(x, bsz, n, k):
+            g = _readable(grad_out, bsz)
+            lam = torch.empty_like(g)
+            _check(lib.tqk_adjoint_matrix_stored(x.data_ptr(), g.data_ptr(), lam.data_ptr(), bsz, n, w, k,
+                                                 m3.data_ptr(), m3.shape[0], None if grad is None else grad.data_ptr(),
+                                                 stream))
+        else:
+            # the in-place step: lam <- U^H g, cotangent of U += g x^H; the stored input x is
+            # recovered with an identity "uncompute" (exact, also for matrices that are not
+            # unitary), on a copy so the saved tensor is never written
+            psi = x.clone()
+            lam = grad_out.reshape(bsz, -1).to(torch.complex64).resolve_conj().resolve_neg().contiguous().clone()
+            eye = torch.eye(d, dtype=torch.complex64, device=x.device).expand(m3.shape[0], d, d).contiguous()
+            _check(lib.tqk_adjoint_matrix(psi.data_ptr(), lam.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0],
+                                          eye.data_ptr(), None if grad is None else grad.data_ptr(), stream))
         g_state = lam.view(ctx.shape) if ctx.needs_input_grad[0] else None
         g_mat = None
         if need_mat:

@@ -21,6 +21,7 @@ enum { MODE_SCL = 0, MODE_VEC = 1, MODE_LOW = 2 };
 // ------------------------------------------------------------------ dense 1/2-target
 template <int D>
 struct DenseParams {
+  const float2* in;       // forward: the state read (== state: in place)
   float2* state;
   float2* lam;            // adjoint only
   int n;
@@ -134,14 +135,105 @@ __global__ void __launch_bounds__(256) k_dense(const DenseParams<D> p) {
   if (t >= pairs) return;
   float2 M[D][D];
   load_mat<D>(p.mat + b * p.mat_stride, M);
-  float2* row = p.state + (b << p.n);
   const int64_t g0 = t * 2;
   const bool two = g0 + 1 < p.groups;
   float2 a[2][D], y[2][D];
-  load_groups<D, MODE>(row, p, g0, two, a);
+  load_groups<D, MODE>(p.in + (b << p.n), p, g0, two, a);
 #pragma unroll
   for (int j = 0; j < 2; ++j) matvec<D>(M, a[j], y[j]);
-  store_groups<D, MODE>(row, p, g0, two, y);
+  store_groups<D, MODE>(p.state + (b << p.n), p, g0, two, y);
+}
+
+// Reverse step against the gate's stored input x (a caller that kept it, as autograd does):
+// out = U^H g and, with GRAD, grad += g x^H.  3 S bytes, where uncomputing x in place takes
+// 4 S and, on saved tensors that may not be written, two copies more.
+// Memory bound where the loads in flight cover the latency: D = 4 keeps 32 matrix values and
+// 32 sums in registers, so 128 threads and 4 CTAs per SM instead of 256 and 1.  A thread takes
+// up to kStoredIter pairs of groups (stride: the grid), so that the block's reduction is paid
+// once for all of them while its float32 sums stay short.  n = 21, bsz = 8 (3 S = 403 MB): 62 us
+// for one wire, 74 us for two, where the in-place step took 106 and 213 us beside three copies
+// of 42 us.
+template <int D>
+struct StoredParams {
+  DenseParams<D> d;       // ins, off, pair, mat, grad, groups
+  const float2* x;
+  const float2* g;
+  float2* out;
+};
+
+// Sum NV = 8 or 32 values over the warp by halves: NV - 1 exchanges (then plain ones for
+// NV = 8) instead of 5 NV.  Lane L ends with the sum of value L * NV / 32.
+template <int NV>
+__device__ __forceinline__ float warp_sum(float (&v)[NV], int lane) {
+#pragma unroll
+  for (int h = NV / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  float s = v[0];
+#pragma unroll
+  for (int o = 16 / NV; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+template <int D>
+constexpr int kStoredThreads = D == 4 ? 128 : 256;
+constexpr int kStoredIter = 4;
+
+template <int D, int MODE, bool GRAD>
+__global__ void __launch_bounds__(kStoredThreads<D>, D == 4 ? 4 : 3)
+    k_dense_stored(const __grid_constant__ StoredParams<D> q) {
+  const DenseParams<D>& p = q.d;
+  const int64_t b = blockIdx.y;
+  const int64_t pairs = (p.groups + 1) >> 1;
+  float acc[GRAD ? 2 * D * D : 1];
+#pragma unroll
+  for (int i = 0; i < (GRAD ? 2 * D * D : 1); ++i) acc[i] = 0.f;
+  float2 M[D][D];
+  load_mat<D>(p.mat + b * p.mat_stride, M);
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < pairs; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t g0 = t * 2;
+    const bool two = g0 + 1 < p.groups;
+    float2 a[2][D], l[2][D], z[2][D];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int r = 0; r < D; ++r) a[j][r] = l[j][r] = make_float2(0.f, 0.f);
+    load_groups<D, MODE>(q.g + (b << p.n), p, g0, two, l);
+    if (GRAD) load_groups<D, MODE>(q.x + (b << p.n), p, g0, two, a);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) matvec_h<D>(M, l[j], z[j]);
+    store_groups<D, MODE>(q.out + (b << p.n), p, g0, two, z);
+    if (GRAD) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int r = 0; r < D; ++r)
+#pragma unroll
+          for (int c = 0; c < D; ++c) {
+            const float2 v = cfma_bconj(l[j][r], a[j][c], make_float2(acc[2 * (r * D + c)], acc[2 * (r * D + c) + 1]));
+            acc[2 * (r * D + c)] = v.x;
+            acc[2 * (r * D + c) + 1] = v.y;
+          }
+    }
+  }
+  if constexpr (GRAD) {
+    constexpr int NV = 2 * D * D;
+    __shared__ float red[kStoredThreads<D> / 32][NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float s = warp_sum<NV>(acc, lane);
+    if (lane % (32 / NV) == 0) red[warp][lane * NV / 32] = s;
+    __syncthreads();
+    if (threadIdx.x < NV) {
+      double t = 0.0;
+      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += static_cast<double>(red[w][threadIdx.x]);
+      atomicAdd(p.grad + b * p.grad_stride + threadIdx.x, t);
+    }
+  }
 }
 
 // Adjoint step: psi <- U^H psi (or U^-1 psi when INV), lam <- U^H lam,
@@ -683,11 +775,12 @@ void launch_dense_adj(const DenseParams<D>& p, int mode, bool grad, dim3 grid, i
 }
 
 template <int D>
-int launch_dense(const GateSetup& s, float2* state, float2* lam, const float2* mat, int64_t mat_batch,
+int launch_dense(const GateSetup& s, const float2* in, float2* state, float2* lam, const float2* mat, int64_t mat_batch,
                  const float2* uinv, double* grad, bool adjoint, cudaStream_t st) {
   DenseParams<D> p;
   int mode;
   fill_dense<D>(p, s, mode);
+  p.in = in;
   p.state = state;
   p.lam = lam;
   p.mat = mat;
@@ -708,6 +801,38 @@ int launch_dense(const GateSetup& s, float2* state, float2* lam, const float2* m
     launch_dense_adj<D, false>(p, mode, grad != nullptr, grid, threads, st);
   }
   return launch_status(adjoint ? "adjoint dense gate" : "dense gate");
+}
+
+template <int D>
+int launch_dense_stored(const GateSetup& s, const float2* x, const float2* g, float2* out, const float2* mat,
+                        int64_t mat_batch, double* grad, cudaStream_t st) {
+  StoredParams<D> q;
+  int mode;
+  fill_dense<D>(q.d, s, mode);
+  q.d.in = q.d.uinv = nullptr;
+  q.d.state = q.d.lam = nullptr;
+  q.d.mat = mat;
+  q.d.mat_stride = mat_batch > 1 ? D * D : 0;
+  q.d.grad = grad;
+  q.d.grad_stride = mat_batch > 1 ? 2 * D * D : 0;
+  q.x = x;
+  q.g = g;
+  q.out = out;
+  const int64_t work = (q.d.groups + 1) >> 1;
+  const int threads = threads_for(work) < kStoredThreads<D> ? threads_for(work) : kStoredThreads<D>;
+  dim3 grid = grid_for(work, threads, s.bsz);
+  // more than one pair per thread once the grid still fills every SM eight times over
+  int64_t iter = static_cast<int64_t>(grid.x) * s.bsz / (8 * 152);
+  iter = iter < 1 ? 1 : (iter > kStoredIter ? kStoredIter : iter);
+  grid.x = static_cast<unsigned>((grid.x + iter - 1) / iter);
+  if (mode == MODE_VEC) {
+    if (grad) k_dense_stored<D, MODE_VEC, true><<<grid, threads, 0, st>>>(q);
+    else k_dense_stored<D, MODE_VEC, false><<<grid, threads, 0, st>>>(q);
+  } else {
+    if (grad) k_dense_stored<D, MODE_LOW, true><<<grid, threads, 0, st>>>(q);
+    else k_dense_stored<D, MODE_LOW, false><<<grid, threads, 0, st>>>(q);
+  }
+  return launch_status("stored reverse step of a dense gate");
 }
 
 int launch_dense_k(const GateSetup& s, float2* state, float2* lam, const float2* mat, const float2* uinv,
@@ -781,8 +906,8 @@ int dense_entry(void* state, void* lam, int64_t bsz, int n, const int32_t* contr
   auto* pl = static_cast<float2*>(lam);
   auto* pm = static_cast<const float2*>(mat);
   auto* pi = static_cast<const float2*>(uinv);
-  if (kt == 1) return launch_dense<2>(s, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
-  if (kt == 2) return launch_dense<4>(s, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
+  if (kt == 1) return launch_dense<2>(s, ps, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
+  if (kt == 2) return launch_dense<4>(s, ps, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
   if (nc > 0) return fail(TQK_UNSUPPORTED, "%s: controlled gates take 1 or 2 targets", what);
   return launch_dense_k(s, ps, pl, pm, pi, mat_batch, grad, adjoint, st);
 }
@@ -878,6 +1003,47 @@ extern "C" int tqk_apply_matrix(void* state, int64_t bsz, int n, const int32_t* 
                                 int64_t mat_batch, void* stream) {
   return dense_entry(state, nullptr, bsz, n, nullptr, 0, wires, k, mat, mat_batch, nullptr, nullptr, false, stream,
                      "tqk_apply_matrix");
+}
+
+extern "C" int tqk_apply_matrix_to(const void* in, void* out, int64_t bsz, int n, const int32_t* wires, int k,
+                                   const void* mat, int64_t mat_batch, void* stream) {
+  const char* what = "tqk_apply_matrix_to";
+  int rc = check_state(in, bsz, n, what);
+  if (rc) return rc;
+  if ((rc = check_state(out, bsz, n, what))) return rc;
+  if ((rc = check_batch(mat_batch, bsz, what))) return rc;
+  if (mat == nullptr) return fail(TQK_BAD_POINTER, "%s: null matrix", what);
+  if (in == out) return fail(TQK_BAD_POINTER, "%s: out must not alias in (tqk_apply_matrix works in place)", what);
+  if (k < 1 || k > 2) return fail(TQK_TOO_MANY_QUBITS, "%s: k=%d unsupported (1 or 2)", what, k);
+  GateSetup s;
+  if ((rc = setup_targets(s, n, bsz, wires, k, nullptr, 0, what))) return rc;
+  auto* pi = static_cast<const float2*>(in);
+  auto* po = static_cast<float2*>(out);
+  auto* pm = static_cast<const float2*>(mat);
+  if (k == 1) return launch_dense<2>(s, pi, po, nullptr, pm, mat_batch, nullptr, nullptr, false, as_stream(stream));
+  return launch_dense<4>(s, pi, po, nullptr, pm, mat_batch, nullptr, nullptr, false, as_stream(stream));
+}
+
+extern "C" int tqk_adjoint_matrix_stored(const void* x, const void* g, void* out, int64_t bsz, int n,
+                                         const int32_t* wires, int k, const void* mat, int64_t mat_batch,
+                                         double* grad, void* stream) {
+  const char* what = "tqk_adjoint_matrix_stored";
+  int rc = check_state(g, bsz, n, what);
+  if (rc) return rc;
+  if ((rc = check_state(out, bsz, n, what))) return rc;
+  if (grad != nullptr && (rc = check_state(x, bsz, n, what))) return rc;
+  if ((rc = check_batch(mat_batch, bsz, what))) return rc;
+  if (mat == nullptr) return fail(TQK_BAD_POINTER, "%s: null matrix", what);
+  if (out == x || out == g) return fail(TQK_BAD_POINTER, "%s: out must not alias x or g", what);
+  if (k < 1 || k > 2) return fail(TQK_TOO_MANY_QUBITS, "%s: k=%d unsupported (1 or 2)", what, k);
+  GateSetup s;
+  if ((rc = setup_targets(s, n, bsz, wires, k, nullptr, 0, what))) return rc;
+  auto* px = static_cast<const float2*>(x);
+  auto* pg = static_cast<const float2*>(g);
+  auto* po = static_cast<float2*>(out);
+  auto* pm = static_cast<const float2*>(mat);
+  if (k == 1) return launch_dense_stored<2>(s, px, pg, po, pm, mat_batch, grad, as_stream(stream));
+  return launch_dense_stored<4>(s, px, pg, po, pm, mat_batch, grad, as_stream(stream));
 }
 
 extern "C" int tqk_apply_controlled(void* state, int64_t bsz, int n, const int32_t* controls, int nc,
