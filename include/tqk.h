@@ -150,7 +150,7 @@ int tqk_pauli_apply_sum(const void* state, int64_t bsz, int n, const uint64_t* x
 int tqk_adjoint_matrix(void* psi, void* lam, int64_t bsz, int n, const int32_t* wires, int k,
                        const void* mat, int64_t mat_batch, const void* uncompute, double* grad,
                        void* stream);
-/* The same for callers that keep a gate's input (1 or 2 wires, no controls):
+/* The same for callers that keep a gate's input (1 to 6 wires, no controls):
  * tqk_apply_matrix_to writes U in to out (in is not written; out must not alias it), and
  * tqk_adjoint_matrix_stored writes U^H g to out and, when grad is not NULL, adds
  * sum g x^H to it (x: the gate's input, read only; may be NULL without grad). */

@@ -65,13 +65,13 @@ def test_entry_points_refuse_aliases_and_wide_gates():
     from torchquantum_gb300 import _lib, binding
 
     lib = binding._load()
-    s = torch.zeros(1, 16, dtype=torch.complex64, device="cuda")
-    m = torch.eye(8, dtype=torch.complex64, device="cuda")
-    w = (ctypes.c_int32 * 3)(0, 1, 2)
+    s = torch.zeros(1, 256, dtype=torch.complex64, device="cuda")
+    m = torch.eye(128, dtype=torch.complex64, device="cuda")
+    w = (ctypes.c_int32 * 7)(*range(7))
     st = torch.cuda.current_stream().cuda_stream
     p, o = s.data_ptr(), torch.zeros_like(s)
-    assert lib.tqk_apply_matrix_to(p, p, 1, 4, w, 1, m.data_ptr(), 1, st) != 0
-    assert lib.tqk_apply_matrix_to(p, o.data_ptr(), 1, 4, w, 3, m.data_ptr(), 1, st) != 0
-    assert lib.tqk_adjoint_matrix_stored(p, p, p, 1, 4, w, 1, m.data_ptr(), 1, None, st) != 0
-    assert lib.tqk_adjoint_matrix_stored(p, p, o.data_ptr(), 1, 4, w, 3, m.data_ptr(), 1, None, st) != 0
+    assert lib.tqk_apply_matrix_to(p, p, 1, 8, w, 1, m.data_ptr(), 1, st) != 0
+    assert lib.tqk_apply_matrix_to(p, o.data_ptr(), 1, 8, w, 7, m.data_ptr(), 1, st) != 0
+    assert lib.tqk_adjoint_matrix_stored(p, p, p, 1, 8, w, 1, m.data_ptr(), 1, None, st) != 0
+    assert lib.tqk_adjoint_matrix_stored(p, p, o.data_ptr(), 1, 8, w, 7, m.data_ptr(), 1, None, st) != 0
     assert _lib.load() is not None

@@ -14,7 +14,7 @@ result is differentiable with respect to both ``state`` and ``mat`` through a
 saved input: the state cotangent ``U^H g`` and the matrix cotangent ``sum g x^H`` over the
 batch (per row for a per-row matrix), as torch's own ``bmm`` backward gives them.
 
-Gates on one or two wires read the caller's state and write the result (``tqk_apply_matrix_to``,
+Gates on up to six wires read the caller's state and write the result (``tqk_apply_matrix_to``,
 ``tqk_adjoint_matrix_stored``: 2 and 3 transfers of the state); wider ones run the in-place
 kernels on copies.
 """
@@ -71,7 +71,7 @@ def _readable(t: torch.Tensor, bsz: int) -> torch.Tensor:
 
 def _out_of_place(x: torch.Tensor, bsz: int, n: int, k: int) -> bool:
     """Whether the kernels that read one state and write another take this gate."""
-    return k <= 2 and x.numel() == bsz << n
+    return k <= 6 and x.numel() == bsz << n
 
 
 class _ApplyUnitary(torch.autograd.Function):

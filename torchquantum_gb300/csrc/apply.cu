@@ -13,6 +13,7 @@
 #include <stdio.h>
 
 #include "common.cuh"
+#include "dense_tile.cuh"
 
 namespace tqk {
 
@@ -289,10 +290,10 @@ __global__ void __launch_bounds__(256) k_dense_adj(const DenseParams<D> p) {
   if (GRAD) block_reduce_add<GRAD ? 2 * D * D : 1>(acc, p.grad + b * p.grad_stride);
 }
 
-// ------------------------------------------------------------------ generic dense k
-// One block stages gpb groups (2^k amplitudes each) in shared memory, applies the
-// matrix (staged in shared memory too when 2^k <= 64) and writes back.  Thread idx
-// maps to (group gi = idx % gpb, row r = idx / gpb), so a warp shares its matrix row.
+// ------------------------------------------------------------------ dense k, 7 wires and more
+// (3 to 6 wires: dense_tile.cu, but for small reverse steps, see dense_entry.)  One block stages gpb groups (2^k amplitudes each) in shared
+// memory, applies the matrix and writes back.  Thread idx maps to (group gi = idx % gpb,
+// row r = idx / gpb), so a warp shares its matrix row.
 struct DenseKParams {
   float2* state;
   float2* lam;                      // adjoint only
@@ -306,7 +307,6 @@ struct DenseKParams {
   double* grad;                     // adjoint: [batch][D][D] complex128 or null
   int64_t grad_stride;
   int gpb;                          // groups per block
-  int mat_in_smem;
 };
 
 __device__ __forceinline__ uint64_t dk_offset(const DenseKParams& p, int r) {
@@ -318,7 +318,7 @@ __device__ __forceinline__ uint64_t dk_offset(const DenseKParams& p, int r) {
 
 constexpr int kDkMaxOut = 16;
 
-// smem: [mat D*D if staged][tile gpb*(D+1)] (tile rows padded by one amplitude)
+// smem: [tile gpb*(D+1)] (tile rows padded by one amplitude)
 __global__ void __launch_bounds__(256) k_dense_k(const DenseKParams p) {
   extern __shared__ float2 sm[];
   const int D = 1 << p.k;
@@ -326,12 +326,8 @@ __global__ void __launch_bounds__(256) k_dense_k(const DenseKParams p) {
   const int64_t b = blockIdx.y;
   const int64_t gbase = (int64_t)blockIdx.x * p.gpb;
   float2* row = p.state + (b << p.n);
-  const float2* Mg = p.mat + b * p.mat_stride;
-  float2* Ms = sm;
-  float2* tile = sm + (p.mat_in_smem ? D * D : 0);
-  if (p.mat_in_smem)
-    for (int i = threadIdx.x; i < D * D; i += blockDim.x) Ms[i] = Mg[i];
-  const float2* M = p.mat_in_smem ? Ms : Mg;
+  const float2* M = p.mat + b * p.mat_stride;
+  float2* tile = sm;
   const int total = p.gpb * D;
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
     const int gi = idx % p.gpb, r = idx / p.gpb;
@@ -853,14 +849,13 @@ int launch_dense_k(const GateSetup& s, float2* state, float2* lam, const float2*
   p.grad = grad;
   p.grad_stride = mat_batch > 1 ? 2ll * D * D : 0;
   const int threads = 256;
-  // groups per block: up to 32 for narrow gates, bounded by 16 outputs per thread
+  // groups per block: bounded by 16 outputs per thread
   int gpb = 32;
   while (gpb > 1 && (int64_t)gpb * D > kDkMaxOut * threads) gpb >>= 1;
   if (gpb > p.groups) gpb = (int)p.groups;
   p.gpb = gpb;
-  p.mat_in_smem = (!adjoint && D <= 64) ? 1 : 0;
   const size_t tile = (size_t)gpb * (D + 1) * sizeof(float2);
-  const size_t smem = adjoint ? 2 * tile : tile + (p.mat_in_smem ? (size_t)D * D * sizeof(float2) : 0);
+  const size_t smem = adjoint ? 2 * tile : tile;
   if (smem > 200 * 1024) return fail(TQK_TOO_MANY_QUBITS, "dense gate: k=%d too wide", s.kt);
   static bool attr_set = false;
   if (!attr_set) {
@@ -909,6 +904,14 @@ int dense_entry(void* state, void* lam, int64_t bsz, int n, const int32_t* contr
   if (kt == 1) return launch_dense<2>(s, ps, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
   if (kt == 2) return launch_dense<4>(s, ps, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
   if (nc > 0) return fail(TQK_UNSUPPORTED, "%s: controlled gates take 1 or 2 targets", what);
+  // 3 to 6 wires: tiles (dense_tile.cu), but for a reverse step with a cotangent on a small
+  // state, which fits a few CTAs: k = 3, 4, 5 at 2^15 / 2^16 amplitudes took 10-11, 12-14 and
+  // 22-23 us op by op, 16, 20 and 27 us in tiles; at 2^21 it is 138, 142, 111 against 39, 50, 66.
+  const bool small_reverse = adjoint && grad != nullptr && kt <= 5 && (bsz << n) <= (1ll << 18);
+  if (kt >= kTileMinWires && kt <= kTileMaxWires && !small_reverse) {
+    DenseTileArgs a{ps, ps, pl, pl, bsz, n, kt, s.tb, pm, pi, mat_batch, grad, false};
+    return adjoint ? launch_dense_tile_adj(a, st) : launch_dense_tile(a, st);
+  }
   return launch_dense_k(s, ps, pl, pm, pi, mat_batch, grad, adjoint, st);
 }
 
@@ -1014,12 +1017,16 @@ extern "C" int tqk_apply_matrix_to(const void* in, void* out, int64_t bsz, int n
   if ((rc = check_batch(mat_batch, bsz, what))) return rc;
   if (mat == nullptr) return fail(TQK_BAD_POINTER, "%s: null matrix", what);
   if (in == out) return fail(TQK_BAD_POINTER, "%s: out must not alias in (tqk_apply_matrix works in place)", what);
-  if (k < 1 || k > 2) return fail(TQK_TOO_MANY_QUBITS, "%s: k=%d unsupported (1 or 2)", what, k);
+  if (k < 1 || k > kTileMaxWires) return fail(TQK_TOO_MANY_QUBITS, "%s: k=%d unsupported (1..%d)", what, k, kTileMaxWires);
   GateSetup s;
   if ((rc = setup_targets(s, n, bsz, wires, k, nullptr, 0, what))) return rc;
   auto* pi = static_cast<const float2*>(in);
   auto* po = static_cast<float2*>(out);
   auto* pm = static_cast<const float2*>(mat);
+  if (k >= kTileMinWires) {
+    DenseTileArgs a{pi, po, nullptr, nullptr, bsz, n, k, s.tb, pm, nullptr, mat_batch, nullptr, false};
+    return launch_dense_tile(a, as_stream(stream));
+  }
   if (k == 1) return launch_dense<2>(s, pi, po, nullptr, pm, mat_batch, nullptr, nullptr, false, as_stream(stream));
   return launch_dense<4>(s, pi, po, nullptr, pm, mat_batch, nullptr, nullptr, false, as_stream(stream));
 }
@@ -1035,13 +1042,17 @@ extern "C" int tqk_adjoint_matrix_stored(const void* x, const void* g, void* out
   if ((rc = check_batch(mat_batch, bsz, what))) return rc;
   if (mat == nullptr) return fail(TQK_BAD_POINTER, "%s: null matrix", what);
   if (out == x || out == g) return fail(TQK_BAD_POINTER, "%s: out must not alias x or g", what);
-  if (k < 1 || k > 2) return fail(TQK_TOO_MANY_QUBITS, "%s: k=%d unsupported (1 or 2)", what, k);
+  if (k < 1 || k > kTileMaxWires) return fail(TQK_TOO_MANY_QUBITS, "%s: k=%d unsupported (1..%d)", what, k, kTileMaxWires);
   GateSetup s;
   if ((rc = setup_targets(s, n, bsz, wires, k, nullptr, 0, what))) return rc;
   auto* px = static_cast<const float2*>(x);
   auto* pg = static_cast<const float2*>(g);
   auto* po = static_cast<float2*>(out);
   auto* pm = static_cast<const float2*>(mat);
+  if (k >= kTileMinWires) {
+    DenseTileArgs a{px, nullptr, pg, po, bsz, n, k, s.tb, pm, nullptr, mat_batch, grad, true};
+    return launch_dense_tile_adj(a, as_stream(stream));
+  }
   if (k == 1) return launch_dense_stored<2>(s, px, pg, po, pm, mat_batch, grad, as_stream(stream));
   return launch_dense_stored<4>(s, px, pg, po, pm, mat_batch, grad, as_stream(stream));
 }
