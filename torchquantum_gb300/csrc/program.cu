@@ -14,6 +14,7 @@
 //   k_block_unbuild  the reverse: from dL/dU, every op's operand cotangent
 //                    (W <- G_j^H W, X <- G_j^H X, grad_j = sum over the other bits of X W^H).
 #include <math.h>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -294,94 +295,20 @@ __global__ void k_param_grads(const tqk_gate_desc* gates, int ngates) {
 }
 
 // ------------------------------------------------------------------ block build / unbuild
-// Rows of a 2^k x 2^k complex128 matrix in shared memory (row-major, ld = D); block wire
-// i <-> row bit (k-1-i).  apply_op_rows applies op (or its adjoint) to every column.
-template <typename C>
-__device__ void apply_op_rows(C* U, int D, const tqk_block_op& op, const double2* opnd, bool adjoint) {
-  const int nw = op.nw;
-  const int kind = op.kind;
-  const int nc = op.nctrl;
-  uint32_t cmask = 0, tmask = 0;
-  for (int j = 0; j < nc; ++j) cmask |= 1u << op.pos[j];
-  for (int j = nc; j < nw; ++j) tmask |= 1u << op.pos[j];
-  const uint32_t allmask = cmask | tmask;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  if (kind == TQK_K_PHASE) {
-    C ph = mkc<C>(opnd[0].x, opnd[0].y);
-    if (adjoint) ph = conj2(ph);
-    for (int e = tid; e < D * D; e += nth) {
-      const int r = e / D;
-      if ((static_cast<uint32_t>(r) & allmask) == allmask) U[e] = cmul2(ph, U[e]);
-    }
-  } else if (kind == TQK_K_DIAG) {
-    for (int e = tid; e < D * D; e += nth) {
-      const int r = e / D;
-      int di = 0;
-      for (int j = 0; j < nw; ++j) di = (di << 1) | ((r >> op.pos[j]) & 1);
-      C dv = mkc<C>(opnd[di].x, opnd[di].y);
-      if (adjoint) dv = conj2(dv);
-      U[e] = cmul2(dv, U[e]);
-    }
-  } else if (kind == TQK_K_X) {
-    const uint32_t want = op.ctrl_val ? cmask : 0u;
-    const uint32_t tb = 1u << op.pos[nw - 1];
-    for (int e = tid; e < D * D; e += nth) {
-      const int r = e / D, c = e % D;
-      if ((static_cast<uint32_t>(r) & tb) == 0 && (static_cast<uint32_t>(r) & cmask) == want) {
-        const int r2 = r | tb;
-        const C a = U[r * D + c], b2 = U[r2 * D + c];
-        U[r * D + c] = b2;
-        U[r2 * D + c] = a;
-      }
-    }
-  } else if (kind == TQK_K_SWAP) {
-    const uint32_t b0 = 1u << op.pos[nc], b1 = 1u << op.pos[nc + 1];
-    for (int e = tid; e < D * D; e += nth) {
-      const int r = e / D, c = e % D;
-      if ((static_cast<uint32_t>(r) & cmask) == cmask && (r & b0) && !(r & b1)) {
-        const int r2 = (r & ~b0) | b1;
-        const C a = U[r * D + c], b2 = U[r2 * D + c];
-        U[r * D + c] = b2;
-        U[r2 * D + c] = a;
-      }
-    }
-  } else {  // dense (all wires targets) or controlled block on the last nw-nc wires
-    const int kt = nw - nc;
-    const int dt = 1 << kt;
-    C M[16];
-    for (int a = 0; a < dt; ++a)
-      for (int b = 0; b < dt; ++b) {
-        const double2 v = adjoint ? opnd[b * dt + a] : opnd[a * dt + b];
-        M[a * dt + b] = adjoint ? conj2(mkc<C>(v.x, v.y)) : mkc<C>(v.x, v.y);
-      }
-    // work item = (column, group of rows sharing all op bits = 0)
-    const int groups = D >> nw;
-    for (int w = tid; w < groups * D; w += nth) {
-      const int c = w % D, g = w / D;
-      // insert zeros at the op's bit positions
-      uint32_t base = static_cast<uint32_t>(g);
-      for (int q = 0; q < 6; ++q) {
-        if (allmask & (1u << q)) base = ((base >> q) << (q + 1)) | (base & ((1u << q) - 1u));
-      }
-      base |= cmask;
-      int rows[4];
-      C x[4], y[4];
-      for (int a = 0; a < dt; ++a) {
-        uint32_t r = base;
-        for (int j = 0; j < kt; ++j)
-          if ((a >> (kt - 1 - j)) & 1) r |= 1u << op.pos[nc + j];
-        rows[a] = static_cast<int>(r);
-        x[a] = U[r * D + c];
-      }
-      for (int a = 0; a < dt; ++a) {
-        C acc = mkc<C>(0, 0);
-        for (int b = 0; b < dt; ++b) acc = cadd2(acc, cmul2(M[a * dt + b], x[b]));
-        y[a] = acc;
-      }
-      for (int a = 0; a < dt; ++a) U[rows[a] * D + c] = y[a];
-    }
-  }
-}
+// A 2^k x 2^k product in shared memory.  Float64 products of a few blocks bound the build
+// (the pipe does 2 FMAs a clock per SM) and chains of small sweeps the reverse, so the work
+// per op is cut and spread:
+//  * Columns are independent (each op multiplies from the left): 2^split CTAs share a block,
+//    each with the columns whose last `split` bits have its value.
+//  * Bits count in the order the ops reach them.  Before an op reaches bit t the product is
+//    the identity on it, so ops work on the 2^t x 2^t entries of the bits reached so far
+//    (join); in reverse the cotangent's partial trace over a bit is all that the ops before
+//    it see (drop).
+//  * Ops and operands are read 32 at a time, one op per lane, ahead of the sweeps; a sweep of
+//    the reverse updates W and X and takes the operand's cotangent together: one barrier an op.
+// Measured (20 wires, 320 gates in 20 blocks, one of 61 ops; 24 wires, 400 gates in 34 blocks for
+// each of 16 rows): build 915 -> 154 us and 937 -> 259 us (of which half is the pipe), reverse
+// 793 -> 147 us and 648 -> 156 us.
 
 // Descriptor limits the block kernels rely on (shared memory holds a 64 x 64 block; an op
 // touches at most 6 wires, a dense part at most 2 targets): a block or op outside them is
@@ -404,274 +331,524 @@ __device__ __forceinline__ bool op_ok(const tqk_block_op& op, int k) {
   }
 }
 
-__global__ void k_block_build(const tqk_block_desc* blocks, const tqk_block_op* ops) {
+constexpr int kChunk = 32;  // ops read at a time
+
+struct ShOp {
+  const double2* opnd;
+  double* grad;
+  int16_t kind, nw, nctrl, reach;  // reach: bits reached with this op; kind -1: skipped
+  uint16_t fixed;                  // rows' control bits (PHASE: all bits)
+  uint8_t pos[6], asc[6];          // the op's bits in its own and in ascending order
+};
+
+template <typename C>
+struct Stage {
+  ShOp op[kChunk];
+  C m[kChunk][16];
+  int first[6];     // op that first touches a bit (num_ops: none)
+  uint8_t rank[6];  // bit -> its place in that order
+  uint8_t at[64];   // row in that order -> row of the block
+};
+
+// Order of the bits and the row table; ends with the block synchronised.
+template <typename C>
+__device__ void order_bits(Stage<C>& sh, const tqk_block_desc& bl, const tqk_block_op* ops) {
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    int first[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) first[q] = bl.num_ops;
+    for (int i0 = 0; i0 < bl.num_ops; i0 += 32) {
+      uint32_t mask = 0;
+      if (i0 + tid < bl.num_ops) {
+        const tqk_block_op& op = ops[bl.first_op + i0 + tid];
+        if (op_ok(op, bl.k))
+          for (int j = 0; j < op.nw; ++j) mask |= 1u << op.pos[j];
+      }
+      bool open = false;
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const uint32_t who = __ballot_sync(0xffffffffu, (mask >> q) & 1u);
+        if (first[q] == bl.num_ops && who != 0) first[q] = i0 + __ffs(who) - 1;
+        open |= q < bl.k && first[q] == bl.num_ops;
+      }
+      if (!open) break;
+    }
+    int rank[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      rank[q] = 0;
+#pragma unroll
+      for (int p = 0; p < 6; ++p)
+        if (p < bl.k && (first[p] < first[q] || (first[p] == first[q] && p < q))) ++rank[q];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t r = 0;
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        if (q < bl.k) r |= (((tid + 32 * h) >> rank[q]) & 1u) << q;
+      sh.at[tid + 32 * h] = static_cast<uint8_t>(r);
+    }
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+      if (tid == q) {
+        sh.first[q] = first[q];
+        sh.rank[q] = static_cast<uint8_t>(rank[q]);
+      }
+  }
+  __syncthreads();
+}
+
+template <typename C>
+__device__ __forceinline__ C from_d2(const double2& v) {
+  return mkc<C>(v.x, v.y);
+}
+
+// Ops i0 .. i0 + 31 of the block into shared memory; ends with the block synchronised.
+template <typename C>
+__device__ void stage_ops(Stage<C>& sh, const tqk_block_desc& bl, const tqk_block_op* ops, int i0, int64_t b) {
+  const int tid = threadIdx.x;
+  if (tid < kChunk && i0 + tid < bl.num_ops) {
+    const tqk_block_op& op = ops[bl.first_op + i0 + tid];
+    ShOp o;
+    o.kind = -1;
+    uint32_t bits = 0;
+    for (int j = 0; j < 6; ++j) bits |= j < op.nw && op.pos[j] >= 0 ? 1u << (op.pos[j] & 31) : 0u;
+    if (op_ok(op, bl.k) && __popc(bits) == op.nw) {  // (a bit named twice: no row has it clear once)
+      const int64_t row = (op.batch > 1 ? b : 0) * op.op_size;
+      o.kind = static_cast<int16_t>(op.kind);
+      o.nw = static_cast<int16_t>(op.nw);
+      o.nctrl = static_cast<int16_t>(op.nctrl);
+      o.opnd = static_cast<const double2*>(op.operand) + row;
+      o.grad = op.grad == nullptr ? nullptr : static_cast<double*>(op.grad) + 2 * row;
+      uint32_t mask = 0, fixed = 0;
+      for (int j = 0; j < op.nw; ++j) {
+        o.pos[j] = sh.rank[op.pos[j]];
+        mask |= 1u << o.pos[j];
+        if (op.kind == TQK_K_PHASE || (op.kind != TQK_K_DIAG && j < op.nctrl)) fixed |= 1u << o.pos[j];
+      }
+      if (op.kind == TQK_K_X && !op.ctrl_val) fixed = 0;  // a flip under open controls
+      o.fixed = static_cast<uint16_t>(fixed);
+      int n = 0, reach = 0;
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        if ((mask >> q) & 1u) o.asc[n++] = static_cast<uint8_t>(q);
+        reach += q < bl.k && sh.first[q] <= i0 + tid;
+      }
+      o.reach = static_cast<int16_t>(reach);
+    }
+    sh.op[tid] = o;
+  }
+  __syncthreads();
+  for (int e = tid; e < kChunk * 16; e += blockDim.x) {
+    const int i = e >> 4, q = e & 15;
+    if (i0 + i >= bl.num_ops) break;
+    const ShOp& o = sh.op[i];
+    int n = 0;
+    if (o.kind == TQK_K_PHASE) n = 1;
+    else if (o.kind == TQK_K_DIAG) n = 1 << min(static_cast<int>(o.nw), 4);
+    else if (o.kind == TQK_K_DENSE || o.kind == TQK_K_CTRL) n = 1 << 2 * (o.nw - o.nctrl);
+    if (q < n) sh.m[i][q] = from_d2<C>(o.opnd[q]);
+  }
+  __syncthreads();
+}
+
+// Row g of those with the op's bits clear.
+__device__ __forceinline__ int clear_row(int g, const ShOp& op) {
+  for (int j = 0; j < op.nw; ++j) {
+    const int p = op.asc[j];
+    g = ((g >> p) << (p + 1)) | (g & ((1 << p) - 1));
+  }
+  return g;
+}
+
+// Rows of the patterns over op bits pos[from], .., pos[from + N - 1] (the first is the pattern's
+// most significant bit).
+template <int N>
+__device__ __forceinline__ void pattern_rows(const ShOp& op, int from, int (&pat)[1 << N]) {
+#pragma unroll
+  for (int a = 0; a < (1 << N); ++a) {
+    pat[a] = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if ((a >> (N - 1 - j)) & 1) pat[a] |= 1 << op.pos[from + j];
+  }
+}
+
+template <typename C>
+__device__ __forceinline__ C fma2(C a, C b, C c) {  // a b + c
+  return C{fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y))};
+}
+
+// A matrix of one CTA: 2^reach rows (leading dimension ld) by 2^lc columns.
+struct Part {
+  int ld, lc;
+  int reach;
+};
+
+// The rows an exchange op (flip, swap) swaps within the rows of one clear_row.
+__device__ __forceinline__ void exchange_rows(const ShOp& op, int& r0, int& r1) {
+  r0 = op.kind == TQK_K_X ? 0 : 1 << op.pos[op.nctrl];
+  r1 = 1 << op.pos[op.kind == TQK_K_X ? op.nw - 1 : op.nctrl + 1];
+}
+
+// One target whose matrix has real diagonal and real (RY, H) or imaginary (RX) off-diagonal
+// entries: half the float64 products.
+__device__ __forceinline__ bool half_real(const C2* m) {
+  return m[0].y == 0.0 && m[3].y == 0.0 && ((m[1].y == 0.0 && m[2].y == 0.0) || (m[1].x == 0.0 && m[2].x == 0.0));
+}
+
+__device__ __forceinline__ void build_half_real(C2* U, const Part& p, const ShOp& op, const C2* m) {
+  const bool real = m[1].y == 0.0 && m[2].y == 0.0;
+  const double d0 = m[0].x, d1 = m[3].x, o0 = real ? m[1].x : m[1].y, o1 = real ? m[2].x : m[2].y;
+  const int items = 1 << (p.reach - op.nw + p.lc), high = p.ld << op.pos[op.nctrl];
+  for (int w = threadIdx.x; w < items; w += blockDim.x) {
+    C2* u = U + (clear_row(w >> p.lc, op) | op.fixed) * p.ld + (w & ((1 << p.lc) - 1));
+    const C2 a = u[0], b = u[high];
+    const C2 ta = real ? a : mul_i(a), tb = real ? b : mul_i(b);
+    u[0] = C2{fma(o0, tb.x, d0 * a.x), fma(o0, tb.y, d0 * a.y)};
+    u[high] = C2{fma(d1, b.x, o1 * ta.x), fma(d1, b.y, o1 * ta.y)};
+  }
+}
+
+template <int KT>
+__device__ __forceinline__ void build_dense(C2* U, const Part& p, const ShOp& op, const C2* m) {
+  constexpr int DT = 1 << KT;
+  int pat[DT];
+  pattern_rows<KT>(op, op.nctrl, pat);
+  C2 M[DT * DT];
+#pragma unroll
+  for (int e = 0; e < DT * DT; ++e) M[e] = m[e];
+  const int items = 1 << (p.reach - op.nw + p.lc);
+  for (int w = threadIdx.x; w < items; w += blockDim.x) {
+    C2* u = U + (clear_row(w >> p.lc, op) | op.fixed) * p.ld + (w & ((1 << p.lc) - 1));
+    C2 x[DT];
+#pragma unroll
+    for (int a = 0; a < DT; ++a) x[a] = u[pat[a] * p.ld];
+#pragma unroll
+    for (int a = 0; a < DT; ++a) {
+      C2 y = cmul2(M[a * DT], x[0]);
+#pragma unroll
+      for (int c = 1; c < DT; ++c) y = fma2(M[a * DT + c], x[c], y);
+      u[pat[a] * p.ld] = y;
+    }
+  }
+}
+
+__device__ void build_op(C2* U, const Part& p, const ShOp& op, const C2* m) {
+  const int cols = 1 << p.lc, items = 1 << (p.reach - op.nw + p.lc);
+  if (op.kind == TQK_K_PHASE) {
+    const C2 ph = m[0];
+    for (int w = threadIdx.x; w < items; w += blockDim.x) {
+      C2& u = U[(clear_row(w >> p.lc, op) | op.fixed) * p.ld + (w & (cols - 1))];
+      u = cmul2(ph, u);
+    }
+  } else if (op.kind == TQK_K_DIAG) {
+    for (int w = threadIdx.x; w < 1 << (p.reach + p.lc); w += blockDim.x) {
+      const int r = w >> p.lc;
+      int di = 0;
+      for (int j = 0; j < op.nw; ++j) di = (di << 1) | ((r >> op.pos[j]) & 1);
+      C2& u = U[r * p.ld + (w & (cols - 1))];
+      u = cmul2(op.nw <= 4 ? m[di] : from_d2<C2>(op.opnd[di]), u);
+    }
+  } else if (op.kind == TQK_K_X || op.kind == TQK_K_SWAP) {
+    int r0, r1;
+    exchange_rows(op, r0, r1);
+    for (int w = threadIdx.x; w < items; w += blockDim.x) {
+      C2* u = U + (clear_row(w >> p.lc, op) | op.fixed) * p.ld + (w & (cols - 1));
+      const C2 v = u[r0 * p.ld];
+      u[r0 * p.ld] = u[r1 * p.ld];
+      u[r1 * p.ld] = v;
+    }
+  } else if (op.nw - op.nctrl == 1 && half_real(m)) {
+    build_half_real(U, p, op, m);
+  } else if (op.nw - op.nctrl == 1) {
+    build_dense<1>(U, p, op, m);
+  } else {
+    build_dense<2>(U, p, op, m);
+  }
+}
+
+__global__ void k_block_build(const tqk_block_desc* blocks, const tqk_block_op* ops, int split) {
   extern __shared__ double2 smem_u[];
+  __shared__ Stage<C2> sh;
   C2* U = reinterpret_cast<C2*>(smem_u);
   const tqk_block_desc bl = blocks[blockIdx.x];
   const int64_t b = blockIdx.y;
+  const int z = blockIdx.z;
   if (b >= bl.batch || !block_ok(bl)) return;
-  const int D = 1 << bl.k;
-  for (int e = threadIdx.x; e < D * D; e += blockDim.x) U[e] = mk((e / D) == (e % D) ? 1.0 : 0.0, 0.0);
+  split = min(split, bl.k);
+  if (z >> split) return;
+  const int tid = threadIdx.x, nth = blockDim.x, whole = bl.k - split;  // bits with all columns
+  Part p{1 << whole, 0, 0};
+  order_bits(sh, bl, ops);
+  if (tid == 0) U[0] = mk(1.0, 0.0);
   __syncthreads();
-  for (int i = 0; i < bl.num_ops; ++i) {
-    const tqk_block_op op = ops[bl.first_op + i];
-    if (!op_ok(op, bl.k)) continue;  // uniform for the CTA
-    const double2* opnd = static_cast<const double2*>(op.operand) + (op.batch > 1 ? b : 0) * op.op_size;
-    apply_op_rows(U, D, op, opnd, false);
-    __syncthreads();
-  }
-  double2* dst = static_cast<double2*>(bl.u) + b * D * D;
-  for (int e = threadIdx.x; e < D * D; e += blockDim.x) dst[e] = make_double2(U[e].x, U[e].y);
-}
-
-// grad of op (operand cotangent) = sum over rows/cols of X[row][col] conj(W[row'][col]) restricted
-// to the op's structure; W = product of the ops before it, X = (ops after)^H dL/dU.
-// One sweep per entry: ops outside the specialised shapes below.
-template <typename C>
-__device__ void op_cotangent_generic(const C* X, const C* W, int D, const tqk_block_op& op, double2* gout, bool accumulate) {
-  const int nw = op.nw, nc = op.nctrl;
-  uint32_t cmask = 0, tmask = 0;
-  for (int j = 0; j < nc; ++j) cmask |= 1u << op.pos[j];
-  for (int j = nc; j < nw; ++j) tmask |= 1u << op.pos[j];
-  const uint32_t allmask = cmask | tmask;
-  int nent, kt = nw - nc;
-  if (op.kind == TQK_K_PHASE) nent = 1;
-  else if (op.kind == TQK_K_DIAG) nent = 1 << nw;
-  else nent = (1 << kt) * (1 << kt);
-  __shared__ double red[32][2];
-  for (int ent = 0; ent < nent; ++ent) {
-    double ax = 0.0, ay = 0.0;
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
-      const int r = e / D, c = e % D;
-      int rr = -1;  // partner row (W side) for this X row
-      if (op.kind == TQK_K_PHASE) {
-        if ((static_cast<uint32_t>(r) & allmask) == allmask) rr = r;
-      } else if (op.kind == TQK_K_DIAG) {
-        int di = 0;
-        for (int j = 0; j < nw; ++j) di = (di << 1) | ((r >> op.pos[j]) & 1);
-        if (di == ent) rr = r;
-      } else {
-        if ((static_cast<uint32_t>(r) & cmask) == cmask) {
-          const int dt = 1 << kt;
-          const int a_want = ent / dt, b_want = ent % dt;
-          int a = 0;
-          for (int j = 0; j < kt; ++j) a = (a << 1) | ((r >> op.pos[nc + j]) & 1);
-          if (a == a_want) {
-            uint32_t r2 = static_cast<uint32_t>(r) & ~tmask;
-            for (int j = 0; j < kt; ++j)
-              if ((b_want >> (kt - 1 - j)) & 1) r2 |= 1u << op.pos[nc + j];
-            rr = static_cast<int>(r2);
-          }
+  for (int i = 0; i <= bl.num_ops; ++i) {
+    const bool last = i == bl.num_ops;  // then only the bits that no op touches are left
+    const int q = i % kChunk;
+    if (!last && q == 0) stage_ops(sh, bl, ops, i, b);
+    if (!last && sh.op[q].kind < 0) continue;  // uniform for the CTA
+    const int reach = last ? bl.k : sh.op[q].reach;
+    while (p.reach < reach) {  // join: U <- U (x) identity on the next bit
+      const int d = 1 << p.reach, cols = 1 << p.lc, v = (z >> max(p.reach - whole, 0)) & 1;
+      const bool both = p.reach < whole;
+      for (int w = tid; w < d << p.lc; w += nth) {
+        C2* u = U + (w >> p.lc) * p.ld + (w & (cols - 1));
+        const C2 val = *u, none = mk(0.0, 0.0);
+        if (both) {
+          u[cols] = none;
+          u[d * p.ld] = none;
+          u[d * p.ld + cols] = val;
+        } else {
+          *u = v ? none : val;
+          u[d * p.ld] = v ? val : none;
         }
       }
-      if (rr >= 0) {
-        const C xv = X[r * D + c], wv = W[rr * D + c];
-        ax += xv.x * wv.x + xv.y * wv.y;  // x * conj(w)
-        ay += xv.y * wv.x - xv.x * wv.y;
-      }
+      p.lc += both;
+      ++p.reach;
+      __syncthreads();
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      ax += __shfl_xor_sync(0xffffffffu, ax, o);
-      ay += __shfl_xor_sync(0xffffffffu, ay, o);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { red[warp][0] = ax; red[warp][1] = ay; }
+    if (last) break;
+    build_op(U, p, sh.op[q], sh.m[q]);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double sx = 0, sy = 0;
-      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) { sx += red[w][0]; sy += red[w][1]; }
-      if (accumulate) {
-        atomicAdd(&gout[ent].x, sx);
-        atomicAdd(&gout[ent].y, sy);
+  }
+  const int D = 1 << bl.k;
+  double2* dst = static_cast<double2*>(bl.u) + b * D * D;
+  for (int e = tid; e < D << whole; e += nth) {
+    const C2 v = U[e];
+    dst[sh.at[e >> whole] * D + sh.at[(e & ((1 << whole) - 1)) | (z << whole)]] = make_double2(v.x, v.y);
+  }
+}
+
+// ---- reverse.  With W the product of the ops before an op and X = (ops after)^H dL/dU, the
+// operand's cotangent is the sum, over the rows with the op's control bits set and over the
+// columns, of X[row with target pattern a] conj(W[row with target pattern b]) at entry (a, b)
+// (diagonal ops: a = b over all op bits; phase ops: the single all-ones pattern).  Threads sum
+// their items in float32 (diagonals on more than two bits in float64), warps and CTAs in float64.
+
+struct Sums {
+  double v[2][8][32];  // by op parity: a warp's sums, written before the barrier that ends the op
+};
+
+// Sums of v over the warp by halves (each step hands half of the values over: NV - 1 + log2(32/NV)
+// float64 additions instead of 5 NV) into out[0 .. NV).
+template <int NV, typename R>
+__device__ __forceinline__ void warp_sums(const R (&v)[NV], double* out) {
+  const int lane = threadIdx.x & 31;
+  double s[NV];
+#pragma unroll
+  for (int h = NV / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      if (h == NV / 2) {  // the first hand-over in the type of the terms
+        const R send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+        s[i] = static_cast<double>(keep) + static_cast<double>(__shfl_xor_sync(0xffffffffu, send, o));
       } else {
-        gout[ent] = make_double2(sx, sy);
+        const double send = up ? s[i] : s[i + h], keep = up ? s[i + h] : s[i];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
-    __syncthreads();
   }
-}
-
-// Row r with zeros inserted at the (ascending) bit positions pos[0..m).
-__device__ __forceinline__ int insert_zeros(int r, const int* pos, int m) {
-  for (int j = 0; j < m; ++j) r = ((r >> pos[j]) << (pos[j] + 1)) | (r & ((1 << pos[j]) - 1));
-  return r;
-}
-
-// Sum of NE complex partial sums over the block; entries added (or stored) into gout.
-template <int NE>
-__device__ void block_reduce_entries(double (&acc)[2 * NE], double2* gout, int nent, bool accumulate) {
-  __shared__ double red[8][2 * 16];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
 #pragma unroll
-  for (int q = 0; q < 2 * NE; ++q) {
-    double v = acc[q];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][q] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 2 * nent) {
-    double t = 0.0;
-    for (int w = 0; w < nwarps; ++w) t += red[w][threadIdx.x];
-    double* g = reinterpret_cast<double*>(gout) + threadIdx.x;
-    if (accumulate) atomicAdd(g, t);
-    else *g = t;
-  }
-  __syncthreads();
+  for (int o = 16 / NV; o >= 1; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+  if (lane % (32 / NV) == 0) out[lane / (32 / NV)] = s[0];
 }
 
-// Cotangent of the op's operand from X (cotangent rows) and W (state rows):
-// entry (a, b) = sum over rows r with the op's control bits set and target pattern a, and
-// columns c, of X[r][c] conj(W[r with target pattern b][c]) (diagonal ops: a = b over
-// all op bits; phase ops: the single all-ones pattern).  One sweep over (row with the op's
-// bits cleared, column) pairs evaluates every entry.
-template <int KT, typename C>
-__device__ void cot_dense(const C* X, const C* W, int D, const tqk_block_op& op, double2* gout, bool accumulate) {
-  using R = typename C::real;
+// X (cotangent) and W to before a dense op; its cotangent's warp sums into out.  Warps without
+// items add nothing (active_warps leaves them out).
+template <int KT>
+__device__ __forceinline__ void unbuild_dense(F2* X, F2* W, const Part& p, const ShOp& op, const F2* m, double* out) {
   constexpr int DT = 1 << KT, NE = DT * DT;
-  const int nc = op.nctrl;
-  uint32_t cmask = 0;
-  for (int j = 0; j < nc; ++j) cmask |= 1u << op.pos[j];
-  int tbit[KT], tsorted[KT];
-#pragma unroll
-  for (int j = 0; j < KT; ++j) tbit[j] = op.pos[nc + j];  // j = 0 is the pattern's most significant bit
-#pragma unroll
-  for (int j = 0; j < KT; ++j) tsorted[j] = tbit[j];
-  if (KT == 2 && tsorted[0] > tsorted[1]) {
-    const int t = tsorted[0];
-    tsorted[0] = tsorted[1];
-    tsorted[1] = t;
-  }
   int pat[DT];
+  pattern_rows<KT>(op, op.nctrl, pat);
+  F2 M[NE];
 #pragma unroll
-  for (int a = 0; a < DT; ++a) {
-    int r = 0;
+  for (int e = 0; e < NE; ++e) M[e] = m[e];
+  float acc[2 * NE];
 #pragma unroll
-    for (int j = 0; j < KT; ++j)
-      if ((a >> (KT - 1 - j)) & 1) r |= 1 << tbit[j];
-    pat[a] = r;
-  }
-  R acc[2 * NE];
-#pragma unroll
-  for (int q = 0; q < 2 * NE; ++q) acc[q] = R(0);
-  const int nbase = D >> KT;
-  for (int w = threadIdx.x; w < nbase * D; w += blockDim.x) {
-    const int c = w % D;
-    const int r = insert_zeros(w / D, tsorted, KT);
-    if ((static_cast<uint32_t>(r) & cmask) != cmask) continue;
-    C xs[DT], ws[DT];
+  for (int q = 0; q < 2 * NE; ++q) acc[q] = 0.f;
+  const int items = 1 << (p.reach - op.nw + p.lc);
+  if (static_cast<int>(threadIdx.x & ~31u) >= items) return;
+  for (int w = threadIdx.x; w < items; w += blockDim.x) {
+    const int at = (clear_row(w >> p.lc, op) | op.fixed) * p.ld + (w & ((1 << p.lc) - 1));
+    F2 xs[DT], ws[DT], wn[DT];
 #pragma unroll
     for (int a = 0; a < DT; ++a) {
-      xs[a] = X[(r | pat[a]) * D + c];
-      ws[a] = W[(r | pat[a]) * D + c];
+      xs[a] = X[at + pat[a] * p.ld];
+      ws[a] = W[at + pat[a] * p.ld];
+    }
+#pragma unroll
+    for (int a = 0; a < DT; ++a) {
+      F2 y = cmul2(conj2(M[a]), ws[0]), g = cmul2(conj2(M[a]), xs[0]);
+#pragma unroll
+      for (int c = 1; c < DT; ++c) {
+        y = fma2(conj2(M[c * DT + a]), ws[c], y);
+        g = fma2(conj2(M[c * DT + a]), xs[c], g);
+      }
+      wn[a] = y;
+      W[at + pat[a] * p.ld] = y;
+      X[at + pat[a] * p.ld] = g;
     }
 #pragma unroll
     for (int a = 0; a < DT; ++a)
 #pragma unroll
-      for (int b2 = 0; b2 < DT; ++b2) {
-        acc[2 * (a * DT + b2)] += xs[a].x * ws[b2].x + xs[a].y * ws[b2].y;  // x * conj(w)
-        acc[2 * (a * DT + b2) + 1] += xs[a].y * ws[b2].x - xs[a].x * ws[b2].y;
+      for (int c = 0; c < DT; ++c) {
+        acc[2 * (a * DT + c)] += xs[a].x * wn[c].x + xs[a].y * wn[c].y;  // x * conj(w)
+        acc[2 * (a * DT + c) + 1] += xs[a].y * wn[c].x - xs[a].x * wn[c].y;
       }
   }
-  double accd[2 * NE];
-#pragma unroll
-  for (int q = 0; q < 2 * NE; ++q) accd[q] = static_cast<double>(acc[q]);
-  block_reduce_entries<NE>(accd, gout, NE, accumulate);
+  if (op.grad != nullptr) warp_sums(acc, out);
 }
 
-// Diagonal ops (entries = pattern over all NW op bits) and phase ops (one entry: all bits set).
-template <int NW, typename C>
-__device__ void cot_diag(const C* X, const C* W, int D, const tqk_block_op& op, double2* gout, bool accumulate,
-                         bool phase) {
-  using R = typename C::real;
+// The same for the 2^NW patterns over the op's last NW bits with its other bits at `fixed`
+// (diagonals of up to 4 bits, parts of larger ones, phases: NW = 0).
+template <int NW>
+__device__ __forceinline__ void unbuild_diag(F2* X, F2* W, const Part& p, const ShOp& op, int fixed, const F2* m,
+                                             double* out) {
   constexpr int DT = 1 << NW;
-  int bit[NW], srt[NW];
-#pragma unroll
-  for (int j = 0; j < NW; ++j) srt[j] = bit[j] = op.pos[j];
-  if (NW == 2 && srt[0] > srt[1]) {
-    const int t = srt[0];
-    srt[0] = srt[1];
-    srt[1] = t;
-  }
   int pat[DT];
+  pattern_rows<NW>(op, op.nw - NW, pat);
+  typename std::conditional<(NW > 2), double, float>::type acc[2 * DT];
 #pragma unroll
-  for (int a = 0; a < DT; ++a) {
-    int r = 0;
-#pragma unroll
-    for (int j = 0; j < NW; ++j)
-      if ((a >> (NW - 1 - j)) & 1) r |= 1 << bit[j];
-    pat[a] = r;
-  }
-  R acc[2 * DT];
-#pragma unroll
-  for (int q = 0; q < 2 * DT; ++q) acc[q] = R(0);
-  const int nbase = D >> NW;
-  for (int w = threadIdx.x; w < nbase * D; w += blockDim.x) {
-    const int c = w % D;
-    const int r = insert_zeros(w / D, srt, NW);
+  for (int q = 0; q < 2 * DT; ++q) acc[q] = 0;
+  const int items = 1 << (p.reach - op.nw + p.lc);
+  if (static_cast<int>(threadIdx.x & ~31u) >= items) return;
+  for (int w = threadIdx.x; w < items; w += blockDim.x) {
+    const int at = (clear_row(w >> p.lc, op) | fixed) * p.ld + (w & ((1 << p.lc) - 1));
 #pragma unroll
     for (int a = 0; a < DT; ++a) {
-      if (phase && a != DT - 1) continue;
-      const C xv = X[(r | pat[a]) * D + c], wv = W[(r | pat[a]) * D + c];
-      acc[2 * a] += xv.x * wv.x + xv.y * wv.y;
-      acc[2 * a + 1] += xv.y * wv.x - xv.x * wv.y;
+      const int i = at + pat[a] * p.ld;
+      const F2 d = conj2(m[a]), x = X[i], w2 = cmul2(d, W[i]);
+      acc[2 * a] += x.x * w2.x + x.y * w2.y;
+      acc[2 * a + 1] += x.y * w2.x - x.x * w2.y;
+      W[i] = w2;
+      X[i] = cmul2(d, x);
     }
   }
-  if (phase) {  // the single entry sits at index DT - 1
-    acc[0] = acc[2 * (DT - 1)];
-    acc[1] = acc[2 * (DT - 1) + 1];
-  }
-  double accd[2 * DT];
-#pragma unroll
-  for (int q = 0; q < 2 * DT; ++q) accd[q] = static_cast<double>(acc[q]);
-  block_reduce_entries<DT>(accd, gout, phase ? 1 : DT, accumulate);
+  if (op.grad != nullptr) warp_sums(acc, out);
 }
 
-template <typename C>
-__device__ void op_cotangent(const C* X, const C* W, int D, const tqk_block_op& op, double2* gout, bool accumulate) {
-  const int kt = op.nw - op.nctrl;
-  const bool diag = op.kind == TQK_K_PHASE || op.kind == TQK_K_DIAG;
-  if ((diag && (op.nw < 1 || op.nw > 4)) || (!diag && (kt < 1 || kt > 2))) {
-    op_cotangent_generic(X, W, D, op, gout, accumulate);
-  } else if (diag) {
-    const bool phase = op.kind == TQK_K_PHASE;
-    if (op.nw == 1) cot_diag<1, C>(X, W, D, op, gout, accumulate, phase);
-    else if (op.nw == 2) cot_diag<2, C>(X, W, D, op, gout, accumulate, phase);
-    else if (op.nw == 3) cot_diag<3, C>(X, W, D, op, gout, accumulate, phase);
-    else cot_diag<4, C>(X, W, D, op, gout, accumulate, phase);
-  } else if (kt == 1) {
-    cot_dense<1, C>(X, W, D, op, gout, accumulate);
-  } else {
-    cot_dense<2, C>(X, W, D, op, gout, accumulate);
-  }
+// After a barrier: the CTA's sums added to the operand's cotangent.
+__device__ __forceinline__ void add_sums(const double (*v)[32], const Part& p, const ShOp& op, double* grad, int count) {
+  if (static_cast<int>(threadIdx.x) >= count) return;
+  const int warps = min(static_cast<int>(blockDim.x >> 5), max(1, (1 << (p.reach - op.nw + p.lc)) >> 5));
+  double t = 0.0;
+  for (int w = 0; w < warps; ++w) t += v[w][threadIdx.x];
+  atomicAdd(grad + threadIdx.x, t);
 }
 
-__global__ void k_block_unbuild(const tqk_block_desc* blocks, const tqk_block_op* ops) {
+// Returns the number of sums.
+__device__ int unbuild_op(F2* X, F2* W, const Part& p, const ShOp& op, F2* m, Sums& sums, int par) {
+  double* out = sums.v[par][threadIdx.x >> 5];
+  if (op.kind == TQK_K_X || op.kind == TQK_K_SWAP) {
+    int r0, r1;
+    exchange_rows(op, r0, r1);
+    const int items = 1 << (p.reach - op.nw + p.lc);
+    for (int w = threadIdx.x; w < items; w += blockDim.x) {
+      const int at = (clear_row(w >> p.lc, op) | op.fixed) * p.ld + (w & ((1 << p.lc) - 1));
+      const int i0 = at + r0 * p.ld, i1 = at + r1 * p.ld;
+      const F2 w0 = W[i0], x0 = X[i0];
+      W[i0] = W[i1];
+      W[i1] = w0;
+      X[i0] = X[i1];
+      X[i1] = x0;
+    }
+    return 0;
+  }
+  if (op.kind == TQK_K_PHASE) {
+    unbuild_diag<0>(X, W, p, op, op.fixed, m, out);
+    return 2;
+  }
+  if (op.kind == TQK_K_DIAG) {
+    if (op.nw == 1) unbuild_diag<1>(X, W, p, op, 0, m, out);
+    else if (op.nw == 2) unbuild_diag<2>(X, W, p, op, 0, m, out);
+    else if (op.nw == 3) unbuild_diag<3>(X, W, p, op, 0, m, out);
+    else {
+      // one part of 16 patterns for each value of the bits before the last four; all but the
+      // last are added here, the last by the caller
+      const int high = op.nw - 4;
+      for (int h = 0;; ++h) {
+        int fixed = 0;
+        for (int j = 0; j < high; ++j)
+          if ((h >> (high - 1 - j)) & 1) fixed |= 1 << op.pos[j];
+        unbuild_diag<4>(X, W, p, op, fixed, m, out);
+        if (h == (1 << high) - 1) break;
+        __syncthreads();
+        if (op.grad != nullptr) add_sums(sums.v[par], p, op, op.grad + 32 * h, 32);
+        if (threadIdx.x < 16) m[threadIdx.x] = from_d2<F2>(op.opnd[16 * (h + 1) + threadIdx.x]);
+        __syncthreads();
+      }
+    }
+    return 2 << min(static_cast<int>(op.nw), 4);
+  }
+  if (op.nw - op.nctrl == 1) {
+    unbuild_dense<1>(X, W, p, op, m, out);
+    return 8;
+  }
+  unbuild_dense<2>(X, W, p, op, m, out);
+  return 32;
+}
+
+__global__ void k_block_unbuild(const tqk_block_desc* blocks, const tqk_block_op* ops, int split) {
   extern __shared__ double2 smem_u[];
+  __shared__ Stage<F2> sh;
+  __shared__ Sums sums;
   const tqk_block_desc bl = blocks[blockIdx.x];
   const int64_t b = blockIdx.y;
+  const int z = blockIdx.z;
   if (b >= bl.batch || bl.gu == nullptr || !block_ok(bl)) return;
+  split = min(split, bl.k);
+  if (z >> split) return;
+  const int tid = threadIdx.x, nth = blockDim.x, whole = bl.k - split;
   const int D = 1 << bl.k;
+  Part p{1 << whole, whole, bl.k};
   F2* W = reinterpret_cast<F2*>(smem_u);
-  F2* X = W + D * D;
+  F2* X = W + (D << whole);
+  order_bits(sh, bl, ops);
   const double2* us = static_cast<const double2*>(bl.u) + b * D * D;
   const double2* gs = static_cast<const double2*>(bl.gu) + b * D * D;
-  for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
-    W[e] = mkc<F2>(us[e].x, us[e].y);
-    X[e] = mkc<F2>(gs[e].x, gs[e].y);
+  for (int e = tid; e < D << whole; e += nth) {
+    const int i = sh.at[e >> whole] * D + sh.at[(e & ((1 << whole) - 1)) | (z << whole)];
+    W[e] = from_d2<F2>(us[i]);
+    X[e] = from_d2<F2>(gs[i]);
   }
-  __syncthreads();
+  int par = 0;
   for (int i = bl.num_ops - 1; i >= 0; --i) {
-    const tqk_block_op op = ops[bl.first_op + i];
-    if (!op_ok(op, bl.k)) continue;  // uniform for the CTA
-    const double2* opnd = static_cast<const double2*>(op.operand) + (op.batch > 1 ? b : 0) * op.op_size;
-    apply_op_rows(W, D, op, opnd, true);  // W <- G^H W = product of the ops before op
-    __syncthreads();
-    if (op.grad != nullptr) {
-      double2* gout = static_cast<double2*>(op.grad) + (op.batch > 1 ? b : 0) * op.op_size;
-      op_cotangent(X, W, D, op, gout, true);
+    const int q = i % kChunk;
+    if (q == kChunk - 1 || i == bl.num_ops - 1) {
+      __syncthreads();  // the sums of the chunk after read its table
+      stage_ops(sh, bl, ops, i - q, b);
     }
-    apply_op_rows(X, D, op, opnd, true);  // X <- G^H X
+    const ShOp& op = sh.op[q];
+    if (op.kind < 0) continue;  // uniform for the CTA
+    while (p.reach > op.reach) {  // drop: X <- its partial trace over the last bit
+      --p.reach;
+      const bool both = p.reach < whole;
+      p.lc -= both;
+      const int d = 1 << p.reach, cols = 1 << p.lc;
+      if (both || ((z >> (p.reach - whole)) & 1)) {
+        for (int w = tid; w < d << p.lc; w += nth) {
+          const int e = (w >> p.lc) * p.ld + (w & (cols - 1)), o = e + d * p.ld;
+          if (both) {
+            X[e] = cadd2(X[e], X[o + cols]);
+          } else {  // this CTA's columns have the bit set: so have the rows that meet W's
+            X[e] = X[o];
+            W[e] = W[o];
+          }
+        }
+        __syncthreads();
+      }
+    }
+    const int count = unbuild_op(X, W, p, op, sh.m[q], sums, par);
     __syncthreads();
+    if (op.grad != nullptr && count > 0) {
+      const int skip = op.kind == TQK_K_DIAG && op.nw > 4 ? 32 * ((1 << (op.nw - 4)) - 1) : 0;
+      add_sums(sums.v[par], p, op, op.grad + skip, count);
+    }
+    par ^= 1;
   }
 }
 
@@ -696,23 +873,22 @@ extern "C" int tqk_param_grads(const tqk_gate_desc* gates, int ngates, void* str
   return launch_status("tqk_param_grads");
 }
 
-static void set_block_smem_attrs() {
-  static int done = 0;
-  if (done) return;
-  const int one = static_cast<int>(64 * 64 * sizeof(double2));
-  cudaFuncSetAttribute(prog::k_block_build, cudaFuncAttributeMaxDynamicSharedMemorySize, one);
-  cudaFuncSetAttribute(prog::k_block_unbuild, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * one);
-  done = 1;
-}
+// Column bits that a block's CTAs share out, and threads: best of splits 0 to 3 with 64 to 256
+// threads on the circuits named at the kernels (build 154 + 259 us against 299 + 299 without a
+// split; reverse 147 + 156 against 152 + 206).  The reverse sums at most 8
+// float32 terms a thread (64 rows x 16 columns over 64 threads, one target).  Idle CTAs (rows
+// of a block without a batch, narrow blocks) leave at once.
+constexpr int kBuildSplit = 3, kBuildThreads = 128;
+constexpr int kUnbuildSplit = 2, kUnbuildThreads = 64;
 
 extern "C" int tqk_block_build(const tqk_block_desc* blocks, int nblocks, int max_batch, const tqk_block_op* ops,
                                void* stream) {
   if (nblocks <= 0) return TQK_OK;
   if (!blocks || !ops) return fail(TQK_BAD_POINTER, "tqk_block_build: null pointer");
   if (max_batch < 1 || max_batch > 65535) return fail(TQK_BAD_SHAPE, "tqk_block_build: batch %d", max_batch);
-  set_block_smem_attrs();
-  dim3 grid(nblocks, max_batch, 1);
-  prog::k_block_build<<<grid, 256, 64 * 64 * sizeof(double2), as_stream(stream)>>>(blocks, ops);
+  const size_t smem = (64 * 64 >> kBuildSplit) * sizeof(double2);
+  dim3 grid(nblocks, max_batch, 1 << kBuildSplit);
+  prog::k_block_build<<<grid, kBuildThreads, smem, as_stream(stream)>>>(blocks, ops, kBuildSplit);
   return launch_status("tqk_block_build");
 }
 
@@ -721,8 +897,8 @@ extern "C" int tqk_block_unbuild(const tqk_block_desc* blocks, int nblocks, int 
   if (nblocks <= 0) return TQK_OK;
   if (!blocks || !ops) return fail(TQK_BAD_POINTER, "tqk_block_unbuild: null pointer");
   if (max_batch < 1 || max_batch > 65535) return fail(TQK_BAD_SHAPE, "tqk_block_unbuild: batch %d", max_batch);
-  set_block_smem_attrs();
-  dim3 grid(nblocks, max_batch, 1);
-  prog::k_block_unbuild<<<grid, 256, 2 * 64 * 64 * sizeof(float2), as_stream(stream)>>>(blocks, ops);
+  const size_t smem = 2 * (64 * 64 >> kUnbuildSplit) * sizeof(float2);
+  dim3 grid(nblocks, max_batch, 1 << kUnbuildSplit);
+  prog::k_block_unbuild<<<grid, kUnbuildThreads, smem, as_stream(stream)>>>(blocks, ops, kUnbuildSplit);
   return launch_status("tqk_block_unbuild");
 }
