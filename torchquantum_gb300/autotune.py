@@ -115,8 +115,8 @@ def _time_ms(fn, dev, reps: int = 3) -> float:
 def batch_candidates(max_n: int):
     from .batch import BatchConfig
 
-    cands = [BatchConfig(14, 512, 1), BatchConfig(13, 512, 1), BatchConfig(13, 256, 3), BatchConfig(12, 256, 4),
-             BatchConfig(12, 128, 6), BatchConfig(11, 128, 8)]
+    cands = [BatchConfig(14, 512, 1), BatchConfig(14, 256, 1), BatchConfig(13, 256, 3), BatchConfig(13, 128, 3),
+             BatchConfig(12, 128, 3), BatchConfig(11, 128, 3)]
     # a tile wider than every circuit only wastes shared memory
     narrow = [c for c in cands if c.tile_bits <= max(max_n, 11)]
     return narrow or cands[-1:]
@@ -126,7 +126,7 @@ def tune_batch(cb, dev: torch.device, return_states: bool = False):
     """Best ``BatchConfig`` for ``cb`` on ``dev`` (measured, cached)."""
     from .batch import BatchConfig
 
-    key = f"batch|{gpu_key(dev)}|{','.join(map(str, cb.signature()))}|{int(return_states)}"
+    key = f"batch|{gpu_key(dev)}|{','.join(map(str, cb.signature()))}|{int(return_states)}|sweeps"
     hit = lookup(key)
     if hit is not None:
         return BatchConfig(**hit["config"])

@@ -3,8 +3,8 @@
 // A circuit is a list of passes (tqk_batch_plan); a pass holds ops whose target bits lie
 // in a tile of 2^tile_bits amplitudes (tile_mask, tile_bits 10..14 per launch), applied
 // tile by tile in shared memory: gather the tile from the circuit's state, apply every op
-// of the pass, scatter it back.  Circuits with n <= tile_bits are one tile and one pass:
-// their whole life is in shared memory.  Diagonal ops (CZ, CZ ladders) and controls need
+// of the pass in register sweeps, scatter it back.  Circuits with n <= tile_bits are one tile
+// and one pass: their whole life is in shared memory.  Diagonal ops (CZ, CZ ladders) and controls need
 // no tile bit -- their signs split into per-tile constants and tile-local terms -- so the
 // planner gives them to any pass.
 //
@@ -12,9 +12,10 @@
 // pass index by a global counter to persistent CTAs (1..8 per SM), so the tiles of a large
 // circuit's pass run on many SMs at once.  An item of pass p > 0 waits (bounded) for the
 // completion counter of pass p - 1; every item's dependencies are handed out before it,
-// so the earliest unfinished item can always run.  A tile publishes its stores
+// so the earliest unfinished item can always run (a CTA takes its next item while it stores
+// the current one, never before).  A tile publishes its stores
 // (__threadfence) before counting itself done; dependent tiles read through L2
-// (ld.global.cg) since their SM's L1 may hold the previous pass's lines.  Last-pass tiles
+// (cp.async.cg) since their SM's L1 may hold the previous pass's lines.  Last-pass tiles
 // add their <Z> partial (float64 atomics) and the tile that completes a circuit stamps
 // its completion time.
 #include <stdint.h>
@@ -23,6 +24,7 @@
 
 #include "bulk.cuh"
 #include "common.cuh"
+#include "sweep.cuh"
 
 namespace tqk {
 namespace batch {
@@ -129,7 +131,7 @@ __device__ __forceinline__ void cz_terms(uint32_t tmask, uint32_t base, int b0, 
 
 template <int THREADS>
 __device__ void apply_op(const tqk_batch_op& op, float2* amp, int n, int tb, uint32_t tmask, uint32_t base,
-                         const Tabs& tabs, const float2* mats) {
+                         const float2* mats) {
   switch (op.kind) {
     case TQK_B_DENSE1: {
       const int b = n - 1 - op.w0;
@@ -186,145 +188,535 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 
-// THREADS threads per CTA, MINB CTAs per SM for the register budget; the tile holds up
-// to 2^max_tb amplitudes (dynamic shared memory).
-template <int THREADS, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB)
+// ------------------------------------------------------------------ sweeps (tiles of >= 2^10)
+// A pass's ops on a tile of at least 2^10 amplitudes run from registers (sweep.cuh): the ops
+// are taken in order, a sweep ending before the op whose target would be the fifth besides
+// tile bit 0 (or after kSweepOps).  A warp of its own reads the ops ahead of the others, cuts
+// the next sweep and writes it out while they run the current one, so a sweep costs them one
+// barrier, the one after its stores.  (Reading and cutting in every warp between the barriers:
+// 13.3 ms below.)
+// What bounds it: float32 multiply-adds (8 per amplitude and one-qubit op: 4.9 us of the 11 us a
+// 2^13-amplitude item of 18 such ops takes an SM), the two shared-memory crossings of a sweep
+// (2.5 us) and the latency of 12 warps an SM, all the registers allow.  256 circuits of n = 8..20
+// and 2..40 layers, ms: one op per crossing and barrier 11.4 (13-bit tiles, 3 CTAs of 256);
+// sweeps of 16 amplitudes a thread 8.9 (3 x 256), of 32 8.7 (3 x 128).  96 circuits of up to 13
+// qubits, one tile each: 0.58 before, 0.38 now (256 threads, 32 amplitudes).
+constexpr int kSweepMinBits = 10;  // a tile fills at least one warp
+constexpr int kMaxAmpBits = 5;     // 2^AB amplitudes per thread: AB = 5, or 4 where CTAs are many
+constexpr int kSweepOps = 8;
+
+// How a sweep's threads run an op.  Patterns: sets of a thread's registers.
+// Below 16: a 2x2 matrix on slot (code & 7); with SW_SOME on the patterns `reg` only.
+enum { SW_SOME = 8, SW_SIGN = 16, SW_NONE = 17 };
+struct alignas(16) SweepOp {
+  int code;
+  uint32_t reg;    // matrix: patterns it acts on; signs: patterns negated in every thread
+  uint32_t need;   // matrix: thread bits that must be set; signs: if not 0, all set negates ..
+  uint32_t reg2;   // signs: .. these patterns
+  uint32_t lin;    // signs: each of these thread bits negates every pattern
+  uint32_t quad;   // signs: each pair of thread bits (b, b + 1), b in quad, negates every pattern
+  uint16_t side[kMaxAmpBits];  // signs: by slot: thread bits that each negate the patterns with it set
+};
+struct SweepRec {
+  int count;
+  uint16_t rphys[kMaxAmpBits - 1];  // places of the register bits (slots 1 ..)
+  uint32_t lane[32], high[32];   // a thread's tile offset (low half) and its place: by lane, by the bits above
+  SweepOp op[kSweepOps];
+  float4 m[kSweepOps][4];  // (re, re, im, -)
+};
+
+__device__ __forceinline__ uint32_t slot_patterns(int s) {
+  constexpr uint32_t p[kMaxAmpBits] = {0xaaaaaaaau, 0xccccccccu, 0xf0f0f0f0u, 0xff00ff00u, 0xffff0000u};
+  return p[s];
+}
+
+// Bits of v at the bits of mask, moved together.
+__device__ __forceinline__ uint32_t gather_bits(uint32_t v, uint32_t mask) {
+  uint32_t r = 0;
+  for (int j = 0; mask != 0; mask &= mask - 1, ++j) r |= ((v >> (__ffs(mask) - 1)) & 1u) << j;
+  return r;
+}
+
+// The warp that prepares the sweeps.  Lane l holds the op whose index is l modulo 32, of the
+// 32 next ones: its reads were issued several sweeps before it is needed.
+template <int AB>
+struct SweepMaker {
+  const tqk_batch_op* ops;
+  const float2* mats;
+  int num_ops, n, tb;
+  uint32_t tmask, base;
+  int at, mine;  // next op; this lane's
+  tqk_batch_op op;
+  float2 m[4];
+  bool fresh;  // op read, its matrix not yet
+
+  __device__ __forceinline__ void read_op() {
+    if (mine < num_ops) {
+      op = ops[mine];
+      fresh = true;
+    }
+  }
+  __device__ __forceinline__ void start(int lane) {
+    at = 0;
+    mine = lane;
+    fresh = false;
+    read_op();
+  }
+
+  // The ladder's or pair's signs: CZ on (b, b + 1), b in `pairs` (bits of the state).
+  __device__ __forceinline__ void ladder(uint32_t pairs, uint32_t regs, const int (&r)[AB], SweepOp& so) const {
+    const uint32_t in = tmask, out = base;  // base: bits outside the tile
+    const uint32_t lin = gather_bits(in & (((out >> 1) & pairs) ^ ((out & pairs) << 1)), in);
+    const uint32_t quad = gather_bits(in & (in >> 1) & pairs, in);
+    signs((__popc(out & (out >> 1) & pairs) & 1) ? ~0u : 0u, lin, quad, regs, r, so);
+  }
+  // Signs from terms in tile bits: constant patterns, single bits and neighbours (b, b + 1).
+  __device__ __forceinline__ void signs(uint32_t constant, uint32_t lin, uint32_t quad, uint32_t regs,
+                                        const int (&r)[AB], SweepOp& so) const {
+    so.code = SW_SIGN;
+    so.reg = constant;
+    so.need = so.reg2 = 0u;
+    so.lin = lin & ~regs;
+    so.quad = quad & ~regs & ~(regs >> 1);
+    uint32_t side[AB];
+#pragma unroll
+    for (int s = 0; s < AB; ++s) {
+      const uint32_t own = slot_patterns(s), bit = 1u << r[s];
+      if (lin & bit) so.reg ^= own;
+      side[s] = 0;
+      if (quad & bit) {  // (r, r + 1)
+        const uint32_t up = bit << 1;
+        if (regs & up) {
+#pragma unroll
+          for (int t = 0; t < AB; ++t)
+            if (r[t] == r[s] + 1) so.reg ^= own & slot_patterns(t);
+        } else {
+          side[s] |= up;
+        }
+      }
+      if (r[s] > 0 && (quad & (bit >> 1)) && !(regs & (bit >> 1))) side[s] ^= bit >> 1;  // (r - 1, r)
+    }
+#pragma unroll
+    for (int s = 0; s < kMaxAmpBits; ++s) so.side[s] = static_cast<uint16_t>(s < AB ? side[s < AB ? s : 0] : 0u);
+  }
+
+  // CZ of two bits of the state.
+  __device__ __forceinline__ void cz(int b0, int b1, uint32_t regs, const int (&r)[AB], SweepOp& so) const {
+    const bool in0 = (tmask >> b0) & 1u, in1 = (tmask >> b1) & 1u;
+    if ((!in0 && !((base >> b0) & 1u)) || (!in1 && !((base >> b1) & 1u))) {  // never set
+      so.code = SW_NONE;
+      return;
+    }
+    uint32_t pat = ~0u, need = 0;
+    auto take = [&](bool in, int b) {
+      if (!in) return;
+      const int l = local_pos(tmask, b);
+      if (!((regs >> l) & 1u)) need |= 1u << l;
+#pragma unroll
+      for (int s = 0; s < AB; ++s)
+        if (r[s] == l) pat &= slot_patterns(s);
+    };
+    take(in0, b0);
+    take(in1, b1);
+    so.code = SW_SIGN;
+    so.lin = so.quad = 0u;
+#pragma unroll
+    for (int s = 0; s < kMaxAmpBits; ++s) so.side[s] = 0;
+    so.need = need;
+    so.reg = need ? 0u : pat;
+    so.reg2 = pat;
+  }
+
+  __device__ __forceinline__ void make(SweepRec& rec) {
+    const int lane = threadIdx.x & 31;
+    if (fresh) {
+      if (op.kind == TQK_B_DENSE1 || op.kind == TQK_B_CTRL1) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m[e] = __ldg(mats + 4 * static_cast<int64_t>(op.mat) + e);
+      }
+      fresh = false;
+    }
+    int target = 0;  // a tile bit; 0 (always a register) for the others
+    if (mine < num_ops && op.kind <= TQK_B_CTRL1)
+      target = local_pos(tmask, n - 1 - (op.kind == TQK_B_DENSE1 ? op.w0 : op.w1));
+    // by position from `at`: the targets of the ops up to each
+    uint32_t tg = __shfl_sync(0xffffffffu, target > 0 ? 1u << target : 0u, (at + lane) & 31);
+    if (at + lane >= num_ops) tg = 0u;
+#pragma unroll
+    for (int d = 1; d < kSweepOps; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, tg, d);
+      if (lane >= d) tg |= v;
+    }
+    const bool fit = lane < kSweepOps && at + lane < num_ops && __popc(tg) <= AB - 1;
+    const int count = __ffs(~__ballot_sync(0xffffffffu, fit)) - 1;  // leading ops that fit
+    uint32_t regs = __shfl_sync(0xffffffffu, tg, count > 0 ? count - 1 : 0);
+    if (count == 0) regs = 0u;
+    for (int b = tb - 1; __popc(regs) < AB - 1; --b) regs |= 1u << b;  // tb >= 9: never bit 0
+    regs |= 1u;
+    int r[AB];
+    {
+      uint32_t left = regs;
+#pragma unroll
+      for (int s = 0; s < AB; ++s, left &= left - 1) r[s] = __ffs(left) - 1;
+    }
+    const int pos = (lane - at) & 31;
+    if (pos < count) {
+      SweepOp so;
+      if (op.kind <= TQK_B_CTRL1) {
+        so.code = __popc(regs & ((1u << target) - 1u));
+        so.reg = ~0u;
+        so.need = 0u;
+        if (op.kind == TQK_B_CTRL1) {
+          const int cb = n - 1 - op.w0;
+          if (!((tmask >> cb) & 1u)) {
+            if (!((base >> cb) & 1u)) so.code = SW_NONE;  // control outside the tile and clear
+          } else {
+            const int lc = local_pos(tmask, cb);
+            if ((regs >> lc) & 1u) {
+              so.code |= SW_SOME;
+#pragma unroll
+              for (int s = 0; s < AB; ++s)
+                if (r[s] == lc) so.reg = slot_patterns(s);
+            } else {
+              so.need = 1u << lc;
+            }
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) rec.m[pos][e] = make_float4(m[e].x, m[e].x, m[e].y, 0.f);
+      } else if (op.kind == TQK_B_CZ) {
+        cz(n - 1 - op.w0, n - 1 - op.w1, regs, r, so);
+      } else {  // ladder: bits n - 1 - w1 .. n - 1 - w0
+        ladder(((1u << (op.w1 - op.w0)) - 1u) << (n - 1 - op.w1), regs, r, so);
+      }
+      rec.op[pos] = so;
+      mine += 32;
+      read_op();
+    }
+    // The thread bits: of the lowest three lane bits one in each class (bit - 1) mod 3 (the 16-byte
+    // pieces of 8 lanes then lie in different banks), the others ascending.
+    uint32_t free = ((1u << tb) - 1u) & ~regs, v = 0, hv = 0;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const uint32_t cls = j < 3 ? free & (0x2492u << j) : 0u, bit = cls ? cls & (~cls + 1u) : free & (~free + 1u);
+      if ((lane >> j) & 1) v |= bit;
+      free ^= bit;
+    }
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const uint32_t bit = free & (~free + 1u);
+      if ((lane >> j) & 1) hv |= bit;
+      free ^= bit;
+    }
+    rec.lane[lane] = v | sweep::swz(v) << 16;
+    rec.high[lane] = hv | sweep::swz(hv) << 16;
+    if (lane == 0) {
+      rec.count = count;
+#pragma unroll
+      for (int s = 1; s < AB; ++s) rec.rphys[s - 1] = static_cast<uint16_t>(sweep::swz(1u << r[s]));
+    }
+    at += count;
+  }
+};
+
+// Negate the register patterns of mask.
+template <int AB>
+__device__ __forceinline__ void flip_patterns(uint32_t mask) {
+  if (mask == 0) return;
+  sweep::unroll<1 << AB>([&](auto q) {
+    const uint32_t s = (mask << (31 - q.value)) & 0x80000000u;
+    f2::Psi::flip<q.value>((static_cast<f2::pair>(s) << 32) | s);
+  });
+}
+
+template <int AB, int S, bool MASK>
+__device__ __forceinline__ void dense_rows(const float4* m4, uint32_t rmask) {
+  f2::Factor m[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(m4 + e);
+    m[e] = {v.x, __uint_as_float(static_cast<uint32_t>(v.y))};
+  }
+  if constexpr (S < AB)
+    sweep::each_pair<S, MASK, 1 << AB>(rmask, [&](auto q, auto u) { f2::Psi::dense2<q.value, u.value>(m); });
+}
+
+// Run a sweep on the tile (all threads but the preparing warp).
+template <int THREADS, int AB>
+__device__ __forceinline__ void run_sweep(const SweepRec& rec, float2* amp, int tb) {
+  const int count = rec.count;
+  // read again at each use: kept, the 16 places are registers that the amplitudes need
+  auto places = [&](uint16_t (&rphys)[AB - 1]) {
+#pragma unroll
+    for (int j = 0; j < AB - 1; ++j) rphys[j] = *const_cast<const volatile uint16_t*>(rec.rphys + j);
+  };
+  const uint32_t slots = 1u << (tb - AB);  // threads' worth of amplitudes
+#pragma unroll 1
+  for (uint32_t vt = threadIdx.x; vt < slots; vt += THREADS) {  // uniform for the warp
+    const uint32_t e = rec.lane[threadIdx.x & 31] ^ rec.high[vt >> 5], tl = e & 0xffffu;
+    {
+      uint16_t rphys[AB - 1];
+      places(rphys);
+      sweep::load_regs<f2::Psi>(rphys, amp, e >> 16);
+    }
+#pragma unroll 1
+    for (int j = 0; j < count; ++j) {
+      const SweepOp& so = rec.op[j];
+      const int4 head = *reinterpret_cast<const int4*>(&so);
+      const int code = head.x;
+      const uint32_t need = static_cast<uint32_t>(head.z);
+      if (code < SW_SIGN) {
+        if ((tl & need) == need) {
+          const float4* m4 = rec.m[j];
+          switch (code) {
+            case 0: dense_rows<AB, 0, false>(m4, 0u); break;
+            case 1: dense_rows<AB, 1, false>(m4, 0u); break;
+            case 2: dense_rows<AB, 2, false>(m4, 0u); break;
+            case 3: dense_rows<AB, 3, false>(m4, 0u); break;
+            case 4: dense_rows<AB, 4, false>(m4, 0u); break;
+            case SW_SOME | 0: dense_rows<AB, 0, true>(m4, so.reg); break;
+            case SW_SOME | 1: dense_rows<AB, 1, true>(m4, so.reg); break;
+            case SW_SOME | 2: dense_rows<AB, 2, true>(m4, so.reg); break;
+            case SW_SOME | 3: dense_rows<AB, 3, true>(m4, so.reg); break;
+            default: dense_rows<AB, 4, true>(m4, so.reg); break;
+          }
+        }
+        __syncwarp();
+      } else if (code == SW_SIGN) {
+        uint32_t mask = so.reg;
+        if ((__popc(tl & so.lin) + __popc(tl & (tl >> 1) & so.quad)) & 1) mask = ~mask;
+        if (so.need != 0u && (tl & so.need) == so.need) mask ^= so.reg2;
+#pragma unroll
+        for (int s = 0; s < AB; ++s)
+          if (__popc(tl & so.side[s]) & 1) mask ^= slot_patterns(s);
+        flip_patterns<AB>(mask);
+      }
+    }
+    uint16_t rphys[AB - 1];
+    places(rphys);
+    sweep::store_regs<f2::Psi>(rphys, amp, e >> 16);
+  }
+}
+
+// The two sides of an item's sweeps, from before the barrier that ends the tile's load.  Calls,
+// not inlined: each side has the registers to itself.
+template <int AB>
+__device__ __noinline__ void make_sweeps(SweepRec* rec, const tqk_batch_op* ops, int num_ops, const float2* mats,
+                                         int n, uint32_t tmask, uint32_t base) {
+  SweepMaker<AB> s;
+  s.ops = ops;
+  s.mats = mats;
+  s.num_ops = num_ops;
+  s.n = n;
+  s.tb = __popc(tmask);
+  s.tmask = tmask;
+  s.base = base;
+  s.start(threadIdx.x & 31);
+  s.make(rec[0]);
+  __syncthreads();
+#pragma unroll 1
+  for (int sw = 0; rec[sw & 1].count != 0; ++sw) {
+    s.make(rec[(sw + 1) & 1]);
+    __syncthreads();
+  }
+}
+
+template <int THREADS, int AB>
+__device__ __noinline__ void run_sweeps(const SweepRec* rec, float2* amp, int tb) {
+  TQK_AMPLITUDE_REGISTERS_32;
+  __syncthreads();
+#pragma unroll 1
+  for (int sw = 0; rec[sw & 1].count != 0; ++sw) {
+    run_sweep<THREADS, AB>(rec[sw & 1], amp, tb);
+    __syncthreads();
+  }
+}
+
+// Shared-memory place of tile amplitude l: tiles that run in sweeps are swizzled.
+__device__ __forceinline__ uint32_t place(uint32_t l, int tb) { return tb >= kSweepMinBits ? sweep::swz(l) : l; }
+
+// An item as its CTA works on it.
+struct Work {
+  int valid;  // 0: no more items; -1: a plan made for a larger tile
+  int circuit, pass, flags, num_ops, n, z_wire, prev_tiles, ntiles;
+  uint32_t tmask, base;  // bits of the tile; value of the others
+  const tqk_batch_op* ops;
+  float2* state;  // NULL: the circuit has none
+};
+
+// The next item into w and its tables into tabs (one warp).
+__device__ __noinline__ void fetch_item(Work& w, Tabs& tabs, const tqk_batch_circuit* circ, const tqk_batch_op* ops,
+                                        const tqk_batch_pass* passes, const tqk_batch_item* items, long long n_items,
+                                        float2* states, int* counter, int max_tb) {
+  const int lane = threadIdx.x & 31;
+  int i = lane == 0 ? atomicAdd(counter, 1) : 0;
+  i = __shfl_sync(0xffffffffu, i, 0);
+  if (i >= n_items) {
+    if (lane == 0) w.valid = 0;
+    return;
+  }
+  const tqk_batch_item it = items[i];
+  const tqk_batch_pass P = passes[it.pass];
+  const tqk_batch_circuit C = circ[it.circuit];
+  const int n = C.n, tb = __popc(P.tile_mask);
+  const uint32_t omask = (n >= 32 ? 0xffffffffu : ((1u << n) - 1u)) & ~P.tile_mask;
+  uint32_t base = 0;
+  for (int b = 0, j = 0; b < n; ++b) {
+    if (!((omask >> b) & 1u)) continue;
+    if ((it.tile >> j) & 1) base |= 1u << b;
+    ++j;
+  }
+  // deposit tables of the tile bits: lo[x] from the first 7, hi[x] from the others (lane: x's
+  // low 5 bits)
+  uint32_t low = 0, add[4] = {0u, 0u, 0u, 0u}, low2 = 0;
+  uint32_t left = P.tile_mask;
+  for (int j = 0; j < 14 && left != 0; ++j, left &= left - 1) {
+    const uint32_t bit = left & (~left + 1u);
+    const int k = j % 7;
+    if (k < 5) {
+      if ((lane >> k) & 1) (j < 7 ? low : low2) |= bit;
+    } else {
+      add[(j < 7 ? 0 : 2) + k - 5] = bit;
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    tabs.lo[32 * x + lane] = low | (x & 1 ? add[0] : 0u) | (x & 2 ? add[1] : 0u);
+    tabs.hi[32 * x + lane] = low2 | (x & 1 ? add[2] : 0u) | (x & 2 ? add[3] : 0u);
+  }
+  if (lane == 0) {
+    w.valid = tb > max_tb || tb < 1 ? -1 : 1;
+    w.circuit = it.circuit;
+    w.pass = it.pass;
+    w.flags = P.flags;
+    w.num_ops = P.num_ops;
+    w.n = n;
+    w.z_wire = C.z_wire;
+    w.prev_tiles = (P.flags & kFirst) ? 0 : 1 << (n - __popc(passes[it.pass - 1].tile_mask));
+    w.ntiles = 1 << (n - tb);
+    w.tmask = P.tile_mask;
+    w.base = base;
+    w.ops = ops + P.first_op;
+    w.state = C.state_off >= 0 ? states + C.state_off : nullptr;
+  }
+}
+
+// THREADS threads per CTA and a warp that prepares (the next item, its sweeps), MINB CTAs per
+// SM for the register budget; the tile holds up to 2^max_tb amplitudes (dynamic shared
+// memory).
+template <int THREADS, int MINB, int AB>
+__global__ void __launch_bounds__(THREADS + 32, MINB)
     k_batch(const tqk_batch_circuit* circ, int ncirc, const tqk_batch_op* ops, const tqk_batch_pass* passes,
             const tqk_batch_item* items, long long n_items, const float2* mats, float2* states, int write_states,
             double* z_out, int* pass_done, unsigned long long* t_done, int* counter, int* status, int max_tb) {
   extern __shared__ float4 amp_raw[];  // 16-byte aligned: ops use float4 accesses
   float2* amp = reinterpret_cast<float2*>(amp_raw);
-  __shared__ Tabs tabs;
-  __shared__ long long s_i;
+  __shared__ Tabs tab_buf[2];
+  __shared__ Work work[2];
+  __shared__ SweepRec rec[2];
   __shared__ double red[THREADS / 32];
-  __shared__ uint64_t full;  // bulk-copy (TMA) tile loads complete here
-  __shared__ int abort_flag;
+  const bool maker = threadIdx.x >= THREADS;  // the warp that prepares
+  const uint32_t tid = threadIdx.x;
   if (t_done != nullptr && blockIdx.x == 0 && threadIdx.x == 0) t_done[ncirc] = global_ns();
-  if (threadIdx.x == 0) {
-    bulk::mbar_init(&full);
-    abort_flag = 0;
-  }
-  uint32_t use = 0;  // loads completed on `full` so far
-  for (;;) {
-    if (threadIdx.x == 0) s_i = atomicAdd(counter, 1);
-    __syncthreads();
-    const long long i = s_i;
-    __syncthreads();
-    if (i >= n_items) break;
-    const tqk_batch_item it = items[i];
-    const tqk_batch_circuit C = circ[it.circuit];
-    const tqk_batch_pass P = passes[it.pass];
-    const int n = C.n;
-    const uint32_t tmask = P.tile_mask;
-    const int tb = __popc(tmask);
-    if (tb > max_tb || tb < 1) {  // a plan made for a larger tile: record and skip the item
+  if (maker) fetch_item(work[0], tab_buf[0], circ, ops, passes, items, n_items, states, counter, max_tb);
+  __syncthreads();
+  for (int cur = 0;; cur ^= 1) {
+    const Work& W = work[cur];
+    const Tabs& tabs = tab_buf[cur];
+    if (W.valid == 0) break;
+    if (W.valid < 0) {  // record and skip the item
       if (threadIdx.x == 0) {
         atomicExch(status, TQK_BAD_SHAPE);
-        atomicAdd(pass_done + it.pass, 1);
+        atomicAdd(pass_done + W.pass, 1);
       }
+      __syncthreads();  // the other slot's item is done with
+      if (maker) fetch_item(work[cur ^ 1], tab_buf[cur ^ 1], circ, ops, passes, items, n_items, states, counter, max_tb);
       __syncthreads();
       continue;
     }
-    const int tsz = 1 << tb;
-    const int ntiles = 1 << (n - tb);
-    const uint32_t omask = (n >= 32 ? 0xffffffffu : ((1u << n) - 1u)) & ~tmask;
-    float2* st = states + (C.state_off >= 0 ? C.state_off : 0);
-    if (!(P.flags & kFirst) && threadIdx.x == 0) {  // every tile of the previous pass must be stored
-      const int prev_tiles = 1 << (n - __popc(passes[it.pass - 1].tile_mask));
-      const volatile int* d = pass_done + it.pass - 1;
-      const long long t0 = clock64();
-      while (*d < prev_tiles) {
-        if (clock64() - t0 > kWaitCycles) {
-          atomicExch(status, TQK_TIMEOUT);
-          break;
+    const int tb = __popc(W.tmask);
+    const uint32_t tsz = 1u << tb;
+    if (W.prev_tiles > 0) {  // every tile of the previous pass must be stored
+      if (threadIdx.x == 0) {
+        const volatile int* d = pass_done + W.pass - 1;
+        const long long t0 = clock64();
+        while (*d < W.prev_tiles) {
+          if (clock64() - t0 > kWaitCycles) {
+            atomicExch(status, TQK_TIMEOUT);
+            break;
+          }
         }
-      }
-      __threadfence();
-    }
-    for (int t = threadIdx.x; t < 256; t += THREADS) {  // deposit tables of the tile bits
-      const int part = t >> 7, x = t & 127;
-      uint32_t v = 0;
-      int j = 0;
-      for (int b = 0; b < n; ++b) {
-        if (!((tmask >> b) & 1u)) continue;
-        const int k = j++ - 7 * part;
-        if (k >= 0 && k < 7 && ((x >> k) & 1)) v |= 1u << b;
-      }
-      (part ? tabs.hi : tabs.lo)[x] = v;
-    }
-    uint32_t base = 0;
-    for (int b = 0, j = 0; b < n; ++b) {
-      if (!((omask >> b) & 1u)) continue;
-      if ((it.tile >> j) & 1) base |= 1u << b;
-      ++j;
-    }
-    __syncthreads();
-    // Runs of 32 amplitudes (tile bits 0-4 are address bits 0-4) or the whole tile when it
-    // is smaller: contiguous in HBM, moved by the bulk-copy engine.
-    const int run = tsz < 32 ? tsz : 32;
-    const int nruns = tsz / run;
-    if (P.flags & kFirst) {
-      for (int l = threadIdx.x; l < tsz; l += THREADS)
-        amp[l] = make_float2((base == 0u && l == 0) ? 1.f : 0.f, 0.f);
-    } else {
-      if (threadIdx.x == 0) bulk::mbar_expect(&full, static_cast<uint32_t>(tsz * sizeof(float2)));
-      __syncthreads();
-      asm volatile("fence.proxy.async.global;" ::: "memory");  // the dependency flag was read by the generic proxy
-      for (int r = threadIdx.x; r < nruns; r += THREADS)
-        bulk::bulk_load(amp + r * run, st + base + dep(tabs, static_cast<uint32_t>(r * run)),
-                        static_cast<uint32_t>(run * sizeof(float2)), &full);
-      if (threadIdx.x == 0 && !bulk::mbar_wait(&full, use & 1u)) {
-        atomicExch(status, TQK_TIMEOUT);
-        abort_flag = 1;
-      }
-      ++use;
-    }
-    __syncthreads();
-    if (abort_flag) break;  // uniform: a tile load never landed
-    for (int oi = 0; oi < P.num_ops; ++oi) {
-      apply_op<THREADS>(ops[P.first_op + oi], amp, n, tb, tmask, base, tabs, mats);
-      __syncthreads();
-    }
-    if (P.flags & kLast) {
-      const int zbit = n - 1 - C.z_wire;
-      double zacc = 0.0;
-      for (int l = threadIdx.x; l < tsz; l += THREADS) {
-        const float2 a = amp[l];
-        const double p2 = static_cast<double>(a.x) * a.x + static_cast<double>(a.y) * a.y;
-        zacc += (((base + dep(tabs, l)) >> zbit) & 1u) ? -p2 : p2;
-      }
-      for (int o = 16; o > 0; o >>= 1) zacc += __shfl_xor_sync(0xffffffffu, zacc, o);
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = zacc;
-    }
-    if (((P.flags & kLast) == 0 || write_states) && C.state_off >= 0) {
-      bulk::fence_async_smem();  // the ops' shared-memory writes, visible to the bulk stores
-      __syncthreads();
-      bool mine = false;
-      for (int r = threadIdx.x; r < nruns; r += THREADS) {
-        bulk::bulk_store(st + base + dep(tabs, static_cast<uint32_t>(r * run)), amp + r * run,
-                         static_cast<uint32_t>(run * sizeof(float2)));
-        mine = true;
-      }
-      if (mine) {
-        bulk::bulk_commit();
-        bulk::bulk_wait_all();  // stored in HBM / L2 before the tile counts as done
-        asm volatile("fence.proxy.async.global;" ::: "memory");
-      }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      if (P.flags & kLast) {
-        double sum = 0.0;
-        for (int w = 0; w < THREADS / 32; ++w) sum += red[w];
-        atomicAdd(z_out + it.circuit, sum);
         __threadfence();
       }
-      const int old = atomicAdd(pass_done + it.pass, 1);
-      if ((P.flags & kLast) && old == ntiles - 1 && t_done != nullptr) t_done[it.circuit] = global_ns();
+      __syncthreads();
+    }
+    if (maker) {
+      if (tb >= kSweepMinBits) {
+        make_sweeps<AB>(rec, W.ops, W.num_ops, mats, W.n, W.tmask, W.base);
+      } else {
+        for (int oi = 0; oi <= W.num_ops; ++oi) __syncthreads();
+      }
+      fetch_item(work[cur ^ 1], tab_buf[cur ^ 1], circ, ops, passes, items, n_items, states, counter, max_tb);
+    } else {
+      if (W.flags & kFirst) {
+        for (uint32_t l = tid; l < tsz; l += THREADS)
+          amp[place(l, tb)] = make_float2((W.base == 0u && l == 0) ? 1.f : 0.f, 0.f);
+      } else if (2u * tid < tsz) {
+        // 16-byte pieces through L2 (another SM may have stored them: .cg skips this SM's L1);
+        // tile bits 0-4 are address bits 0-4, so a warp's pieces are 256-byte runs
+        // (both places are linear: that of tile index l + k is the sum or XOR of theirs)
+        const float2* src = W.state + W.base + dep(tabs, 2u * tid);
+        const uint32_t dst = place(2u * tid, tb);
+        for (uint32_t k = 0; k < tsz; k += 2u * THREADS)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bulk::smem_addr(amp + (dst ^ place(k, tb)))),
+                       "l"(src + dep(tabs, k))
+                       : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+      }
+      if (tb >= kSweepMinBits) {
+        run_sweeps<THREADS, AB>(rec, amp, tb);
+      } else {
+        __syncthreads();
+        for (int oi = 0; oi < W.num_ops; ++oi) {
+          apply_op<THREADS>(W.ops[oi], amp, W.n, tb, W.tmask, W.base, mats);
+          __syncthreads();
+        }
+      }
+      if (W.flags & kLast) {
+        const int zbit = W.n - 1 - W.z_wire;
+        const bool in = (W.tmask >> zbit) & 1u;
+        const int zl = local_pos(W.tmask, zbit);
+        const uint32_t out = (W.base >> zbit) & 1u;
+        double zacc = 0.0;
+        for (uint32_t l = tid; l < tsz; l += THREADS) {
+          const float2 a = amp[place(l, tb)];
+          const bool minus = in ? (l >> zl) & 1u : out;
+          zacc = fma(static_cast<double>(a.x), static_cast<double>(minus ? -a.x : a.x), zacc);
+          zacc = fma(static_cast<double>(a.y), static_cast<double>(minus ? -a.y : a.y), zacc);
+        }
+        for (int o = 16; o > 0; o >>= 1) zacc += __shfl_xor_sync(0xffffffffu, zacc, o);
+        if ((tid & 31) == 0) red[tid >> 5] = zacc;
+      }
+      if (((W.flags & kLast) == 0 || write_states) && W.state != nullptr && 2u * tid < tsz) {
+        float2* dst = W.state + W.base + dep(tabs, 2u * tid);
+        const uint32_t src = place(2u * tid, tb);
+        for (uint32_t k = 0; k < tsz; k += 2u * THREADS)
+          *reinterpret_cast<float4*>(dst + dep(tabs, k)) =
+              *reinterpret_cast<const float4*>(amp + (src ^ place(k, tb)));
+      }
+      __threadfence();  // stored before the tile counts as done
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+      if (W.flags & kLast) {
+        double sum = 0.0;
+        for (int w = 0; w < THREADS / 32; ++w) sum += red[w];
+        atomicAdd(z_out + W.circuit, sum);
+        __threadfence();
+      }
+      const int old = atomicAdd(pass_done + W.pass, 1);
+      if ((W.flags & kLast) && old == W.ntiles - 1 && t_done != nullptr) t_done[W.circuit] = global_ns();
+    }
   }
 }
 
@@ -451,13 +843,14 @@ extern "C" int64_t tqk_batch_items(const tqk_batch_circuit* circuits, int ncirc,
 }
 
 namespace {
-// Kernel variants: (threads per CTA, CTAs per SM the register budget is sized for).
-template <int THREADS, int MINB>
+// Kernel variants: (threads per CTA, CTAs per SM the register budget is sized for, amplitudes
+// per thread as a power of two).
+template <int THREADS, int MINB, int AB>
 int launch_batch(const tqk_batch_circuit* circuits, int ncirc, const tqk_batch_op* ops, const tqk_batch_pass* passes,
                  const tqk_batch_item* items, int64_t n_items, const void* mats, void* states, int write_states,
                  double* z_out, int* pass_done, uint64_t* t_done, int* counter, int* status, int tile_bits,
                  int ctas_per_sm, cudaStream_t stream) {
-  auto kern = batch::k_batch<THREADS, MINB>;
+  auto kern = batch::k_batch<THREADS, MINB, AB>;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -471,11 +864,11 @@ int launch_batch(const tqk_batch_circuit* circuits, int ncirc, const tqk_batch_o
     attr_set[dev] = 1;
   }
   int fit = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, THREADS, smem) != cudaSuccess || fit < 1) fit = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, THREADS + 32, smem) != cudaSuccess || fit < 1) fit = 1;
   const int per_sm = ctas_per_sm < fit ? ctas_per_sm : fit;
   const int64_t slots = static_cast<int64_t>(sms) * per_sm;
   const int grid = static_cast<int>(n_items < slots ? n_items : slots);
-  kern<<<grid, THREADS, smem, stream>>>(circuits, ncirc, ops, passes, items, n_items,
+  kern<<<grid, THREADS + 32, smem, stream>>>(circuits, ncirc, ops, passes, items, n_items,
                                         static_cast<const float2*>(mats), static_cast<float2*>(states), write_states,
                                         z_out, pass_done, reinterpret_cast<unsigned long long*>(t_done), counter,
                                         status, tile_bits);
@@ -505,11 +898,11 @@ extern "C" int tqk_batch_run(const tqk_batch_circuit* circuits, int ncirc, const
                        t_done, counter, status, cfg.tile_bits, cfg.ctas_per_sm, s
   switch (cfg.threads) {
     case 512:
-      return launch_batch<512, 1>(TQK_BATCH_ARGS);
+      return launch_batch<512, 1, 4>(TQK_BATCH_ARGS);
     case 256:
-      return cfg.ctas_per_sm >= 4 ? launch_batch<256, 4>(TQK_BATCH_ARGS) : launch_batch<256, 2>(TQK_BATCH_ARGS);
+      return cfg.ctas_per_sm >= 2 ? launch_batch<256, 3, 4>(TQK_BATCH_ARGS) : launch_batch<256, 1, 5>(TQK_BATCH_ARGS);
     case 128:
-      return launch_batch<128, 8>(TQK_BATCH_ARGS);
+      return cfg.ctas_per_sm >= 4 ? launch_batch<128, 6, 4>(TQK_BATCH_ARGS) : launch_batch<128, 3, 5>(TQK_BATCH_ARGS);
     default:
       return fail(TQK_BAD_SHAPE, "%s: threads %d (128, 256 or 512)", what, cfg.threads);
   }

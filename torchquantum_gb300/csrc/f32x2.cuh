@@ -32,8 +32,10 @@ __device__ __forceinline__ pair make(float lo, float hi) {
   return r;
 }
 
-// Once per kernel, before any other use.
+// Once per kernel, before any other use: for 16 amplitudes of two states and sums, or for
+// 32 of one state.
 #define TQK_AMPLITUDE_REGISTERS asm volatile(".reg .b64 ta<16>, tb<16>, gr<4>, hr;\n .reg .f32 gi<4>, hi;")
+#define TQK_AMPLITUDE_REGISTERS_32 asm volatile(".reg .b64 ta<32>;")
 
 // P: 'a' or 'b'.  Load / store the amplitudes Q, Q + 1 (16 bytes of shared memory).
 #define TQK_DEFINE_REGS(NAME, P)                                                                                  \
@@ -51,6 +53,11 @@ __device__ __forceinline__ pair make(float lo, float hi) {
       asm volatile(                                                                                               \
           "{\n .reg .b64 t;\n mov.b64 t, t" P "%0;\n mov.b64 t" P "%0, t" P "%1;\n mov.b64 t" P "%1, t;\n}" ::"n"(Q), \
           "n"(U));                                                                                                \
+    }                                                                                                             \
+    /* exclusive or with a sign pattern */                                                                        \
+    template <int Q>                                                                                              \
+    static __device__ __forceinline__ void flip(pair s) {                                                         \
+      asm volatile("xor.b64 t" P "%0, t" P "%0, %1;" ::"n"(Q), "l"(s));                                            \
     }                                                                                                             \
     /* (Q, U) <- real 2x2 */                                                                                      \
     template <int Q, int U>                                                                                       \

@@ -27,11 +27,6 @@
 //   (32 amplitudes per thread: 3 % faster forward, 10 % slower in reverse; 4 CTAs of 64
 //   registers: 10 % slower forward.)
 //
-// Shared memory layout: amplitude l of the tile lives at l ^ (g(l) << 1), g(l) the XOR of
-// the 3-bit fields of l >> 4: linear over XOR, keeps 16-byte pairs (bit 0) whole, and makes
-// the 16-byte accesses of 8 lanes conflict free whenever the three lowest lane bits map
-// to tile bits of different classes (bit - 1) mod 3, which the host picks where it can.
-//
 // The reverse pass holds the psi and lam tiles of the same amplitudes and walks the run
 // backwards: psi <- U^H psi, lam <- U^H lam and, for ops with a cotangent slot,
 // sum lam_in conj(psi_out): float32 over a thread's amplitudes and a warp, float64 beyond.
@@ -41,10 +36,12 @@
 
 #include "bulk.cuh"
 #include "common.cuh"
-#include "f32x2.cuh"
+#include "sweep.cuh"
 
 namespace tqk {
 namespace tiled {
+
+using namespace sweep;
 
 constexpr int kAmpBits = 4;  // 2^4 amplitudes per thread
 constexpr int kAmps = 1 << kAmpBits;
@@ -105,10 +102,6 @@ struct Params {
   Sweep sweeps[TQK_STAGED_MAX_OPS];
   SOp ops[TQK_STAGED_MAX_OPS];
 };
-
-__host__ __device__ __forceinline__ uint32_t swz(uint32_t l) {
-  return l ^ ((((l >> 4) ^ (l >> 7) ^ (l >> 10)) & 7u) << 1);
-}
 
 // t deposited into the bits of mask
 __device__ __forceinline__ uint64_t deposit(uint64_t t, uint64_t mask) {
@@ -180,39 +173,6 @@ __device__ __forceinline__ uint32_t thread_offset(const volatile uint32_t* tab, 
   return tab[s * kTabEntries + (threadIdx.x & 31)] ^ tab[s * kTabEntries + 32 + (threadIdx.x >> 5)];
 }
 
-// Compile-time loop: f(Const<0>) ... f(Const<N - 1>).
-template <int I>
-struct Const {
-  static constexpr int value = I;
-};
-template <int N, int I = 0, typename F>
-__device__ __forceinline__ void unroll(const F& f) {
-  if constexpr (I < N) {
-    f(Const<I>{});
-    unroll<N, I + 1>(f);
-  }
-}
-
-// A thread's amplitudes by register pattern (bit 0 = index bit 0, bit j = slot j), between
-// a tile in shared memory and the named registers of A.  Pair q: slots 1..3 as its bits.
-__device__ __forceinline__ uint32_t piece(const Sweep& s, int q) {
-  uint32_t o = 0;
-#pragma unroll
-  for (int j = 0; j < kAmpBits - 1; ++j)
-    if ((q >> j) & 1) o ^= s.rphys[j];
-  return o;
-}
-template <typename A>
-__device__ __forceinline__ void load_regs(const Sweep& s, const float2* tile, uint32_t tp) {
-  const uint32_t at = bulk::smem_addr(tile);
-  unroll<kAmps / 2>([&](auto q) { A::template load<2 * q.value>(at + 8 * (tp ^ piece(s, q.value))); });
-}
-template <typename A>
-__device__ __forceinline__ void store_regs(const Sweep& s, float2* tile, uint32_t tp) {
-  const uint32_t at = bulk::smem_addr(tile);
-  unroll<kAmps / 2>([&](auto q) { A::template store<2 * q.value>(at + 8 * (tp ^ piece(s, q.value))); });
-}
-
 // ------------------------------------------------------------------ op tables
 // What the op loop reads of an op, in shared memory.
 struct Decoded {
@@ -260,18 +220,9 @@ struct Source {
 };
 
 // ------------------------------------------------------------------ ops on one state
-// The pairs of register patterns that differ in slot S; MASK: those in rmask only.
-template <int S, bool MASK, typename F>
-__device__ __forceinline__ void each_pair(uint32_t rmask, const F& f) {
-  unroll<kAmps>([&](auto q) {
-    if constexpr (!((q.value >> S) & 1))
-      if (!MASK || ((rmask >> q.value) & 1u)) f(q, Const<q.value | (1 << S)>{});
-  });
-}
-
 template <int S, bool MASK, typename A>
 __device__ __forceinline__ void x_slot(uint32_t rmask) {
-  each_pair<S, MASK>(rmask, [&](auto q, auto u) { A::template swap<q.value, u.value>(); });
+  each_pair<S, MASK, kAmps>(rmask, [&](auto q, auto u) { A::template swap<q.value, u.value>(); });
 }
 
 // Diagonal ops: entry-index bits that do not vary over the thread's registers, the bits
@@ -321,7 +272,7 @@ template <int S, bool REAL, bool MASK>
 __device__ __forceinline__ void fwd_dense(int j, const Source& src) {
   f2::Factor m[4];
   src.matrix(j, m);
-  each_pair<S, MASK>(MASK ? src.p.ops[j].rmask : 0u, [&](auto q, auto u) {
+  each_pair<S, MASK, kAmps>(MASK ? src.p.ops[j].rmask : 0u, [&](auto q, auto u) {
     if constexpr (REAL) f2::Psi::real2<q.value, u.value>(m);
     else f2::Psi::dense2<q.value, u.value>(m);
   });
@@ -385,14 +336,14 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_tiled(const __grid_constant_
       const Sweep& sw = p.sweeps[s];
       const uint32_t e = thread_offset(tab, s);
       const uint32_t tl = e & 0xffffu;
-      load_regs<f2::Psi>(sw, tile, e >> 16);
+      load_regs<f2::Psi>(sw.rphys, tile, e >> 16);
 #pragma unroll 1
       for (int j = sw.first; j < sw.first + sw.count; ++j) {
         const Decoded d = dec[j];
         if ((base & d.omask) != d.oval || (tl & d.tmask) != d.tval) continue;
         apply_fwd(j, d.go, src, tl, base);
       }
-      store_regs<f2::Psi>(sw, tile, thread_offset(tab, s) >> 16);
+      store_regs<f2::Psi>(sw.rphys, tile, thread_offset(tab, s) >> 16);
       __syncthreads();
     }
     store_tile(p, frame(p, base), p.psi, tile);
@@ -407,7 +358,7 @@ template <int S, bool GRAD, bool REAL, bool MASK>
 __device__ __forceinline__ void adj_dense(int j, const Source& src) {
   f2::Factor m[4];
   src.matrix(j, m);
-  each_pair<S, MASK>(MASK ? src.p.ops[j].rmask : 0u, [&](auto q, auto u) {
+  each_pair<S, MASK, kAmps>(MASK ? src.p.ops[j].rmask : 0u, [&](auto q, auto u) {
     constexpr int Q = q.value, U = u.value;
     if constexpr (REAL) f2::Psi::real2<Q, U>(m);
     else f2::Psi::dense2<Q, U>(m);
@@ -547,8 +498,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
       const Sweep& sw = p.sweeps[s];
       const uint32_t e = thread_offset(tab, s);
       const uint32_t tl = e & 0xffffu;
-      load_regs<f2::Psi>(sw, ps, e >> 16);
-      load_regs<f2::Lam>(sw, ls, e >> 16);
+      load_regs<f2::Psi>(sw.rphys, ps, e >> 16);
+      load_regs<f2::Lam>(sw.rphys, ls, e >> 16);
 #pragma unroll 1
       for (int j = sw.first + sw.count - 1; j >= sw.first; --j) {
         const Decoded d = dec[j];
@@ -575,8 +526,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
         if ((lane & 3) == 0) gw[lane >> 2] = sum;
       }
       const uint32_t tp = thread_offset(tab, s) >> 16;
-      store_regs<f2::Psi>(sw, ps, tp);
-      store_regs<f2::Lam>(sw, ls, tp);
+      store_regs<f2::Psi>(sw.rphys, ps, tp);
+      store_regs<f2::Lam>(sw.rphys, ls, tp);
       __syncthreads();
     }
     {
