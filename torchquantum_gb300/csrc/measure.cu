@@ -256,11 +256,19 @@ __global__ void __launch_bounds__(kFinishThreads) k_expval_finish(const double* 
 // CTA: sixteen warps and three stages.  At the top of each iteration every thread issues
 // its 16-byte cp.async pieces of the coset two iterations ahead into the stage the previous
 // iteration finished reading, and arrives on that stage's full mbarrier once they land;
-// then all wait for the current stage.  Expvals: each warp sums its segment of the strings'
-// pair visits in float32, the CTA reduces in float64 and writes one partial per (coset,
-// string); the partials are summed per row in a fixed order (k_expval_finish).  Backward
-// seed: each thread forms sum_s c_s (P_s psi)_u for two amplitudes and stores them to the
-// output row (added to what is there for groups after the first).
+// then all wait for the current stage.  A thread owns eight amplitude pairs of a full stage.
+// Expvals: it keeps them in registers and visits each string's partners in the stage (from one
+// side only where it can), float32 sums over its pairs and its warp; the CTA reduces in float64
+// and writes one partial per (coset, string); the partials are summed per row in a fixed order
+// (k_expval_finish).  Backward seed: it forms sum_s c_s (P_s psi)_u for its pairs and stores
+// them to the output row, added to what earlier groups left there, which it reads before it
+// waits for the stage.
+// What bounds it: DRAM moves a 64 KB stage in 2800 cycles an SM, the strings' partner reads take
+// 2500 to 4600 of shared memory and about as many issue cycles; they overlap in part.  n = 22,
+// 4 rows, 24 strings: expvals 201 -> 152 us (three groups; 60 at the DRAM rate), seed 369 -> 244 us
+// (158 at the DRAM rate); before, each warp took a segment of the strings' visits (two stage
+// reads, a shift, a population count and a flip each), the seed read the earlier groups' output
+// after its sums, and every thread divided for its coset.
 // Every mbarrier wait is bounded: on expiry the CTA records TQK_TIMEOUT in the status
 // word, stops issuing copies and waiting, writes NaN expval partials (the seed skips its
 // stores), waits (bounded) for its copies in flight and exits.
@@ -285,8 +293,6 @@ struct CosetParams {
   uint32_t xs[kMaxStringsPerPass], gam[kMaxStringsPerPass], zh[kMaxStringsPerPass];
   uint32_t fl[kMaxStringsPerPass];   // constant sign bit (expvals: ny >> 1; seed: (ny & 1) ^ (ny >> 1))
   uint32_t odd[kMaxStringsPerPass];  // ny & 1
-  uint32_t kind[kMaxStringsPerPass]; // expvals: 0 diagonal (xs = 0), 1 xs = 1, 2 other, 3 padding
-  uint32_t hb[kMaxStringsPerPass];   // expvals, kind 2: highest set bit of xs
   int col[kMaxStringsPerPass];
 };
 
@@ -319,65 +325,136 @@ __device__ __forceinline__ uint32_t coset_rep(uint32_t t, const CosetParams& p) 
 // every access below is a 32-bit shared-memory load.
 extern __shared__ __align__(128) float4 coset_stage4[];
 
-// One string's sum over a warp's segment of a staged coset (stage base b4, in float4 units;
-// the lane visits j = j0, j0 + 32, ... < j1), each amplitude pair (u, u + 1) with bit h of u
-// clear (j counts those pairs) against its partner pair
-// ((u ^ x) & ~1); SW: x is odd, so the partner pair is in swapped order; ODD: odd number of Y
-// factors (imaginary part).  Returns the thread's float32 partial of the half sum.
-template <bool SW, bool ODD>
-__device__ __forceinline__ float coset_string_sum(uint32_t b4, uint32_t j0, uint32_t j1, uint32_t h, uint32_t x,
-                                                  uint32_t gam, uint32_t rho) {
-  const uint32_t lo = (1u << h) - 1u;
-  const uint32_t g1 = gam & 1u;
-  const uint32_t x4 = x >> 1;  // partner pair index = (u >> 1) ^ (x >> 1)
+// A thread's pairs of amplitudes of a coset: pair k is q0 + k * kCosetThreads, q0 the thread
+// index (u = 2 pair).
+constexpr int kCosetPairBits = 3;
+constexpr int kCosetPairs = 1 << kCosetPairBits;
+constexpr int kCosetThreadBits = 9;
+static_assert(kCosetThreads == 1 << kCosetThreadBits &&
+                  kCosetTileBits == 1 + kCosetThreadBits + kCosetPairBits,
+              "a full tile is kCosetPairs pairs per thread");
+
+// Parities of (k * 2 kCosetThreads) & gam by bit k, the same for every thread.
+__device__ __forceinline__ uint32_t pair_signs(uint32_t gam) {
+  const uint32_t g = gam >> (kCosetThreadBits + 1);
+  return (g & 1u ? 0xaau : 0u) ^ (g & 2u ? 0xccu : 0u) ^ (g & 4u ? 0xf0u : 0u);
+}
+__device__ __forceinline__ float flip_by_bit(float v, uint32_t bits, int k) {
+  return __uint_as_float(__float_as_uint(v) ^ ((bits << (31 - k)) & 0x80000000u));
+}
+
+// Pair q0 ^ x of k = 0 moved to k: at16 = 16 (q0 ^ x4), bytes from the stage's start b16.
+__device__ __forceinline__ float4 stage_pair(uint32_t b16, uint32_t at16, int k) {
+  const uint32_t off = b16 + (at16 ^ (static_cast<uint32_t>(k) * kCosetThreads * 16u));
+  return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(coset_stage4) + off);
+}
+
+// One string's sum over the thread's pairs v (u, u + 1), each against its partner pair
+// ((u ^ x) & ~1) in the stage; SW: x is odd, so the partner pair is in swapped order; ODD: odd
+// number of Y factors (imaginary part).  H < kCosetPairBits: only the pairs whose bit H of k
+// is clear.  The thread's own sign is the caller's.  Fewer pairs than threads x kCosetPairs: FULL
+// is false.
+template <int H, bool SW, bool ODD, bool FULL>
+__device__ __forceinline__ float coset_pair_sum(const float4 (&v)[kCosetPairs], uint32_t b16, uint32_t at16,
+                                                uint32_t npairs, uint32_t signs, float g1) {
   float a = 0.f;
-#pragma unroll 4
-  for (uint32_t j = j0; j < j1; j += 32) {
-    // pair index of u: j with a zero inserted at bit h - 1 (u = 2 x pair index, h >= 1)
-    const uint32_t pu = ((j >> (h - 1)) << h) | (j & (lo >> 1));
-    const float4 v = coset_stage4[b4 + pu];
-    const float4 w = coset_stage4[b4 + (pu ^ x4)];
-    const float2 a0 = lo2(v), a1 = hi2(v);
+#pragma unroll
+  for (int k = 0; k < kCosetPairs; ++k) {
+    if (H < kCosetPairBits && ((k >> H) & 1)) continue;
+    if (!FULL && threadIdx.x + static_cast<uint32_t>(k) * kCosetThreads >= npairs) break;
+    const float4 w = stage_pair(b16, at16, k);
+    const float2 a0 = lo2(v[k]), a1 = hi2(v[k]);
     const float2 b0 = SW ? hi2(w) : lo2(w), b1 = SW ? lo2(w) : hi2(w);
-    const float c0 = ODD ? a0.x * b0.y - a0.y * b0.x : a0.x * b0.x + a0.y * b0.y;
-    const float c1 = ODD ? a1.x * b1.y - a1.y * b1.x : a1.x * b1.x + a1.y * b1.y;
-    a += flip_if_odd(c0 + flip_if_odd(c1, g1), static_cast<uint32_t>(__popc((pu << 1) & gam)) + rho);
+    const float c0 = ODD ? fmaf(a0.x, b0.y, -(a0.y * b0.x)) : fmaf(a0.x, b0.x, a0.y * b0.y);
+    const float c1 = ODD ? fmaf(a1.x, b1.y, -(a1.y * b1.x)) : fmaf(a1.x, b1.x, a1.y * b1.y);
+    a = fmaf(flip_by_bit(1.f, signs, k), fmaf(g1, c1, c0), a);
   }
   return a;
 }
 
-// Diagonal string (x = 0): sum of +-|psi_u|^2 over every pair of the coset.
-__device__ __forceinline__ float coset_diag_sum(uint32_t b4, uint32_t j0, uint32_t j1, uint32_t gam, uint32_t rho) {
-  const uint32_t g1 = gam & 1u;
-  float a = 0.f;
-  for (uint32_t j = j0; j < j1; j += 32) {
-    const float4 v = coset_stage4[b4 + j];
-    const float p0 = v.x * v.x + v.y * v.y, p1 = v.z * v.z + v.w * v.w;
-    a += flip_if_odd(p0 + flip_if_odd(p1, g1), static_cast<uint32_t>(__popc((j << 1) & gam)) + rho);
+// A string's constants, worked out once per CTA.
+struct CosetString {
+  uint32_t x16;     // 16 times the partner pair's distance (XOR of pair indices)
+  uint32_t signs;   // pair_signs
+  uint32_t mode;    // expvals: 0 diagonal, 1 / 2 x = 1 (even / odd number of Y), else 4 + 4 H + 2 SW + ODD;
+                    // seed: 4 SW + 2 ODD + G1
+  float g1;         // expvals: -1 if the string's sign differs between u and u + 1
+  float weight;     // expvals: 2 where one side of each exchange is visited, else 1
+  uint32_t by_warp; // expvals: warps with this bit set leave the string to the others
+};
+
+// P is Hermitian: the two sides of an exchange (u, u ^ x) contribute the same real part, so one
+// side is visited and counted twice wherever a bit of x tells the sides apart by k or by warp; a
+// bit of the lane would leave half of the lanes idle, both sides are visited then.
+template <bool SEED>
+__device__ __forceinline__ CosetString coset_string(const CosetParams& p, int s) {
+  CosetString c;
+  const uint32_t x = p.xs[s], odd = p.odd[s], g1 = p.gam[s] & 1u;
+  c.x16 = (x >> 1) << 4;
+  c.signs = pair_signs(p.gam[s]);
+  c.g1 = g1 ? -1.f : 1.f;
+  c.weight = 1.f;
+  c.by_warp = 0u;
+  if (SEED) {
+    c.mode = (x & 1u) << 2 | odd << 1 | g1;
+  } else if (x <= 1u) {
+    c.mode = x == 0u ? 0u : 1u + odd;
+    c.weight = x == 0u ? 1.f : 2.f;
+  } else {
+    const uint32_t by_k = x >> (kCosetThreadBits + 1), by_warp = (x >> 6) & (kCosetWarps - 1);
+    const uint32_t h = by_k ? 31u - __clz(by_k) : static_cast<uint32_t>(kCosetPairBits);
+    c.mode = 4u + 4u * h + 2u * (x & 1u) + odd;
+    if (by_k || by_warp) c.weight = 2.f;
+    if (!by_k && by_warp) c.by_warp = 1u << (31 - __clz(by_warp));
   }
-  return a;
+  return c;
 }
 
-// x = 1: each pair (u, u + 1) is its own partner; the u-side term (counted twice by the caller).
-__device__ __forceinline__ float coset_x1_sum(uint32_t b4, uint32_t j0, uint32_t j1, bool odd, uint32_t gam,
-                                              uint32_t rho) {
-  float a = 0.f;
-  for (uint32_t j = j0; j < j1; j += 32) {
-    const float4 v = coset_stage4[b4 + j];
-    const float c0 = odd ? v.x * v.w - v.y * v.z : v.x * v.z + v.y * v.w;
-    a += flip_if_odd(c0, static_cast<uint32_t>(__popc((j << 1) & gam)) + rho);
+// One string's sum over a coset, the thread's part (without the thread's sign and the weight).
+template <bool FULL>
+__device__ __forceinline__ float coset_string_sum(const float4 (&v)[kCosetPairs], uint32_t b16, uint32_t npairs,
+                                                  const CosetString& c) {
+  const uint32_t at16 = (threadIdx.x << 4) ^ c.x16, signs = c.signs;
+  const float g1 = c.g1;
+  if (c.mode < 4u) {  // diagonal, or each pair is its own partner
+    float a = 0.f;
+#pragma unroll
+    for (int k = 0; k < kCosetPairs; ++k) {
+      const float4 t = v[k];  // zero past the tile
+      float d;
+      if (c.mode == 0u) d = fmaf(g1, fmaf(t.z, t.z, t.w * t.w), fmaf(t.x, t.x, t.y * t.y));
+      else d = c.mode == 2u ? fmaf(t.x, t.w, -(t.y * t.z)) : fmaf(t.x, t.z, t.y * t.w);
+      a = fmaf(flip_by_bit(1.f, signs, k), d, a);
+    }
+    return a;
   }
-  return a;
+  if ((threadIdx.x >> 5) & c.by_warp) return 0.f;
+  switch (c.mode) {
+    case 4: return coset_pair_sum<0, false, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 5: return coset_pair_sum<0, false, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 6: return coset_pair_sum<0, true, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 7: return coset_pair_sum<0, true, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 8: return coset_pair_sum<1, false, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 9: return coset_pair_sum<1, false, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 10: return coset_pair_sum<1, true, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 11: return coset_pair_sum<1, true, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 12: return coset_pair_sum<2, false, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 13: return coset_pair_sum<2, false, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 14: return coset_pair_sum<2, true, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 15: return coset_pair_sum<2, true, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 16: return coset_pair_sum<3, false, false, FULL>(v, b16, at16, npairs, signs, g1);
+    case 17: return coset_pair_sum<3, false, true, FULL>(v, b16, at16, npairs, signs, g1);
+    case 18: return coset_pair_sum<3, true, false, FULL>(v, b16, at16, npairs, signs, g1);
+    default: return coset_pair_sum<3, true, true, FULL>(v, b16, at16, npairs, signs, g1);
+  }
 }
 
-// Stage `st` <- the coset of pipeline iteration `item` (one call per thread: its 16-byte
-// pieces k = tid, tid + threads, ..., then an arrive on the stage's full barrier once they
-// have landed).  Slot a of the stage holds the chunk at high index rep ^ slot_hi[a].
-__device__ __forceinline__ void coset_issue(const CosetParams& p, int64_t item, int st, const uint32_t* slot_hi,
-                                            uint64_t* full) {
+// Stage `st` <- the coset rep of row b (one call per thread: its 16-byte pieces k = tid, tid +
+// threads, ..., then an arrive on the stage's full barrier once they have landed).  Slot a of
+// the stage holds the chunk at high index rep ^ slot_hi[a].
+__device__ __forceinline__ void coset_issue(const CosetParams& p, int64_t b, uint32_t rep, int st,
+                                            const uint32_t* slot_hi, uint64_t* full) {
   const uint32_t tile = 1u << p.tb;
-  const int64_t b = item / p.cosets;
-  const uint32_t rep = coset_rep(static_cast<uint32_t>(item - b * p.cosets), p);
   const uint32_t pmask = (1u << (p.c - 1)) - 1u;  // 16-byte pieces per chunk, minus one
   const float2* row = p.state + (static_cast<uint64_t>(b) << p.n);
   float2* dst = reinterpret_cast<float2*>(coset_stage4) + static_cast<size_t>(st) * tile;
@@ -389,32 +466,19 @@ __device__ __forceinline__ void coset_issue(const CosetParams& p, int64_t item, 
   cp_async_arrive(&full[st]);
 }
 
-// Backward seed, one string over a thread's output pairs of a staged coset: pair k is
-// q0 + k * kCosetThreads (local index u = 2q), its partner pair (q ^ x4) in the stage.  The
-// sign (-1)^popcount(u & gam) splits into the thread's part (bits of 2 q0, folded into cft)
-// and the part from k * 2 kCosetThreads, the same for every thread; SW: x odd (the partner
-// pair is in swapped order); ODD: odd number of Y factors.
-constexpr int kSeedPairs = (1 << kCosetTileBits) / 2 / kCosetThreads;
-
-template <bool SW, bool ODD, bool FULL>
-__device__ __forceinline__ void seed_string(float2 (&o)[kSeedPairs][2], uint32_t b4, uint32_t q0, uint32_t npairs,
-                                            uint32_t x4, uint32_t gam, float cft) {
-  const uint32_t g1 = gam & 1u;
-  // FULL (tiles of 2^13 amplitudes): every thread has all its pairs, so the loads of all
-  // of them can be issued before the first product
-  float4 w[kSeedPairs];
+// Backward seed, one string over a thread's output pairs o of a staged coset; signs, SW, ODD
+// as above, cft the coefficient with the thread's sign, G1: the string's sign differs between
+// u and u + 1.
+template <bool SW, bool ODD, bool G1, bool FULL>
+__device__ __forceinline__ void seed_string(float2 (&o)[kCosetPairs][2], uint32_t b16, uint32_t at16,
+                                            uint32_t npairs, uint32_t signs, float cft) {
 #pragma unroll
-  for (int k = 0; k < kSeedPairs; ++k) {
-    const uint32_t q = q0 + static_cast<uint32_t>(k) * kCosetThreads;
-    w[k] = (FULL || q < npairs) ? coset_stage4[b4 + (q ^ x4)] : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-#pragma unroll
-  for (int k = 0; k < kSeedPairs; ++k) {
-    const uint32_t q = q0 + static_cast<uint32_t>(k) * kCosetThreads;
-    if (!FULL && q >= npairs) break;  // tiles of fewer than 2^13 amplitudes
-    const uint32_t up = static_cast<uint32_t>(__popc((static_cast<uint32_t>(k) * 2u * kCosetThreads) & gam));
-    const float c0 = flip_if_odd(cft, up), c1 = flip_if_odd(cft, up + g1);
-    const float2 b0 = SW ? hi2(w[k]) : lo2(w[k]), b1 = SW ? lo2(w[k]) : hi2(w[k]);
+  for (int k = 0; k < kCosetPairs; ++k) {
+    // tiles of fewer than 2^13 amplitudes
+    if (!FULL && threadIdx.x + static_cast<uint32_t>(k) * kCosetThreads >= npairs) break;
+    const float4 w = stage_pair(b16, at16, k);
+    const float c0 = flip_by_bit(cft, signs, k), c1 = G1 ? -c0 : c0;
+    const float2 b0 = SW ? hi2(w) : lo2(w), b1 = SW ? lo2(w) : hi2(w);
     if (ODD) {
       o[k][0].x = fmaf(-c0, b0.y, o[k][0].x);
       o[k][0].y = fmaf(c0, b0.x, o[k][0].y);
@@ -429,149 +493,171 @@ __device__ __forceinline__ void seed_string(float2 (&o)[kSeedPairs][2], uint32_t
   }
 }
 
-template <bool SEED, int NS>
+template <bool FULL>
+__device__ __forceinline__ void seed_string(float2 (&o)[kCosetPairs][2], uint32_t b16, uint32_t npairs,
+                                            const CosetString& c, float cft) {
+  const uint32_t at16 = (threadIdx.x << 4) ^ c.x16, signs = c.signs;
+  switch (c.mode) {
+    case 0: seed_string<false, false, false, FULL>(o, b16, at16, npairs, signs, cft); break;
+    case 1: seed_string<false, false, true, FULL>(o, b16, at16, npairs, signs, cft); break;
+    case 2: seed_string<false, true, false, FULL>(o, b16, at16, npairs, signs, cft); break;
+    case 3: seed_string<false, true, true, FULL>(o, b16, at16, npairs, signs, cft); break;
+    case 4: seed_string<true, false, false, FULL>(o, b16, at16, npairs, signs, cft); break;
+    case 5: seed_string<true, false, true, FULL>(o, b16, at16, npairs, signs, cft); break;
+    case 6: seed_string<true, true, false, FULL>(o, b16, at16, npairs, signs, cft); break;
+    default: seed_string<true, true, true, FULL>(o, b16, at16, npairs, signs, cft); break;
+  }
+}
+
+// FULL: stages of 2^13 amplitudes (every thread has all its pairs).
+template <bool SEED, bool FULL>
 __global__ void __launch_bounds__(kCosetThreads, 1) k_coset(const CosetParams p) {
   __shared__ __align__(8) uint64_t full[kCosetStages];
   __shared__ uint32_t slot_hi[1 << kCosetMaxRank];  // sum_k a_k b_k for slot a
-  __shared__ float red[2][kCosetWarps][kMaxStringsPerPass];
+  __shared__ CosetString strings[kMaxStringsPerPass];
+  // expvals, by iteration parity: halves of the warps' lanes, sums of half a string's
+  __shared__ __align__(16) float half_sum[SEED ? 1 : 2][kMaxStringsPerPass][kCosetThreads / 2];
+  __shared__ float red[2][kCosetWarps];
   __shared__ int quit;
+  static_assert(kCosetWarps == 2 * kMaxStringsPerPass, "two warps add a string's sums");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tile = 1u << p.tb;
+  const uint32_t tile = 1u << p.tb, npairs = tile >> 1, q0 = threadIdx.x;
   for (int a = threadIdx.x; a < (1 << p.r); a += kCosetThreads) {
     uint32_t h = 0;
     for (int k = 0; k < p.r; ++k)
       if ((a >> k) & 1) h ^= p.basis[k];
     slot_hi[a] = h;
   }
+  if (threadIdx.x < kMaxStringsPerPass) strings[threadIdx.x] = coset_string<SEED>(p, threadIdx.x);
   if (threadIdx.x == 0) {
     for (int st = 0; st < kCosetStages; ++st) mbar_init_count(&full[st], kCosetThreads);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     quit = 0;
   }
+  // signs by string: the thread's (bit s), and what lane s needs for the coset's
+  uint32_t own = 0;
+  for (int s = 0; s < p.ns; ++s) own |= (static_cast<uint32_t>(__popc((q0 << 1) & p.gam[s])) & 1u) << s;
+  const uint32_t zh = lane < p.ns ? p.zh[lane] : 0u, fl = lane < p.ns ? p.fl[lane] : 0u;
+  const int col = lane < p.ns ? p.col[lane] : 0;
   __syncthreads();
   const int64_t total = p.bsz * p.cosets;
+  const int cosets_log = p.n - p.tb;
+  auto rep_of = [&](int64_t item) {
+    return coset_rep(static_cast<uint32_t>(item) & static_cast<uint32_t>(p.cosets - 1), p);
+  };
   volatile int* vquit = &quit;
   // prologue: the first kCosetStages - 1 cosets in flight
   int64_t issued = 0;  // pipeline iterations whose loads this CTA issued
-  for (; issued < kCosetStages - 1 && blockIdx.x + issued * gridDim.x < total; ++issued)
-    coset_issue(p, blockIdx.x + issued * gridDim.x, static_cast<int>(issued), slot_hi, full);
-  // expvals: pair visits of all strings in a coset (tile / 4 per string, tile / 2 for x = 0
-  // or 1; strings past ns are padding)
-  uint32_t visits = 0;
-  for (int s = 0; s < p.ns; ++s) visits += p.kind[s] == 3u ? 0u : (p.kind[s] == 2u ? tile >> 2 : tile >> 1);
+  uint32_t reps[kCosetStages] = {0u, 0u, 0u};  // of this iteration's coset and the next ones
+#pragma unroll
+  for (int k = 0; k < kCosetStages - 1; ++k) {
+    const int64_t item = blockIdx.x + static_cast<int64_t>(k) * gridDim.x;
+    if (item >= total) break;
+    reps[k] = rep_of(item);
+    coset_issue(p, item >> cosets_log, reps[k], k, slot_hi, full);
+    ++issued;
+  }
   const uint32_t lmask = (1u << p.c) - 1u;
-  int it = 0;
+  int it = 0, st = 0;
+  // the previous iteration's partials: its sums meet in red after the barrier that follows
+  auto put_partial = [&](int64_t item, int parity) {
+    if (!SEED && static_cast<int>(threadIdx.x) < p.ns) {
+      const double sum = static_cast<double>(red[parity][2 * threadIdx.x]) +
+                         static_cast<double>(red[parity][2 * threadIdx.x + 1]);
+      p.partial[item * kMaxStringsPerPass + threadIdx.x] =
+          (*vquit == 0) ? sum : __longlong_as_double(0x7ff8000000000000ll);
+    }
+  };
   for (int64_t item = blockIdx.x; item < total; item += gridDim.x, ++it) {
-    const int st = it % kCosetStages;
     // every thread finished reading the stage of iteration it - 1 (the barrier that closed
     // it): refill it with the coset kCosetStages - 1 iterations ahead
     const int64_t ahead = item + static_cast<int64_t>(kCosetStages - 1) * gridDim.x;
     if (ahead < total && *vquit == 0) {
-      coset_issue(p, ahead, static_cast<int>(issued % kCosetStages), slot_hi, full);
+      reps[kCosetStages - 1] = rep_of(ahead);
+      coset_issue(p, ahead >> cosets_log, reps[kCosetStages - 1], st == 0 ? kCosetStages - 1 : st - 1, slot_hi, full);
       ++issued;
     }
-    const int64_t b = item / p.cosets;
-    const uint32_t rep = coset_rep(static_cast<uint32_t>(item - b * p.cosets), p);
+    const int64_t b = item >> cosets_log;
+    const uint32_t rep = reps[0];
+    // output pair k; what earlier passes left there is read now, for the end
+    auto out_at = [&](int k) {
+      const uint32_t u = (q0 + static_cast<uint32_t>(k) * kCosetThreads) << 1;
+      return p.out + (static_cast<uint64_t>(b) << p.n) + (static_cast<uint64_t>(rep ^ slot_hi[u >> p.c]) << p.c) +
+             (u & lmask);
+    };
+    float4 old[SEED ? kCosetPairs : 1];
+    if (SEED && p.accumulate) {
+#pragma unroll
+      for (int k = 0; k < kCosetPairs; ++k)
+        if (FULL || q0 + static_cast<uint32_t>(k) * kCosetThreads < npairs) old[SEED ? k : 0] = ld4(out_at(k));
+    }
+    // bit s: parity of string s's constant sign, the coset's and the thread's
+    const uint32_t flips =
+        own ^ __ballot_sync(0xffffffffu, (static_cast<uint32_t>(__popc(rep & zh)) ^ fl) & 1u);
+    const float coef = SEED && lane < p.ns ? __ldg(p.coef + b * p.m + col) : 0.f;
     bool ok = *vquit == 0;
     if (ok && !bulk::mbar_wait(&full[st], static_cast<uint32_t>(it / kCosetStages) & 1u)) {
       ok = false;
-      if (lane == 0) {
-        atomicExch(p.status, TQK_TIMEOUT);
-        *vquit = 1;
-      }
+      atomicExch(p.status, TQK_TIMEOUT);
+      *vquit = 1;
     }
-    const uint32_t b4 = static_cast<uint32_t>(st) * (tile >> 1);  // stage start, float4 units
+    ok = __all_sync(0xffffffffu, ok);
+    const uint32_t b16 = static_cast<uint32_t>(st) * tile * 8u;  // stage start, bytes
     if (ok && SEED) {
       // string by string over the thread's output pairs (outputs in registers), then one
       // store per pair; each string's orientation and Y parity are fixed for its loop
-      const uint32_t npairs = tile >> 1, q0 = threadIdx.x;
-      float2 o[kSeedPairs][2];
+      float2 o[kCosetPairs][2];
 #pragma unroll
-      for (int k = 0; k < kSeedPairs; ++k) o[k][0] = o[k][1] = make_float2(0.f, 0.f);
+      for (int k = 0; k < kCosetPairs; ++k) o[k][0] = o[k][1] = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int s = 0; s < p.ns; ++s) {
-        const uint32_t x = p.xs[s], gam_s = p.gam[s];
-        const uint32_t rho_s = (static_cast<uint32_t>(__popc(rep & p.zh[s])) ^ p.fl[s]) & 1u;
-        const float cft = flip_if_odd(__ldg(p.coef + b * p.m + p.col[s]),
-                                      static_cast<uint32_t>(__popc((q0 << 1) & gam_s)) + rho_s);
-        const uint32_t x4 = x >> 1;
-        const int variant = ((x & 1u) ? 2 : 0) + (p.odd[s] ? 1 : 0);
-        if (npairs == static_cast<uint32_t>(kSeedPairs * kCosetThreads)) {
-          if (variant == 3) seed_string<true, true, true>(o, b4, q0, npairs, x4, gam_s, cft);
-          else if (variant == 2) seed_string<true, false, true>(o, b4, q0, npairs, x4, gam_s, cft);
-          else if (variant == 1) seed_string<false, true, true>(o, b4, q0, npairs, x4, gam_s, cft);
-          else seed_string<false, false, true>(o, b4, q0, npairs, x4, gam_s, cft);
-        } else {
-          if (variant == 3) seed_string<true, true, false>(o, b4, q0, npairs, x4, gam_s, cft);
-          else if (variant == 2) seed_string<true, false, false>(o, b4, q0, npairs, x4, gam_s, cft);
-          else if (variant == 1) seed_string<false, true, false>(o, b4, q0, npairs, x4, gam_s, cft);
-          else seed_string<false, false, false>(o, b4, q0, npairs, x4, gam_s, cft);
-        }
-      }
+      for (int s = 0; s < p.ns; ++s)
+        seed_string<FULL>(o, b16, npairs, strings[s], flip_if_odd(__shfl_sync(0xffffffffu, coef, s), (flips >> s) & 1u));
 #pragma unroll
-      for (int k = 0; k < kSeedPairs; ++k) {
-        const uint32_t q = q0 + static_cast<uint32_t>(k) * kCosetThreads;
-        if (q >= npairs) break;
-        const uint32_t u = q << 1;
-        float2* dst = p.out + (static_cast<uint64_t>(b) << p.n) +
-                      (static_cast<uint64_t>(rep ^ slot_hi[u >> p.c]) << p.c) + (u & lmask);
+      for (int k = 0; k < kCosetPairs; ++k) {
+        if (!FULL && q0 + static_cast<uint32_t>(k) * kCosetThreads >= npairs) break;
         float2 o0 = o[k][0], o1 = o[k][1];
         if (p.accumulate) {
-          const float4 old = ld4(dst);
-          o0.x += old.x;
-          o0.y += old.y;
-          o1.x += old.z;
-          o1.y += old.w;
+          o0.x += old[SEED ? k : 0].x;
+          o0.y += old[SEED ? k : 0].y;
+          o1.x += old[SEED ? k : 0].z;
+          o1.y += old[SEED ? k : 0].w;
         }
-        st4(dst, pack4(o0, o1));
+        st4(out_at(k), pack4(o0, o1));
       }
     } else if (ok) {
-      // expvals: the visits of all strings in a row (tile / 4 pairs per string, tile / 2 for
-      // x = 0 or 1) are cut into one contiguous segment per warp, so a warp takes one or two
-      // strings, each with its orientation and Y parity fixed for the loop.  A pair of
-      // amplitude pairs (u, u + 1) / ((u ^ xs) & ~1) is visited once, from the side whose bit
-      // hb (the highest of xs) is clear -- enumerated directly by inserting a zero at hb --
-      // and counted twice (P is Hermitian: both sides contribute the same real part).
-      const uint32_t per = ((visits + kCosetWarps - 1) / kCosetWarps + 31u) & ~31u;
-      const uint32_t w0 = static_cast<uint32_t>(warp) * per, w1 = min(visits, w0 + per);
-      // the warp's row of red: zero, then the sums of the strings its segment touches (one
-      // string body in the code, looped at run time, instead of one per string)
-      if (lane < NS) red[it & 1][warp][lane] = 0.f;
-      __syncwarp();
-      uint32_t f0 = 0;
-#pragma unroll 1
-      for (int s = 0; s < p.ns && f0 < w1; ++s) {
-        const uint32_t ks = p.kind[s];
-        const uint32_t f1 = f0 + (ks == 3u ? 0u : (ks == 2u ? tile >> 2 : tile >> 1));
-        const uint32_t lo = max(f0, w0), hi = min(f1, w1);
-        if (lo < hi) {  // uniform for the warp
-          const uint32_t j0 = lo - f0 + lane, j1 = hi - f0;
-          const uint32_t xs_s = p.xs[s], gam_s = p.gam[s], hb_s = p.hb[s], odd_s = p.odd[s];
-          const uint32_t rho_s = (static_cast<uint32_t>(__popc(rep & p.zh[s])) ^ p.fl[s]) & 1u;
-          float a;
-          if (ks == 0u) a = coset_diag_sum(b4, j0, j1, gam_s, rho_s);
-          else if (ks == 1u) a = 2.f * coset_x1_sum(b4, j0, j1, odd_s != 0u, gam_s, rho_s);
-          else if (xs_s & 1u)
-            a = 2.f * (odd_s ? coset_string_sum<true, true>(b4, j0, j1, hb_s, xs_s, gam_s, rho_s)
-                             : coset_string_sum<true, false>(b4, j0, j1, hb_s, xs_s, gam_s, rho_s));
-          else
-            a = 2.f * (odd_s ? coset_string_sum<false, true>(b4, j0, j1, hb_s, xs_s, gam_s, rho_s)
-                             : coset_string_sum<false, false>(b4, j0, j1, hb_s, xs_s, gam_s, rho_s));
+      // expvals: the thread's pairs in registers, string by string against their partners in
+      // the stage
+      float4 v[kCosetPairs];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-          if (lane == 0) red[it & 1][warp][s] = a;
-        }
-        f0 = f1;
+      for (int k = 0; k < kCosetPairs; ++k) {
+        const uint32_t q = q0 + static_cast<uint32_t>(k) * kCosetThreads;
+        v[k] = FULL || q < npairs ? stage_pair(b16, q0 << 4, k) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-    } else if (!SEED) {
-      if (lane < NS) red[it & 1][warp][lane] = 0.f;  // a stage that never arrived: its partials are NaN below
+#pragma unroll 1
+      for (int s = 0; s < p.ns; ++s) {
+        const CosetString& c = strings[s];
+        float a = flip_if_odd(c.weight, (flips >> s) & 1u) * coset_string_sum<FULL>(v, b16, npairs, c);
+        a += __shfl_xor_sync(0xffffffffu, a, 16);
+        if (lane < 16) half_sum[SEED ? 0 : it & 1][s][16 * warp + lane] = a;
+      }
     }
     __syncthreads();  // the stage is read: the next iteration may refill it
-    if (!SEED && warp == 0 && lane < p.ns) {
-      double sum = 0.0;
-      for (int w = 0; w < kCosetWarps; ++w) sum += static_cast<double>(red[it & 1][w][lane]);
-      p.partial[item * kMaxStringsPerPass + lane] = (*vquit == 0) ? sum : __longlong_as_double(0x7ff8000000000000ll);
+    if (!SEED) {
+      if (it > 0) put_partial(item - gridDim.x, (it - 1) & 1);
+      // warps 2 s and 2 s + 1: half of string s's sums each
+      const float4 h = *reinterpret_cast<const float4*>(&half_sum[SEED ? 0 : it & 1][warp >> 1][128 * (warp & 1) + 4 * lane]);
+      float a = (h.x + h.y) + (h.z + h.w);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) red[it & 1][warp] = a;
     }
+#pragma unroll
+    for (int k = 0; k < kCosetStages - 1; ++k) reps[k] = reps[k + 1];
+    st = st == kCosetStages - 1 ? 0 : st + 1;
+  }
+  if (!SEED && it > 0) {
+    __syncthreads();
+    put_partial(blockIdx.x + static_cast<int64_t>(it - 1) * gridDim.x, (it - 1) & 1);
   }
   // after a timeout, wait (bounded) for this CTA's copies still in flight before exiting
   if (quit && threadIdx.x == 0) {
@@ -672,8 +758,7 @@ static void coset_params(const CosetGroup& g, int n, const uint64_t* xmask, cons
   const uint32_t lmask = (1u << g.c) - 1u;
   for (int s = 0; s < kMaxStringsPerPass; ++s) {
     if (s >= g.ns) {
-      p.xs[s] = p.gam[s] = p.zh[s] = p.fl[s] = p.odd[s] = p.hb[s] = 0u;
-      p.kind[s] = 3u;
+      p.xs[s] = p.gam[s] = p.zh[s] = p.fl[s] = p.odd[s] = 0u;
       p.col[s] = 0;
       continue;
     }
@@ -690,14 +775,12 @@ static void coset_params(const CosetGroup& g, int n, const uint64_t* xmask, cons
     p.zh[s] = zh;
     p.odd[s] = static_cast<uint32_t>(ny & 1);
     p.fl[s] = seed ? static_cast<uint32_t>((ny & 1) ^ (ny >> 1)) : static_cast<uint32_t>(ny >> 1);
-    p.kind[s] = p.xs[s] == 0u ? 0u : (p.xs[s] == 1u ? 1u : 2u);
-    p.hb[s] = p.xs[s] == 0u ? 0u : static_cast<uint32_t>(31 - __builtin_clz(p.xs[s]));
     p.col[s] = j;
   }
 }
 
-template <bool SEED, int NS>
-static int launch_coset_ns(const CosetParams& p, cudaStream_t st) {
+template <bool SEED, bool FULL>
+static int launch_coset_as(const CosetParams& p, cudaStream_t st) {
   static std::atomic<uint64_t> configured{0};  // devices whose attribute is set
   const size_t smem = static_cast<size_t>(kCosetStages) * (8ull << p.tb);
   int dev = 0;
@@ -705,7 +788,7 @@ static int launch_coset_ns(const CosetParams& p, cudaStream_t st) {
   const uint64_t bit = 1ull << (dev & 63);
   if (!(configured.load() & bit)) {
     // the largest dynamic request (2^13-amplitude stages)
-    if (cudaFuncSetAttribute(k_coset<SEED, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_coset<SEED, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(kCosetStages * (8ull << kCosetTileBits))) != cudaSuccess)
       return fail(TQK_CUDA_ERROR, "coset pass: cannot reserve %d bytes of shared memory",
                   static_cast<int>(kCosetStages * (8ull << kCosetTileBits)));
@@ -715,16 +798,13 @@ static int launch_coset_ns(const CosetParams& p, cudaStream_t st) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t total = p.bsz * p.cosets;
   const int64_t grid = total < sms ? total : sms;
-  k_coset<SEED, NS><<<static_cast<unsigned>(grid), kCosetThreads, smem, st>>>(p);
+  k_coset<SEED, FULL><<<static_cast<unsigned>(grid), kCosetThreads, smem, st>>>(p);
   return TQK_OK;
 }
 
 template <bool SEED>
 static int launch_coset(const CosetParams& p, cudaStream_t st) {
-  if (p.ns <= 1) return launch_coset_ns<SEED, 1>(p, st);
-  if (p.ns <= 2) return launch_coset_ns<SEED, 2>(p, st);
-  if (p.ns <= 4) return launch_coset_ns<SEED, 4>(p, st);
-  return launch_coset_ns<SEED, 8>(p, st);
+  return p.tb == kCosetTileBits ? launch_coset_as<SEED, true>(p, st) : launch_coset_as<SEED, false>(p, st);
 }
 
 __global__ void __launch_bounds__(256) k_probs(const float2* state, float* out, int64_t total_half) {
