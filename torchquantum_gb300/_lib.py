@@ -8,6 +8,7 @@ returns a non-zero status.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import re
 from typing import Optional, Sequence
@@ -154,8 +155,11 @@ def _u64(vals: Sequence[int]):
     return (ctypes.c_uint64 * max(1, len(vals)))(*vals)
 
 
+_raw_stream = torch._C._cuda_getCurrentRawStream  # without building a Stream object
+
+
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.device.index)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -232,6 +236,11 @@ def coset_groups(xmasks, n: int):
     strings in order, a group growing while it holds at most 8 strings and its X-masks'
     parts above the lowest c bits span at most T - c dimensions for c = min(4, T),
     T = min(n, 13).  Returns [(string indices, c, rank)] with the widest such c."""
+    return _coset_groups(tuple(xmasks), n)
+
+
+@functools.lru_cache(maxsize=256)
+def _coset_groups(xmasks: tuple, n: int):
     T = min(n, COSET_TILE_BITS)
     cmin = min(COSET_MIN_CHUNK_BITS, T)
     groups, cur = [], []
@@ -527,7 +536,8 @@ def cross_to_complex(mr: torch.Tensor) -> torch.Tensor:
 
 # ------------------------------------------------------------------ gate programs
 def _dstream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = device.index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def gate_operands(table, ngates, device):

@@ -22,6 +22,7 @@ kernel maps any six wires onto its tiles), so no qubit-reordering pass is schedu
 """
 from __future__ import annotations
 
+import copy
 import json
 import os
 import threading
@@ -260,6 +261,9 @@ WIDE_BEAMS = ((8, 32), (16, 128))
 WIDE_BEAM_MIN_AMPS = 1 << 27
 
 
+_CHOICES: dict = {}
+
+
 def choose_fusion(wire_lists: Sequence[Sequence[int]], n: int, bsz: int, dev: torch.device, tc_ok: bool,
                   with_adjoint: bool, widths: Sequence[int] = (4, 5, 6), stored: bool = False,
                   lone_kind: Optional[Sequence[int]] = None):
@@ -269,6 +273,7 @@ def choose_fusion(wire_lists: Sequence[Sequence[int]], n: int, bsz: int, dev: to
     see ``plan_cost``)."""
     from . import fusion
 
+    wire_lists = tuple(map(tuple, wire_lists))
     try:
         costs = pass_costs(n, bsz, dev, tc_ok)
     except torch.cuda.OutOfMemoryError:
@@ -277,6 +282,13 @@ def choose_fusion(wire_lists: Sequence[Sequence[int]], n: int, bsz: int, dev: to
         torch.cuda.empty_cache()
         costs = {"dense": {str(k): (1.0 + 0.25 * k, 2.0 + 0.5 * k) for k in range(1, 7)},
                  "tc": (1.0, 2.0, 1.5) if tc_ok else None, "rows": 0}
+    # memoised on the circuit's structure (with the measured costs, which a later measurement
+    # may replace): a circuit recorded again every step costs its nine candidates once
+    key = (wire_lists, n, bsz, str(dev), tc_ok, with_adjoint, tuple(widths), stored,
+           None if lone_kind is None else tuple(lone_kind))
+    hit = _CHOICES.get(key)
+    if hit is not None and hit[0] == costs:
+        return hit[1], list(hit[2]), hit[3], costs
     best = None
     # on large states (a pass of >= 1 GiB) wide beams are tried too for 6-wire blocks
     # (width 32, and width 128 with a 16-gate front): they plan once per circuit structure
@@ -291,4 +303,7 @@ def choose_fusion(wire_lists: Sequence[Sequence[int]], n: int, bsz: int, dev: to
             cost, flags = plan_cost(plan, costs, tc_ok, with_adjoint, stored, lone_kind)
             if best is None or cost < best[0]:
                 best = (cost, plan, flags, k)
+    if len(_CHOICES) > 256:
+        _CHOICES.clear()
+    _CHOICES[key] = (copy.deepcopy(costs), best[1], tuple(best[2]), best[3])
     return best[1], best[2], best[3], costs

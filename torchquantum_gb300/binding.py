@@ -85,7 +85,7 @@ class _ApplyUnitary(torch.autograd.Function):
         m = mat.detach().to(x.device, torch.complex64)
         m3 = (m if m.dim() == 3 else m.unsqueeze(0)).resolve_conj().resolve_neg().contiguous()
         w = (ctypes.c_int32 * k)(*wires)
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+        stream = torch._C._cuda_getCurrentRawStream(x.device.index)
         if _out_of_place(x, bsz, n, k):
             out = torch.empty_like(x)
             _check(lib.tqk_apply_matrix_to(x.data_ptr(), out.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0],
@@ -107,7 +107,7 @@ class _ApplyUnitary(torch.autograd.Function):
         need_mat = ctx.needs_input_grad[1]
         grad = torch.zeros(m3.shape[0] * d * d * 2, dtype=torch.float64, device=x.device) if need_mat else None
         w = (ctypes.c_int32 * k)(*ctx.wires)
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+        stream = torch._C._cuda_getCurrentRawStream(x.device.index)
         if _out_of_place(x, bsz, n, k):
             g = _readable(grad_out, bsz)
             lam = torch.empty_like(g)

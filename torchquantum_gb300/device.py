@@ -73,6 +73,8 @@ _PLAIN_ATTRS = frozenset({"n_wires", "device_name", "bsz", "device", "record_op"
 
 
 class QuantumDevice(nn.Module):
+    is_density = False  # (density.NoiseDevice: True)
+
     def __setattr__(self, name, value):
         if name in _PLAIN_ATTRS:
             self.__dict__[name] = value
@@ -148,16 +150,24 @@ class QuantumDevice(nn.Module):
         b = op.batch
         if b and b not in (1, self.bsz):
             raise ValueError(f"gate operand batch {b} does not match QuantumDevice bsz {self.bsz}")
-        n = self.n_wires
+        wires, d = op.wires, self.__dict__
+        if wires:
+            n = d["n_wires"]
+            if min(wires) < 0 or max(wires) >= n or len(set(wires)) != len(wires):
+                self._refuse_wires(wires, n)
+        d["_pending"].append(op)
+        d["_out"] = None
+
+    @staticmethod
+    def _refuse_wires(wires, n: int) -> None:
+        """The checks (and messages) of the kernels' host validation."""
         seen = set()
-        for w in op.wires:  # same checks (and messages) as the kernels' host validation
+        for w in wires:
             if w < 0 or w >= n:
                 raise _lib.TQKError(1, f"wire {w} out of range for n_wires={n}")
             if w in seen:
                 raise _lib.TQKError(1, f"wire {w} used twice")
             seen.add(w)
-        self._pending.append(op)
-        self._out = None
 
     def _flush(self) -> None:
         """Compile the recorded gates into a segment and apply it to the state buffer."""
@@ -186,7 +196,9 @@ class QuantumDevice(nn.Module):
         if mode is True:
             return True
         free, _ = torch.cuda.mem_get_info(self.device)
-        cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        stats = torch.cuda.memory_stats_as_nested_dict(self.device)  # (memory_reserved() flattens it first)
+        cached = sum(s * stats[k]["all"]["current"] for s, k in ((1, "reserved_bytes"), (-1, "allocated_bytes"))) \
+            if stats else 0
         return seg.stored_bytes(self._buf) <= CHECKPOINT_MEMORY_SHARE * (free + cached)
 
     def _output(self) -> torch.Tensor:

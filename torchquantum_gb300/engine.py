@@ -38,6 +38,13 @@ class TapeOp:
     ``source`` is the autograd-tracked tensor it was taken from (or None).
     """
 
+    native = None   # the parameterised gate (program.NativeGate) the operand is built from ..
+    op128 = None    # .. its complex128 operand and that operand's address
+    ptr128 = 0
+    members = None  # the ops of a fused block
+    const = None    # the constant gate (its template op) this is an application of
+    _op128_keep = None  # complex128 operand of an op without parameters
+
     def __init__(self, kind, wires, controls=(), targets=(), ctrl_val=1, operand=None, source=None, uncompute=None):
         self.kind = kind
         self.wires = list(wires)

@@ -104,7 +104,8 @@ def _op_from_matrix(name: str, matrix: torch.Tensor, wires, device) -> engine.Ta
     return mk(engine.KIND_DENSE, matrix)
 
 
-_STRUCT_NCTRL = {"dense": 0, "diag": 0, "phase": 0}
+_STRUCT_KIND = {"dense": engine.KIND_DENSE, "ctrl": engine.KIND_CTRL, "diag": engine.KIND_DIAG,
+                "phase": engine.KIND_PHASE}
 
 
 def _native_record(cname, wires, params, inverse, q_device):
@@ -118,8 +119,7 @@ def _native_record(cname, wires, params, inverse, q_device):
     if params.dtype not in (torch.float32, torch.float64):
         params = params.to(torch.float32)
     kind_name = gd.struct[0]
-    kind = {"dense": engine.KIND_DENSE, "ctrl": engine.KIND_CTRL, "diag": engine.KIND_DIAG,
-            "phase": engine.KIND_PHASE}[kind_name]
+    kind = _STRUCT_KIND[kind_name]
     nctrl = gd.struct[1] if kind_name == "ctrl" else 0
     return program.NativeGate(cname, wires, params, inverse, kind, nctrl)
 
@@ -144,6 +144,7 @@ def _const_op(cname, k, wires, inverse, fused, device) -> engine.TapeOp:
     op = engine.TapeOp(tpl.kind, wires, controls=[wires[i] for i in tpl.controls],
                        targets=[wires[i] for i in tpl.targets], ctrl_val=tpl.ctrl_val, operand=tpl.operand,
                        source=tpl.source, uncompute=tpl.uncompute)
+    op.const = tpl
     return op
 
 

@@ -21,6 +21,7 @@ host for ``random.choices``.
 """
 from __future__ import annotations
 
+import functools
 from collections import OrderedDict
 from typing import Dict, List, Optional, Sequence, Union
 
@@ -37,6 +38,7 @@ __all__ = ["expval_joint_analytical", "expval_joint_analytical_batch", "expval",
            "expval_joint_sampling_grouping"]
 
 
+@functools.lru_cache(maxsize=4096)
 def pauli_masks(observable: str, n: int):
     """(xmask, zmask) over the in-row index for a Pauli string; P[0] acts on wire 0 (bit n-1)."""
     x = z = 0
@@ -233,19 +235,35 @@ def _parity64(v: torch.Tensor) -> torch.Tensor:
     return v & 1
 
 
+_ROTATIONS: dict = {}
+
+
+def _diagonalizing_names(ch: str) -> list:
+    """Names of the gates that diagonalise a Pauli letter (asked of the operator once)."""
+    names = _ROTATIONS.get(ch)
+    if names is None:
+        from .operators import op_name_dict
+
+        pauli = op_name_dict[{"X": "paulix", "Y": "pauliy", "Z": "pauliz", "I": "i"}[ch]]()
+        names = _ROTATIONS[ch] = [g.op_name for g in pauli.diagonalizing_gates()]
+    return names
+
+
 def _rotated_samples(qdev, basis: str, n_shots: int, generator=None) -> torch.Tensor:
     """Outcome indices [bsz, n_shots] after rotating a copy of the state into ``basis``."""
     from .device import QuantumDevice
-    from .operators import op_name_dict
+    from .functional import func_name_dict
 
     n = qdev.n_wires
-    qc = QuantumDevice(n_wires=n, bsz=qdev.bsz, device=qdev.device)
-    qc.set_states(qdev.get_states_1d().detach())
-    names = {"X": "paulix", "Y": "pauliy", "Z": "pauliz", "I": "i"}
-    for w, ch in enumerate(basis):
-        for rot in op_name_dict[names[ch]]().diagonalizing_gates():
-            rot(qc, wires=w)
-    st = kernel_operand(_state_2d(qc))
+    state = qdev.get_states_1d().detach()
+    rotations = [(w, name) for w, ch in enumerate(basis) for name in _diagonalizing_names(ch)]
+    if rotations:
+        qc = QuantumDevice(n_wires=n, bsz=1, device=qdev.device)
+        qc.set_states(state)
+        for w, name in rotations:
+            func_name_dict[name](qc, wires=w)
+        state = _state_2d(qc)
+    st = kernel_operand(state)
     u = torch.rand(st.shape[0], int(n_shots), dtype=torch.float64, device=st.device, generator=generator)
     return _lib.sample(st, n, u)
 

@@ -26,6 +26,8 @@ torch-built operand and its autograd graph (``generic`` ops).
 from __future__ import annotations
 
 import ctypes
+import math
+import struct
 import weakref
 from typing import Dict, List, Optional
 
@@ -47,6 +49,9 @@ _WIDE_TYPES = {16, 17, 18, 19}                    # 4x4 dense operands
 
 KIND_ID = {engine.KIND_DENSE: 0, engine.KIND_CTRL: 1, engine.KIND_X: 2, engine.KIND_PHASE: 3,
            engine.KIND_DIAG: 4, engine.KIND_SWAP: 5}
+
+
+_CONTROLLED = (engine.KIND_CTRL, engine.KIND_X, engine.KIND_SWAP)
 
 
 def operand_size(type_id: int) -> int:
@@ -76,6 +81,26 @@ class BlockDesc(ctypes.Structure):
 
 
 assert ctypes.sizeof(GateDesc) == 80 and ctypes.sizeof(BlockOp) == 64 and ctypes.sizeof(BlockDesc) == 32
+
+
+# The same records packed by one call each (fields in order), for tables built every step:
+# setting the fields of a ctypes record one by one took 4 to 8 us a gate.
+_GATE = struct.Struct("=4iQ2q2i4Q")
+_BLOCK_OP = struct.Struct("=12i2Q")
+_BLOCK_DESC = struct.Struct("=4i2Q")
+_GATE_T = np.dtype({"names": ["op128", "op64", "op_grad", "grad"], "formats": ["u8"] * 4,
+                    "offsets": [48, 56, 64, 72], "itemsize": 80})
+_BLOCK_OP_T = np.dtype({"names": ["grad"], "formats": ["u8"], "offsets": [56], "itemsize": 64})
+_BLOCK_DESC_T = np.dtype({"names": ["gu"], "formats": ["u8"], "offsets": [24], "itemsize": 32})
+assert (_GATE.size, _BLOCK_OP.size, _BLOCK_DESC.size) == tuple(map(ctypes.sizeof, (GateDesc, BlockOp, BlockDesc)))
+
+
+def _upload(data, device):
+    """Packed records (bytes-like) -> (device uint8 tensor, its pinned staging copy)."""
+    src = np.frombuffer(data, dtype=np.uint8)
+    host = torch.empty(max(src.size, 1), dtype=torch.uint8, pin_memory=True)
+    host.numpy()[:src.size] = src
+    return host.to(device, non_blocking=True), host
 
 
 def _to_device_table(structs, device) -> torch.Tensor:
@@ -138,14 +163,17 @@ class Segment:
         self.natives = natives
         # operands laid out by shape: the natives of one operand shape are consecutive, so
         # their views come from one view + unbind per shape instead of per-gate slicing
-        shapes = [_operand_shape(g, operand_size(g.type_id)) for g in natives]
         by_shape: Dict[tuple, List[int]] = {}
-        for i, shp in enumerate(shapes):
+        shape_of: Dict[tuple, tuple] = {}
+        for i, g in enumerate(natives):
+            shp = shape_of.get((g.type_id, g.batch))
+            if shp is None:
+                shp = shape_of[g.type_id, g.batch] = _operand_shape(g, operand_size(g.type_id))
             by_shape.setdefault(shp, []).append(i)
         offsets = [0] * len(natives)
         total = 0
         for shp, idx in by_shape.items():
-            numel = int(np.prod(shp))
+            numel = math.prod(shp)
             for i in idx:
                 offsets[i] = total
                 total += numel
@@ -154,30 +182,24 @@ class Segment:
         views64, views128 = [None] * len(natives), [None] * len(natives)
         for shp, idx in by_shape.items():
             a, cnt = offsets[idx[0]], len(idx)
-            size = cnt * int(np.prod(shp))
+            size = cnt * math.prod(shp)
             for i, v64, v128 in zip(idx, self.op64[a:a + size].view(cnt, *shp).unbind(0),
                                     self.op128[a:a + size].view(cnt, *shp).unbind(0)):
                 views64[i], views128[i] = v64, v128
         self.gate_offsets = offsets
-        descs = []
         self._keep = []
         p64, p128 = self.op64.data_ptr(), self.op128.data_ptr()
+        table = bytearray()
+        pack = _GATE.pack
         for g, off in zip(natives, offsets):
             p = g.params
-            d = GateDesc()
-            d.type, d.inverse, d.batch, d.nparam = g.type_id, int(g.inverse), g.batch, g.nparam
-            d.p = p.data_ptr()
-            d.p_row_stride = p.stride(0) if g.batch > 1 else 0
-            d.p_col_stride = p.stride(1)
-            d.p_is_double = int(p.dtype == torch.float64)
-            d.op128 = p128 + 16 * off
-            d.op64 = p64 + 8 * off
-            descs.append(d)
-        self.gate_descs = descs
-        if descs:
-            table, host = _to_device_table(descs, dev)
-            self._keep += [table, host]
-            _lib.gate_operands(table, len(descs), dev)
+            table += pack(g.type_id, g.inverse, g.batch, g.nparam, p.data_ptr(), p.stride(0) if g.batch > 1 else 0,
+                          p.stride(1), p.dtype == torch.float64, 0, p128 + 16 * off, p64 + 8 * off, 0, 0)
+        self.gate_table = np.frombuffer(table, dtype=np.uint8).reshape(-1, _GATE.size)
+        if natives:
+            dev_table, host = _upload(table, dev)
+            self._keep += [dev_table, host]
+            _lib.gate_operands(dev_table, len(natives), dev)
         # ---- exec ops: one TapeOp per record (operands point into op64 / op128)
         ops = []
         gi = 0
@@ -187,6 +209,7 @@ class Segment:
                                    operand=views64[gi])
                 op.native = r
                 op.op128 = views128[gi]
+                op.ptr128 = p128 + 16 * offsets[gi]
                 gi += 1
             else:
                 op = r
@@ -236,11 +259,13 @@ class Segment:
             self.exec_ops = tile_runs(ops, n, self.bsz) if getattr(qdev, "stage_low", True) else ops
         # ---- differentiable inputs
         self.bases: Dict[int, tuple] = {}
-        for g in natives:
+        self.grad_gates = []  # (gate, its base's id, element offset of its parameters in the base)
+        for i, g in enumerate(natives):
             if g.params.requires_grad:
-                base, _ = _param_base(g.params)
+                base, eoff = _param_base(g.params)
                 self.bases.setdefault(id(base), (base, None))
-        self.generic_sources = [op for op in ops if not hasattr(op, "native") and op.needs_grad]
+                self.grad_gates.append((i, id(base), eoff))
+        self.generic_sources = [op for op in ops if op.native is None and op.needs_grad]
         self.diff_inputs = [b for b, _ in self.bases.values()] + [op.source for op in self.generic_sources]
 
     # -------------------------------------------------------------- blocks
@@ -269,31 +294,33 @@ class Segment:
         sizes = [b.block_batch * (1 << (2 * b.k)) for b in self.blocks]
         self.u128 = torch.empty(max(sum(sizes), 1), dtype=torch.complex128, device=dev)
         off = 0
-        bdescs, bops = [], []
+        # one upload: the ops' records, then the blocks'
+        table, descs = bytearray(), []
+        nops, p_u = 0, self.u128.data_ptr()
         for blk, sz in zip(self.blocks, sizes):
             d = 1 << blk.k
             blk.u128 = self.u128[off:off + sz].view(blk.block_batch, d, d)
+            blk.ptr_u = p_u + 16 * off
             off += sz
             where = {w: blk.k - 1 - i for i, w in enumerate(blk.wires)}
-            bd = BlockDesc()
-            bd.first_op, bd.num_ops, bd.k, bd.batch = len(bops), len(blk.members), blk.k, blk.block_batch
-            bd.u = blk.u128.data_ptr()
-            bd.gu = None
-            bdescs.append(bd)
+            descs.append((nops, len(blk.members), blk.k, blk.block_batch, blk.ptr_u, 0))
+            nops += len(blk.members)
             for m in blk.members:
-                bops.append(self._block_op(m, where))
-        self.block_descs, self.block_ops = bdescs, bops
-        bt, bh = _to_device_table(bdescs, dev)
-        ot, oh = _to_device_table(bops, dev)
-        self._keep += [bt, bh, ot, oh]
-        maxb = max(b.block_batch for b in self.blocks)
-        _lib.block_build(bt, len(bdescs), maxb, ot, dev)
+                table += self._block_op(m, where)
+        self.num_block_ops = nops
+        for d in descs:
+            table += _BLOCK_DESC.pack(*d)
+        self.block_table = table
+        self.max_block_batch = max(b.block_batch for b in self.blocks)
+        dev_table, host = _upload(table, dev)
+        self._keep += [dev_table, host]
+        _lib.block_build(dev_table[64 * nops:], len(descs), self.max_block_batch, dev_table, dev)
         for blk in self.blocks:
             if not blk.tc:
                 blk.operand = blk.u128.to(torch.complex64)
         self._prepare_images(adjoint=False)
         # keep operands of non-native members alive in complex128
-        self._member128 = [getattr(m, "_op128_keep", None) for b in self.blocks for m in b.members]
+        self._member128 = [m._op128_keep for b in self.blocks for m in b.members]
 
     def _prepare_images(self, adjoint: bool) -> None:
         """Tensor-core operand images of every block of the segment (of U, or of U^H for
@@ -320,24 +347,21 @@ class Segment:
         setattr(self, "_keep_images_h" if adjoint else "_keep_images", (table, host))
         _lib.fused_prepare_many(table, len(jobs), max(b.block_batch for b in tcb))
 
-    def _block_op(self, m, where):
-        bo = BlockOp()
-        bo.kind = KIND_ID[m.kind]
-        wires = m.wires
-        bo.nw = len(wires)
-        for j, w in enumerate(wires):
-            bo.pos[j] = where[w]
-        bo.nctrl = len(m.controls) if m.kind in (engine.KIND_CTRL, engine.KIND_X, engine.KIND_SWAP) else 0
-        bo.ctrl_val = m.ctrl_val
-        if m.kind in (engine.KIND_X, engine.KIND_SWAP):
-            bo.batch, bo.op_size, bo.operand = 1, 1, self._dummy_ptr()
-            return bo
-        o128 = m.op128 if hasattr(m, "op128") else _generic128(m)
-        bo.batch = int(o128.shape[0])
-        bo.op_size = int(o128[0].numel())
-        bo.operand = o128.data_ptr()
-        bo.grad = None
-        return bo
+    def _block_op(self, m, where) -> bytes:
+        """The ``tqk_block_op`` record of a block's member (no cotangent slot)."""
+        pos = [where[w] for w in m.wires]
+        nw = len(pos)
+        pos += [0] * (6 - nw)
+        k = m.kind
+        nctrl = len(m.controls) if k in _CONTROLLED else 0
+        if k in (engine.KIND_X, engine.KIND_SWAP):
+            return _BLOCK_OP.pack(KIND_ID[k], nw, *pos, nctrl, m.ctrl_val, 1, 1, self._dummy_ptr(), 0)
+        if m.native is not None:
+            return _BLOCK_OP.pack(KIND_ID[k], nw, *pos, nctrl, m.ctrl_val, m.native.batch,
+                                  operand_size(m.native.type_id), m.ptr128, 0)
+        o128 = _generic128(m)
+        return _BLOCK_OP.pack(KIND_ID[k], nw, *pos, nctrl, m.ctrl_val, o128.shape[0], o128[0].numel(),
+                              o128.data_ptr(), 0)
 
     def _dummy_ptr(self):
         if not hasattr(self, "_dummy"):
@@ -364,7 +388,7 @@ class Segment:
         for i, op in enumerate(self.exec_ops):
             if isinstance(op, StagedRun):
                 recs.append(_staged_record(op, op.descs(), keep))
-            elif getattr(op, "members", None) is not None:
+            elif op.members is not None:
                 if not op.tc:
                     recs.append(_exec(_lib.X_BLOCK_DENSE, op.wires, batch=op.block_batch, operand=op.operand))
                     continue
@@ -460,14 +484,14 @@ class Segment:
                 for m in op.ops:
                     slot = None
                     if need_grads:
-                        if hasattr(m, "native") and m.native.params.requires_grad:
-                            slot = m.op128.data_ptr() + dopg
+                        if m.native is not None and m.native.params.requires_grad:
+                            slot = m.ptr128 + dopg
                         elif id(m) in gslots:
                             slot = torch.view_as_real(gslots[id(m)]).view(-1)
                     slots.append(slot)
                 recs.append(_staged_record(op, op.descs(slots), keep))
                 continue
-            if getattr(op, "members", None) is not None:
+            if op.members is not None:
                 slot = None
                 if gu is not None and _block_needs_grad(op):
                     slot = _as_real(gu, op.u128, self.u128)
@@ -495,8 +519,8 @@ class Segment:
                 continue
             slot = None
             if need_grads:
-                if hasattr(op, "native") and op.native.params.requires_grad:
-                    slot = op.op128.data_ptr() + dopg
+                if op.native is not None and op.native.params.requires_grad:
+                    slot = op.ptr128 + dopg
                 elif id(op) in gslots:
                     slot = torch.view_as_real(gslots[id(op)]).view(-1)
             recs.append(_plain_record(op, slot))
@@ -521,29 +545,23 @@ class Segment:
             return [None] * len(self.diff_inputs)
         # block cotangents -> member operand cotangents
         if self.blocks and gu is not None:
-            bops = []
-            bdescs = []
-            for bi, blk in enumerate(self.blocks):
-                bd = BlockDesc()
-                src = self.block_descs[bi]
-                bd.first_op, bd.num_ops, bd.k, bd.batch = src.first_op, src.num_ops, src.k, src.batch
-                bd.u = blk.u128.data_ptr()
-                bd.gu = gu.data_ptr() + (blk.u128.data_ptr() - self.u128.data_ptr()) \
-                    if _block_needs_grad(blk) else None
-                bdescs.append(bd)
-                for m, src_op in zip(blk.members, self.block_ops[src.first_op:src.first_op + src.num_ops]):
-                    bo = BlockOp.from_buffer_copy(src_op)
-                    bo.grad = None
-                    if hasattr(m, "native") and m.native.params.requires_grad:
-                        bo.grad = opg.data_ptr() + (m.op128.data_ptr() - self.op128.data_ptr())
-                    elif id(m) in gslots:
-                        bo.grad = gslots[id(m)].data_ptr()
-                    bops.append(bo)
-            bt, bh = _to_device_table(bdescs, dev)
-            ot, oh = _to_device_table(bops, dev)
-            maxb = max(b.block_batch for b in self.blocks)
-            _lib.block_unbuild(bt, len(bdescs), maxb, ot, dev)
-            self._keep_bw = [bt, bh, ot, oh]
+            nops = self.num_block_ops
+            table = bytearray(self.block_table)
+            grad_col = np.frombuffer(table, dtype=_BLOCK_OP_T, count=nops)["grad"]
+            gu_col = np.frombuffer(table, dtype=_BLOCK_DESC_T, offset=64 * nops)["gu"]
+            dgu = gu.data_ptr() - self.u128.data_ptr()
+            slots = []
+            for m in (m for blk in self.blocks for m in blk.members):
+                if m.native is not None and m.native.params.requires_grad:
+                    slots.append(m.ptr128 + dopg)
+                else:
+                    g = gslots.get(id(m))
+                    slots.append(0 if g is None else g.data_ptr())
+            grad_col[:] = slots
+            gu_col[:] = [blk.ptr_u + dgu if _block_needs_grad(blk) else 0 for blk in self.blocks]
+            dev_table, host = _upload(table, dev)
+            _lib.block_unbuild(dev_table[64 * nops:], len(self.blocks), self.max_block_batch, dev_table, dev)
+            self._keep_bw = [dev_table, host]
         # operand cotangents -> parameter gradients
         grads = []
         if self.natives and self.bases:
@@ -554,22 +572,17 @@ class Segment:
             starts = np.cumsum([0] + spans[:-1]).tolist()
             flat = torch.zeros(max(sum(spans), 1), dtype=torch.float64, device=dev)
             start_of = {k: st for k, st in zip(self.bases.keys(), starts)}
-            descs = []
-            fp = flat.data_ptr()
-            for g, d, off in zip(self.natives, self.gate_descs, self.gate_offsets):
-                if not g.params.requires_grad:
-                    continue
-                base, eoff = _param_base(g.params)
-                nd = GateDesc.from_buffer_copy(d)
-                nd.op128 = None
-                nd.op64 = None
-                nd.op_grad = opg.data_ptr() + 16 * off
-                nd.grad = fp + 8 * (start_of[id(base)] + eoff)
-                descs.append(nd)
-            if descs:
-                table, host = _to_device_table(descs, dev)
-                _lib.param_grads(table, len(descs), dev)
-                self._keep_pg = [table, host]
+            if self.grad_gates:
+                rows = [i for i, _, _ in self.grad_gates]
+                table = self.gate_table[rows]  # a copy
+                col = table.reshape(-1).view(_GATE_T)
+                col["op128"] = 0
+                col["op64"] = 0
+                col["op_grad"] = [opg.data_ptr() + 16 * self.gate_offsets[i] for i in rows]
+                col["grad"] = [flat.data_ptr() + 8 * (start_of[base] + eoff) for _, base, eoff in self.grad_gates]
+                dev_table, host = _upload(table, dev)
+                _lib.param_grads(dev_table, len(rows), dev)
+                self._keep_pg = [dev_table, host]
             dtypes = {b.dtype for b in bases}
             conv = flat.to(bases[0].dtype) if len(dtypes) == 1 else None
             for b, st in zip(bases, starts):
@@ -587,20 +600,20 @@ _PLAIN_KIND = {engine.KIND_DENSE: _lib.X_DENSE, engine.KIND_CTRL: _lib.X_CTRL, e
                engine.KIND_PHASE: _lib.X_PHASE, engine.KIND_DIAG: _lib.X_DIAG, engine.KIND_SWAP: _lib.X_SWAP}
 
 
+EXEC_MAX_WIRES = len(_lib.ExecOp().wires)
+
+
+def _address(t):
+    return t if t is None or isinstance(t, int) else t.data_ptr()
+
+
 def _exec(kind: int, wires, nctrl: int = 0, ctrl_val: int = 1, batch: int = 1, operand=None, uncompute=None,
           image=None, image_h=None, u=None, grad=None, mr=None) -> "_lib.ExecOp":
     """One ``tqk_exec_op`` record (tensors, or device addresses as ints)."""
-    r = _lib.ExecOp()
-    r.kind, r.nw, r.nctrl, r.ctrl_val, r.batch = kind, len(wires), nctrl, ctrl_val, batch
-    if len(wires) > len(r.wires):
-        raise _lib.TQKError(1, f"an op on {len(wires)} wires exceeds the {len(r.wires)} one op may touch")
-    for j, w in enumerate(wires):
-        r.wires[j] = w
-    for name, t in (("operand", operand), ("uncompute", uncompute), ("image", image), ("image_h", image_h),
-                    ("u", u), ("grad", grad), ("mr", mr)):
-        if t is not None:
-            setattr(r, name, t if isinstance(t, int) else t.data_ptr())
-    return r
+    if len(wires) > EXEC_MAX_WIRES:
+        raise _lib.TQKError(1, f"an op on {len(wires)} wires exceeds the {EXEC_MAX_WIRES} one op may touch")
+    return _lib.ExecOp(kind, len(wires), nctrl, ctrl_val, tuple(wires), batch, _address(operand), _address(uncompute),
+                       _address(image), _address(image_h), _address(u), None, None, _address(grad), _address(mr))
 
 
 def _plain_record(op, grad=None) -> "_lib.ExecOp":
@@ -697,25 +710,19 @@ class StagedRun:
     def _build_descs(self):
         out = []
         for o in self.ops:
-            d = _lib.StagedOp()
+            kind, ctrl_val = _lib.S_DIAG, 0
+            ws = o.wires
             if o.kind == engine.KIND_X:
-                ws, d.kind, d.ctrl_val = o.controls + o.targets, _lib.S_X, o.ctrl_val
-            elif o.kind in (engine.KIND_DENSE, engine.KIND_CTRL):
-                ws, d.kind = (o.controls + o.targets) if o.kind == engine.KIND_CTRL else o.wires, _lib.S_DENSE1
+                ws, kind, ctrl_val = o.controls + o.targets, _lib.S_X, o.ctrl_val
+            elif o.kind == engine.KIND_CTRL:
+                ws, kind = o.controls + o.targets, _lib.S_DENSE1
+            elif o.kind == engine.KIND_DENSE:
+                kind = _lib.S_DENSE1
             elif o.kind == engine.KIND_PHASE:
-                ws, d.kind = o.wires, _lib.S_PHASE
-            else:
-                ws, d.kind = o.wires, _lib.S_DIAG
-            d.nwires = len(ws)
-            for j, w in enumerate(ws):
-                d.wires[j] = w
-            if o.kind != engine.KIND_X:
-                d.operand = o.operand.data_ptr()
-                d.batch = int(o.operand.shape[0])
-            else:
-                d.batch = 1
-            d.grad = None
-            out.append(d)
+                kind = _lib.S_PHASE
+            flip = o.kind == engine.KIND_X
+            out.append(_lib.StagedOp(kind, len(ws), tuple(ws), ctrl_val, 0, None if flip else o.operand.data_ptr(),
+                                     1 if flip else o.operand.shape[0], None))
         return out
 
 
@@ -870,13 +877,19 @@ def _as_real(buf: torch.Tensor, view: torch.Tensor, base: torch.Tensor) -> torch
 
 
 def _block_needs_grad(blk) -> bool:
-    return any((hasattr(m, "native") and m.native.params.requires_grad) or m.needs_grad for m in blk.members)
+    return any((m.native is not None and m.native.params.requires_grad) or m.needs_grad for m in blk.members)
 
 
 def _generic128(m) -> torch.Tensor:
-    t = m.source if m.source is not None else m.operand
-    t = engine.kernel_operand(t.to(torch.complex128))
+    const = m.const
+    if const is not None and const._op128_keep is not None:
+        m._op128_keep = const._op128_keep
+        return m._op128_keep
+    src = m.source if m.source is not None else m.operand
+    t = engine.kernel_operand(src.to(torch.complex128))
     m._op128_keep = t
+    if const is not None and t.data_ptr() == src.data_ptr():  # a view of the constant: no work was queued for it
+        const._op128_keep = t
     return t
 
 
@@ -886,7 +899,7 @@ def planner_wires(ops, n: int) -> List[List[int]]:
     7 placeholder wires, wider than any block, so every planner leaves it alone (also when
     n <= 6, where all n wires would fit in one block)."""
     barrier = list(range(n)) + [-1 - i for i in range(7)]
-    return [list(op.wires) if fusable(op) else barrier for op in ops]
+    return [op.wires if fusable(op) else barrier for op in ops]
 
 
 def fusable(op) -> bool:
