@@ -151,9 +151,11 @@ __global__ void __launch_bounds__(256) k_dense(const DenseParams<D> p) {
 // Memory bound where the loads in flight cover the latency: D = 4 keeps 32 matrix values and
 // 32 sums in registers, so 128 threads and 4 CTAs per SM instead of 256 and 1.  A thread takes
 // up to kStoredIter pairs of groups (stride: the grid), so that the block's reduction is paid
-// once for all of them while its float32 sums stay short.  n = 21, bsz = 8 (3 S = 403 MB): 62 us
-// for one wire, 74 us for two, where the in-place step took 106 and 213 us beside three copies
-// of 42 us.
+// once for all of them; a pair's products are summed before they join the thread's float32 sums
+// and the last steps of the warp's are in float64, so the cotangent's error stays below that of
+// one pair a thread (n = 21, two wires: 7.7e-8 of its norm either way; 1.06e-7 without both).
+// n = 21, bsz = 8 (3 S = 403 MB): 68 us for one wire, 85 us for two (74 and 135 with one pair a
+// thread), where the in-place step took 106 and 213 us beside three copies of 42 us.
 template <int D>
 struct StoredParams {
   DenseParams<D> d;       // ins, off, pair, mat, grad, groups
@@ -163,11 +165,13 @@ struct StoredParams {
 };
 
 // Sum NV = 8 or 32 values over the warp by halves: NV - 1 exchanges (then plain ones for
-// NV = 8) instead of 5 NV.  Lane L ends with the sum of value L * NV / 32.
+// NV = 8) instead of 5 NV, the first two in float32, the others in float64 (7 or 3 additions).
+// Lane L ends with the sum of value L * NV / 32.
 template <int NV>
-__device__ __forceinline__ float warp_sum(float (&v)[NV], int lane) {
+__device__ __forceinline__ double warp_sum(float (&v)[NV], int lane) {
+  double s[NV / 4];
 #pragma unroll
-  for (int h = NV / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+  for (int h = NV / 2, o = 16; h >= NV / 4; h >>= 1, o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int i = 0; i < h; ++i) {
@@ -175,10 +179,21 @@ __device__ __forceinline__ float warp_sum(float (&v)[NV], int lane) {
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  float s = v[0];
 #pragma unroll
-  for (int o = 16 / NV; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
+  for (int i = 0; i < NV / 4; ++i) s[i] = v[i];
+#pragma unroll
+  for (int h = NV / 8, o = 4; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double send = up ? s[i] : s[i + h], keep = up ? s[i + h] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  double t = s[0];
+#pragma unroll
+  for (int o = 16 / NV; o >= 1; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
 }
 
 template <int D>
@@ -211,27 +226,25 @@ __global__ void __launch_bounds__(kStoredThreads<D>, D == 4 ? 4 : 3)
     store_groups<D, MODE>(q.out + (b << p.n), p, g0, two, z);
     if (GRAD) {
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int r = 0; r < D; ++r)
 #pragma unroll
-        for (int r = 0; r < D; ++r)
-#pragma unroll
-          for (int c = 0; c < D; ++c) {
-            const float2 v = cfma_bconj(l[j][r], a[j][c], make_float2(acc[2 * (r * D + c)], acc[2 * (r * D + c) + 1]));
-            acc[2 * (r * D + c)] = v.x;
-            acc[2 * (r * D + c) + 1] = v.y;
-          }
+        for (int c = 0; c < D; ++c) {  // the pair's sum by itself first: short chains of roundings
+          const float2 v = cfma_bconj(l[1][r], a[1][c], cfma_bconj(l[0][r], a[0][c], make_float2(0.f, 0.f)));
+          acc[2 * (r * D + c)] += v.x;
+          acc[2 * (r * D + c) + 1] += v.y;
+        }
     }
   }
   if constexpr (GRAD) {
     constexpr int NV = 2 * D * D;
-    __shared__ float red[kStoredThreads<D> / 32][NV];
+    __shared__ double red[kStoredThreads<D> / 32][NV];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float s = warp_sum<NV>(acc, lane);
+    const double s = warp_sum<NV>(acc, lane);
     if (lane % (32 / NV) == 0) red[warp][lane * NV / 32] = s;
     __syncthreads();
     if (threadIdx.x < NV) {
       double t = 0.0;
-      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += static_cast<double>(red[w][threadIdx.x]);
+      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += red[w][threadIdx.x];
       atomicAdd(p.grad + b * p.grad_stride + threadIdx.x, t);
     }
   }
