@@ -97,6 +97,10 @@ int tqk_probs(const void* state, int64_t bsz, int n, float* out, void* stream);
 int64_t tqk_sample_scratch_bytes(int64_t bsz, int n);
 int tqk_sample(const void* state, int64_t bsz, int n, const double* uniforms, int64_t shots, int64_t* out,
                void* scratch, int64_t scratch_bytes, void* stream);
+/* out[j*bsz + b] = mean over row b's shots (outcomes[b*shots + s], int64) of
+ * (-1)^popcount(outcome & masks[j]): the sampled value of m Z-type strings (masks: host). */
+int tqk_sample_parity(const int64_t* outcomes, int64_t bsz, int64_t shots, const uint64_t* masks, int m,
+                      float* out, void* stream);
 
 /* Expectation values of m Pauli strings, out[b*m + j] = Re <psi_b| P_j |psi_b> (float64).
  * P_j is given by bit masks over the in-row index (bit n-1-w <-> wire w):

@@ -66,6 +66,7 @@ _SIGS = {
     "tqk_fused_cross_add_many": (_int, [_vp, _int, _i64, _vp]),
     "tqk_sample_scratch_bytes": (_i64, [_i64, _int]),
     "tqk_sample": (_int, [_vp, _i64, _int, _vp, _i64, _vp, _vp, _i64, _vp]),
+    "tqk_sample_parity": (_int, [_vp, _i64, _i64, _u64p, _int, _vp, _vp]),
     "tqk_staged_apply": (_int, [_vp, _i64, _int, _vp, _int, _int, _vp, _vp]),
     "tqk_staged_adjoint": (_int, [_vp, _vp, _i64, _int, _vp, _int, _int, _vp, _vp]),
     "tqk_tiled_apply": (_int, [_vp, _i64, _int, _vp, _int, ctypes.c_uint64, _vp, _vp]),
@@ -319,6 +320,18 @@ def sample(state, n, uniforms):
     scratch = torch.empty(max(1, nbytes // 8), dtype=torch.float64, device=state.device)
     _check(lib.tqk_sample(state.data_ptr(), bsz, n, uniforms.data_ptr(), shots, out.data_ptr(), scratch.data_ptr(),
                           nbytes, _stream(state)), launches=3)
+    return out
+
+
+def sample_parity(outcomes, masks):
+    """Means over the shots of (-1)^popcount(outcome & mask): outcomes [bsz, shots] int64,
+    masks m integers -> [m, bsz] float32."""
+    bsz, shots = outcomes.shape
+    if shots == 0:  # a mean of nothing
+        return torch.full((len(masks), bsz), float("nan"), dtype=torch.float32, device=outcomes.device)
+    out = torch.empty(len(masks), bsz, dtype=torch.float32, device=outcomes.device)
+    _check(load().tqk_sample_parity(outcomes.data_ptr(), bsz, shots, _u64(masks), len(masks), out.data_ptr(),
+                                    _stream(outcomes)), launches=(len(masks) + 31) // 32)
     return out
 
 

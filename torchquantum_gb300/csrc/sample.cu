@@ -3,12 +3,17 @@
 // Upstream's tq.measure copies |psi|^2 to the host and draws shots with
 // random.choices (measurement/measurements.py:37-74).  Here each shot is an inverse-CDF
 // draw on the device: given a uniform u in [0, 1), the outcome is the first index i
-// whose running sum of |psi_j|^2 (j <= i) exceeds u * sum_j |psi_j|^2.  Three kernels:
+// whose running sum of |psi_j|^2 (j <= i) exceeds u * sum_j |psi_j|^2.  Kernels:
 //   k_tile_sums  one warp per tile of 2^tb amplitudes: the tile's probability (float64);
 //   k_tile_scan  one block per row: inclusive prefix sums of the tile probabilities;
-//   k_draw       one thread per (row, shot): binary search over the tile prefixes, then
-//                a running sum over the chosen tile's amplitudes.
+//   k_draw       one warp per (row, shot): search over the tile prefixes, then the running
+//                sum over the chosen tile's amplitudes;
+//   k_parity     one block per (row, string): the share of even minus odd parities of the
+//                outcomes on a string's sites.
 // Uniforms come from the caller (a seeded torch generator), so draws are reproducible.
+//
+// What bounds them: float64 (one warp operation in 16 cycles) in the sums and the scan; reads
+// of one tile per shot in the draw.
 #include <stdint.h>
 
 #include "common.cuh"
@@ -17,6 +22,11 @@ namespace tqk {
 namespace sample {
 
 constexpr int kTileBits = 8;
+constexpr int kDrawWarps = 8;  // warps of a k_draw block
+constexpr int kParityStrings = 32;  // strings a launch
+struct ParityMasks {
+  unsigned long long m[kParityStrings];
+};
 
 __device__ __forceinline__ double prob(float2 a) { return (double)a.x * a.x + (double)a.y * a.y; }
 
@@ -29,67 +39,160 @@ __global__ void __launch_bounds__(256) k_tile_sums(const float2* state, int n, i
   if (tile >= ntiles) return;
   const float2* src = state + (b << n) + (tile << tb);
   double s = 0.0;
-  for (int j = lane; j < (1 << tb); j += 32) s += prob(src[j]);
+  for (int j = lane; j < (1 << tb); j += 32) {
+    const double x = src[j].x, y = src[j].y;
+    s = fma(x, x, fma(y, y, s));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) tile_sum[b * ntiles + tile] = s;
 }
 
-// one block (1024 threads) per row: in-place inclusive scan in chunks of 1024
+// One block (1024 threads) per row: in-place inclusive scan in chunks of 8192: a thread's 8
+// values, the warp's threads, the block's warps.  (Ten additions a value, all in float64, took
+// 21 us for 4 rows of 4096 tiles.)
+constexpr int kScanPer = 8;
 __global__ void __launch_bounds__(1024) k_tile_scan(double* tile_sum, int64_t ntiles) {
-  __shared__ double buf[1024];
-  __shared__ double carry;
+  __shared__ double warp_sum[32];
   double* row = tile_sum + (int64_t)blockIdx.x * ntiles;
-  if (threadIdx.x == 0) carry = 0.0;
-  __syncthreads();
-  for (int64_t base = 0; base < ntiles; base += 1024) {
-    const int64_t i = base + threadIdx.x;
-    buf[threadIdx.x] = i < ntiles ? row[i] : 0.0;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {  // Hillis-Steele scan
-      const double v = threadIdx.x >= off ? buf[threadIdx.x - off] : 0.0;
-      __syncthreads();
-      buf[threadIdx.x] += v;
-      __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double carry = 0.0;
+  for (int64_t base = 0; base < ntiles; base += 1024 * kScanPer) {
+    const int64_t i0 = base + (int64_t)threadIdx.x * kScanPer;
+    double v[kScanPer];
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+      v[k] = i0 + k < ntiles ? row[i0 + k] : 0.0;
+      if (k > 0) v[k] += v[k - 1];
     }
-    if (i < ntiles) row[i] = buf[threadIdx.x] + carry;
+    double incl = v[kScanPer - 1];  // of the warp's threads up to this one
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 1023) carry += buf[1023];
+    if (warp == 0) {
+      double w = warp_sum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += u;
+      }
+      warp_sum[lane] = w;
+    }
+    __syncthreads();
+    const double up = __shfl_up_sync(0xffffffffu, incl, 1);
+    const double before = carry + ((warp > 0 ? warp_sum[warp - 1] : 0.0) + (lane > 0 ? up : 0.0));
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k)
+      if (i0 + k < ntiles) row[i0 + k] = before + v[k];
+    carry += warp_sum[31];
     __syncthreads();
   }
 }
 
+// The draw within a tile, amplitude by amplitude in float64.
+__device__ int64_t draw_in_tile(const float2* src, int count, double before, double target) {
+  double acc = before;
+  int64_t last_nonzero = 0;
+  for (int j = 0; j < count; ++j) {
+    const double p = prob(src[j]);
+    if (p > 0.0) last_nonzero = j;
+    acc += p;
+    if (acc > target) return j;
+  }
+  return last_nonzero;  // rounding left target at the tile's end
+}
+
+// One warp per shot.  The tile: the first whose inclusive prefix exceeds the target, 32 places
+// at a time.  Within it a lane sums 8 neighbouring amplitudes: float32 sums tell the outcome
+// apart wherever the target is farther from both of its ends than their error (all but about
+// one shot in 5000); the others go through the tile in float64.  Outcomes are the float64
+// ones either way.  n = 20, 4 rows, 8192 shots: 118 -> @@ us (a thread per shot walked its
+// tile alone).
 __global__ void __launch_bounds__(256) k_draw(const float2* state, int n, int tb, int64_t ntiles,
                                               const double* prefix, const double* uniforms, int64_t shots,
                                               int64_t* out) {
   const int64_t b = blockIdx.y;
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= shots) return;
+  const int lane = threadIdx.x & 31;
   const double* pre = prefix + b * ntiles;
   const double total = pre[ntiles - 1];
-  const double target = uniforms[b * shots + s] * total;
-  // first tile whose inclusive prefix exceeds target
-  int64_t lo = 0, hi = ntiles - 1;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (pre[mid] > target) hi = mid;
-    else lo = mid + 1;
-  }
-  const double before = lo > 0 ? pre[lo - 1] : 0.0;
-  const float2* src = state + (b << n) + (lo << tb);
-  double acc = before;
-  int64_t pick = -1, last_nonzero = 0;
-  for (int j = 0; j < (1 << tb); ++j) {
-    const double p = prob(src[j]);
-    if (p > 0.0) last_nonzero = j;
-    acc += p;
-    if (acc > target) {
-      pick = j;
-      break;
+  for (int64_t s = (int64_t)blockIdx.x * kDrawWarps + (threadIdx.x >> 5); s < shots; s += (int64_t)gridDim.x * kDrawWarps) {
+    const double target = uniforms[b * shots + s] * total;
+    int64_t lo = 0, hi = ntiles - 1;  // the tile lies in [lo, hi]
+    while (lo < hi) {
+      const int64_t step = (hi - lo + 32) >> 5;  // pieces of `step` tiles, a lane each: their last tiles
+      const int64_t at = min(lo + (lane + 1) * step - 1, hi);
+      const uint32_t over = __ballot_sync(0xffffffffu, pre[at] > target);
+      const int first = over ? __ffs(over) - 1 : 31;
+      const int64_t l2 = lo + first * step;
+      hi = min(l2 + step - 1, hi);
+      lo = min(l2, hi);
     }
+    const double before = lo > 0 ? pre[lo - 1] : 0.0;
+    const float2* src = state + (b << n) + (lo << tb);
+    int64_t pick = -1;
+    if (tb == kTileBits) {
+      float c[8];  // running sums over the lane's amplitudes
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 v = ld4(src + 8 * lane + 2 * k);
+        c[2 * k] = fmaf(v.x, v.x, v.y * v.y) + (k > 0 ? c[2 * k - 1] : 0.f);
+        c[2 * k + 1] = fmaf(v.z, v.z, v.w * v.w) + c[2 * k];
+      }
+      float incl = c[7];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      const float all = __shfl_sync(0xffffffffu, incl, 31);
+      const float start = incl - c[7];
+      const float t = static_cast<float>(target - before);
+      // float32: at most 16 roundings of sums up to `all` (and the one of t); float64: the walk's
+      // 256 additions, on sums up to `total`; the last term: float32 underflow
+      const float margin = 32.f * 5.9604645e-8f * (all + fabsf(t)) + static_cast<float>(total * 1e-12) + 1e-37f;
+      int j = 8;  // the lane's first amplitude whose sum exceeds t
+#pragma unroll
+      for (int k = 7; k >= 0; --k)
+        if (start + c[k] > t) j = k;
+      const uint32_t who = __ballot_sync(0xffffffffu, j < 8);
+      if (who != 0) {
+        const int w = __ffs(who) - 1;
+        float below = start, above = start;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (k == j) above = start + c[k];
+          if (k == j - 1) below = start + c[k];
+        }
+        const bool sure = above - t > margin && t - below > margin;
+        if (__shfl_sync(0xffffffffu, sure ? 1 : 0, w)) pick = 8 * w + __shfl_sync(0xffffffffu, j, w);
+      }
+    }
+    if (pick < 0) pick = draw_in_tile(src, 1 << tb, before, target);  // every lane the same
+    if (lane == 0) out[b * shots + s] = (lo << tb) + pick;
   }
-  if (pick < 0) pick = last_nonzero;  // rounding left target at the tile's end
-  out[b * shots + s] = (lo << tb) + pick;
+}
+
+// out[string][row] = mean over the shots of (-1)^popcount(outcome & mask)
+__global__ void __launch_bounds__(256) k_parity(const int64_t* outcomes, int64_t shots, const ParityMasks masks,
+                                                int64_t bsz, float* out) {
+  __shared__ unsigned long long odd;
+  const int64_t b = blockIdx.x;
+  const unsigned long long mask = masks.m[blockIdx.y];
+  if (threadIdx.x == 0) odd = 0;
+  __syncthreads();
+  unsigned long long mine = 0;
+  for (int64_t s = threadIdx.x; s < shots; s += blockDim.x) {
+    mine += __popcll(static_cast<unsigned long long>(outcomes[b * shots + s]) & mask) & 1;
+  }
+  if (mine) atomicAdd(&odd, mine);
+  __syncthreads();
+  if (threadIdx.x == 0)
+    out[blockIdx.y * bsz + b] = static_cast<float>(
+        static_cast<double>(shots - 2 * static_cast<int64_t>(odd)) * (1.0 / static_cast<double>(shots)));
 }
 
 }  // namespace sample
@@ -123,7 +226,28 @@ extern "C" int tqk_sample(const void* state, int64_t bsz, int n, const double* u
   cudaStream_t s = as_stream(stream);
   sample::k_tile_sums<<<dim3((unsigned)((ntiles + 7) / 8), (unsigned)bsz), 256, 0, s>>>(st, n, tb, ntiles, pre);
   sample::k_tile_scan<<<(unsigned)bsz, 1024, 0, s>>>(pre, ntiles);
-  sample::k_draw<<<dim3((unsigned)((shots + 255) / 256), (unsigned)bsz), 256, 0, s>>>(st, n, tb, ntiles, pre,
+  const int64_t blocks = (shots + sample::kDrawWarps - 1) / sample::kDrawWarps;
+  sample::k_draw<<<dim3((unsigned)(blocks < (1 << 20) ? blocks : (1 << 20)), (unsigned)bsz),
+                   32 * sample::kDrawWarps, 0, s>>>(st, n, tb, ntiles, pre,
                                                                                       uniforms, shots, out);
   return launch_status(what);
+}
+
+extern "C" int tqk_sample_parity(const int64_t* outcomes, int64_t bsz, int64_t shots, const uint64_t* masks, int m,
+                                 float* out, void* stream) {
+  const char* what = "tqk_sample_parity";
+  if (bsz < 1 || bsz > 0x7fffffffll) return fail(TQK_BAD_SHAPE, "%s: bsz %lld", what, (long long)bsz);
+  if (shots < 1) return fail(TQK_BAD_SHAPE, "%s: shots %lld", what, (long long)shots);
+  if (m <= 0) return TQK_OK;
+  if (!outcomes || !masks || !out) return fail(TQK_BAD_POINTER, "%s: null pointer", what);
+  for (int j0 = 0; j0 < m; j0 += sample::kParityStrings) {
+    const int cnt = m - j0 < sample::kParityStrings ? m - j0 : sample::kParityStrings;
+    sample::ParityMasks pm;
+    for (int j = 0; j < sample::kParityStrings; ++j) pm.m[j] = j < cnt ? masks[j0 + j] : 0ull;
+    sample::k_parity<<<dim3((unsigned)bsz, (unsigned)cnt), 256, 0, as_stream(stream)>>>(outcomes, shots, pm, bsz,
+                                                                                       out + (int64_t)j0 * bsz);
+    const int rc = launch_status(what);
+    if (rc) return rc;
+  }
+  return TQK_OK;
 }

@@ -229,12 +229,6 @@ def find_observable_groups(observables: Sequence[str]) -> Dict[str, List[str]]:
     return groups
 
 
-def _parity64(v: torch.Tensor) -> torch.Tensor:
-    for sh in (32, 16, 8, 4, 2, 1):
-        v = v ^ (v >> sh)
-    return v & 1
-
-
 _ROTATIONS: dict = {}
 
 
@@ -268,13 +262,10 @@ def _rotated_samples(qdev, basis: str, n_shots: int, generator=None) -> torch.Te
     return _lib.sample(st, n, u)
 
 
-def _sampled_expval(idx: torch.Tensor, observable: str, n: int) -> torch.Tensor:
-    mask = 0
-    for w, ch in enumerate(observable):
-        if ch != "I":
-            mask |= 1 << (n - 1 - w)
-    par = _parity64(idx & mask)
-    return (1.0 - 2.0 * par.to(torch.float64)).mean(dim=1).to(torch.float32)
+def _sampled_expvals(idx: torch.Tensor, observables: Sequence[str], n: int) -> torch.Tensor:
+    """[m, bsz] float32: each string's mean over the outcomes ``idx``."""
+    masks = [sum(1 << (n - 1 - w) for w, ch in enumerate(o) if ch != "I") for o in observables]
+    return _lib.sample_parity(idx, masks)
 
 
 def expval_joint_sampling(qdev, observable: str, n_shots: int = 1024, generator=None) -> torch.Tensor:
@@ -283,7 +274,7 @@ def expval_joint_sampling(qdev, observable: str, n_shots: int = 1024, generator=
     share with odd parity, counted on the GPU."""
     observable = observable.upper()
     idx = _rotated_samples(qdev, observable, n_shots, generator)
-    return _sampled_expval(idx, observable, qdev.n_wires)
+    return _sampled_expvals(idx, [observable], qdev.n_wires)[0]
 
 
 def expval_joint_sampling_grouping(qdev, observables: Sequence[str], n_shots_per_group: int = 1024,
@@ -295,8 +286,7 @@ def expval_joint_sampling_grouping(qdev, observables: Sequence[str], n_shots_per
     out = {}
     for basis, members in find_observable_groups(obs).items():
         idx = _rotated_samples(qdev, basis, n_shots_per_group, generator)
-        for ob in members:
-            out[ob] = _sampled_expval(idx, ob, qdev.n_wires)
+        out.update(zip(members, _sampled_expvals(idx, members, qdev.n_wires).unbind(0)))
     return out
 
 
