@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(256) k_tile_sums(const float2* state, int n, i
 }
 
 // One block (1024 threads) per row: in-place inclusive scan in chunks of 8192: a thread's 8
-// values, the warp's threads, the block's warps.  (Ten additions a value, all in float64, took
-// 21 us for 4 rows of 4096 tiles.)
+// values, the warp's threads, the block's warps.  (Ten additions a value and 80
+// barriers took 21 us for 4 rows of 4096 tiles, this takes 9.)
 constexpr int kScanPer = 8;
 __global__ void __launch_bounds__(1024) k_tile_scan(double* tile_sum, int64_t ntiles) {
   __shared__ double warp_sum[32];
@@ -93,25 +93,84 @@ __global__ void __launch_bounds__(1024) k_tile_scan(double* tile_sum, int64_t nt
   }
 }
 
-// The draw within a tile, amplitude by amplitude in float64.
-__device__ int64_t draw_in_tile(const float2* src, int count, double before, double target) {
+// The draw within a tile of 2^kTileBits amplitudes, amplitude by amplitude in float64: each lane
+// squares 8 of them, the additions go through all lanes in order.
+__device__ __noinline__ int draw_in_tile(const float2* src, double before, double target) {
+  const int lane = threadIdx.x & 31;
+  double p[8];
+  uint32_t some = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    p[k] = prob(src[8 * lane + k]);
+    if (p[k] > 0.0) some = 8 * lane + k;
+  }
   double acc = before;
-  int64_t last_nonzero = 0;
+  for (int l = 0; l < 32; ++l) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      acc += __shfl_sync(0xffffffffu, p[k], l);
+      if (acc > target) return 8 * l + k;  // the same for every lane
+    }
+  }
+  return __reduce_max_sync(0xffffffffu, some);  // rounding left target at the tile's end: the last one not zero
+}
+
+// The same in a row of fewer amplitudes.
+__device__ __noinline__ int draw_in_row(const float2* src, int count, double before, double target) {
+  double acc = before;
+  int last_nonzero = 0;
   for (int j = 0; j < count; ++j) {
     const double p = prob(src[j]);
     if (p > 0.0) last_nonzero = j;
     acc += p;
     if (acc > target) return j;
   }
-  return last_nonzero;  // rounding left target at the tile's end
+  return last_nonzero;
+}
+
+// The outcome from sums in R (a lane's 8 neighbouring amplitudes, then the warp's), or -1 where
+// the target t (from the tile's start) is not farther than the margin from both of the
+// outcome's ends.  float32: at most 16 roundings of sums up to the tile's and t's own; `walk`
+// covers the float64 walk's 256 additions on sums up to the row's.
+template <typename R>
+__device__ __forceinline__ int sure_draw(const float4 (&v)[4], R t, R walk) {
+  const int lane = threadIdx.x & 31;
+  R c[8];  // running sums over the lane's amplitudes
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const R x0 = v[k].x, y0 = v[k].y, x1 = v[k].z, y1 = v[k].w;
+    c[2 * k] = fma(x0, x0, y0 * y0) + (k > 0 ? c[2 * k - (k > 0)] : R(0));
+    c[2 * k + 1] = fma(x1, x1, y1 * y1) + c[2 * k];
+  }
+  R incl = c[7];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const R u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  const R all = __shfl_sync(0xffffffffu, incl, 31), start = incl - c[7];
+  const R margin = (sizeof(R) == 4 ? R(32 * 5.9604645e-8) * (all + fabs(t)) + R(1e-37) : R(0)) + walk;
+  int j = 8;  // the lane's first amplitude whose sum exceeds t
+#pragma unroll
+  for (int k = 7; k >= 0; --k)
+    if (start + c[k] > t) j = k;
+  const uint32_t who = __ballot_sync(0xffffffffu, j < 8);
+  if (who == 0) return -1;
+  R below = start, above = start;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k == j) above = start + c[k];
+    if (k == j - 1) below = start + c[k];
+  }
+  const int mine = above - t > margin && t - below > margin ? 8 * lane + j : -1;
+  return __shfl_sync(0xffffffffu, mine, __ffs(who) - 1);
 }
 
 // One warp per shot.  The tile: the first whose inclusive prefix exceeds the target, 32 places
-// at a time.  Within it a lane sums 8 neighbouring amplitudes: float32 sums tell the outcome
-// apart wherever the target is farther from both of its ends than their error (all but about
-// one shot in 5000); the others go through the tile in float64.  Outcomes are the float64
-// ones either way.  n = 20, 4 rows, 8192 shots: 118 -> @@ us (a thread per shot walked its
-// tile alone).
+// at a time.  Within it float32 sums settle all but about one shot in 500, float64 ones all but
+// the odd one of the others, and those go through the tile in order: outcomes are the ordered
+// walk's either way.  n = 20, 4 rows, 8192 shots: 118 -> 29 us (a thread per shot walked its tile
+// alone).
 __global__ void __launch_bounds__(256) k_draw(const float2* state, int n, int tb, int64_t ntiles,
                                               const double* prefix, const double* uniforms, int64_t shots,
                                               int64_t* out) {
@@ -119,7 +178,8 @@ __global__ void __launch_bounds__(256) k_draw(const float2* state, int n, int tb
   const int lane = threadIdx.x & 31;
   const double* pre = prefix + b * ntiles;
   const double total = pre[ntiles - 1];
-  for (int64_t s = (int64_t)blockIdx.x * kDrawWarps + (threadIdx.x >> 5); s < shots; s += (int64_t)gridDim.x * kDrawWarps) {
+  for (int64_t s = (int64_t)blockIdx.x * kDrawWarps + (threadIdx.x >> 5); s < shots;
+       s += (int64_t)gridDim.x * kDrawWarps) {
     const double target = uniforms[b * shots + s] * total;
     int64_t lo = 0, hi = ntiles - 1;  // the tile lies in [lo, hi]
     while (lo < hi) {
@@ -133,62 +193,37 @@ __global__ void __launch_bounds__(256) k_draw(const float2* state, int n, int tb
     }
     const double before = lo > 0 ? pre[lo - 1] : 0.0;
     const float2* src = state + (b << n) + (lo << tb);
-    int64_t pick = -1;
+    int pick = -1;
     if (tb == kTileBits) {
-      float c[8];  // running sums over the lane's amplitudes
+      float4 v[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float4 v = ld4(src + 8 * lane + 2 * k);
-        c[2 * k] = fmaf(v.x, v.x, v.y * v.y) + (k > 0 ? c[2 * k - 1] : 0.f);
-        c[2 * k + 1] = fmaf(v.z, v.z, v.w * v.w) + c[2 * k];
-      }
-      float incl = c[7];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-      }
-      const float all = __shfl_sync(0xffffffffu, incl, 31);
-      const float start = incl - c[7];
-      const float t = static_cast<float>(target - before);
-      // float32: at most 16 roundings of sums up to `all` (and the one of t); float64: the walk's
-      // 256 additions, on sums up to `total`; the last term: float32 underflow
-      const float margin = 32.f * 5.9604645e-8f * (all + fabsf(t)) + static_cast<float>(total * 1e-12) + 1e-37f;
-      int j = 8;  // the lane's first amplitude whose sum exceeds t
-#pragma unroll
-      for (int k = 7; k >= 0; --k)
-        if (start + c[k] > t) j = k;
-      const uint32_t who = __ballot_sync(0xffffffffu, j < 8);
-      if (who != 0) {
-        const int w = __ffs(who) - 1;
-        float below = start, above = start;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (k == j) above = start + c[k];
-          if (k == j - 1) below = start + c[k];
-        }
-        const bool sure = above - t > margin && t - below > margin;
-        if (__shfl_sync(0xffffffffu, sure ? 1 : 0, w)) pick = 8 * w + __shfl_sync(0xffffffffu, j, w);
-      }
+      for (int k = 0; k < 4; ++k) v[k] = ld4(src + 8 * lane + 2 * k);
+      const double t = target - before, walk = 1e-12 * total;
+      pick = sure_draw<float>(v, static_cast<float>(t), static_cast<float>(walk));
+      if (pick < 0) pick = sure_draw<double>(v, t, walk);
     }
-    if (pick < 0) pick = draw_in_tile(src, 1 << tb, before, target);  // every lane the same
+    if (pick < 0)
+      pick = tb == kTileBits ? draw_in_tile(src, before, target) : draw_in_row(src, 1 << tb, before, target);
     if (lane == 0) out[b * shots + s] = (lo << tb) + pick;
   }
 }
 
 // out[string][row] = mean over the shots of (-1)^popcount(outcome & mask)
-__global__ void __launch_bounds__(256) k_parity(const int64_t* outcomes, int64_t shots, const ParityMasks masks,
-                                                int64_t bsz, float* out) {
+__global__ void __launch_bounds__(1024) k_parity(const int64_t* outcomes, int64_t shots, const ParityMasks masks,
+                                                 int64_t bsz, float* out) {
   __shared__ unsigned long long odd;
   const int64_t b = blockIdx.x;
   const unsigned long long mask = masks.m[blockIdx.y];
+  const int64_t* row = outcomes + b * shots;
   if (threadIdx.x == 0) odd = 0;
   __syncthreads();
   unsigned long long mine = 0;
-  for (int64_t s = threadIdx.x; s < shots; s += blockDim.x) {
-    mine += __popcll(static_cast<unsigned long long>(outcomes[b * shots + s]) & mask) & 1;
-  }
-  if (mine) atomicAdd(&odd, mine);
+#pragma unroll 4
+  for (int64_t s = threadIdx.x; s < shots; s += 1024)
+    mine += __popcll(static_cast<unsigned long long>(row[s]) & mask) & 1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&odd, mine);
   __syncthreads();
   if (threadIdx.x == 0)
     out[blockIdx.y * bsz + b] = static_cast<float>(
@@ -244,7 +279,7 @@ extern "C" int tqk_sample_parity(const int64_t* outcomes, int64_t bsz, int64_t s
     const int cnt = m - j0 < sample::kParityStrings ? m - j0 : sample::kParityStrings;
     sample::ParityMasks pm;
     for (int j = 0; j < sample::kParityStrings; ++j) pm.m[j] = j < cnt ? masks[j0 + j] : 0ull;
-    sample::k_parity<<<dim3((unsigned)bsz, (unsigned)cnt), 256, 0, as_stream(stream)>>>(outcomes, shots, pm, bsz,
+    sample::k_parity<<<dim3((unsigned)bsz, (unsigned)cnt), 1024, 0, as_stream(stream)>>>(outcomes, shots, pm, bsz,
                                                                                        out + (int64_t)j0 * bsz);
     const int rc = launch_status(what);
     if (rc) return rc;
