@@ -249,6 +249,10 @@ int tqk_fused_adjoint(void* psi, void* lam, int64_t bsz, int n, const int32_t* w
  * with u = NULL).  Reads two states and writes one, where tqk_fused_adjoint writes two. */
 int tqk_fused_adjoint_stored(const void* psi_in, void* lam, int64_t bsz, int n, const int32_t* wires,
                              const void* image_h, int64_t u_batch, double* mr_out, int* status, void* stream);
+/* The same out of place: lam = U^H lam_in, lam_in unchanged (lam_in == lam: in place). */
+int tqk_fused_adjoint_stored_to(const void* psi_in, const void* lam_in, void* lam, int64_t bsz, int n,
+                                const int32_t* wires, const void* image_h, int64_t u_batch, double* mr_out,
+                                int* status, void* stream);
 
 /* ---------------------------------------------------------------- gate programs
  * Parameterised gates whose operand the GPU builds from the parameters in place.
@@ -363,6 +367,10 @@ int tqk_tiled_apply(void* state, int64_t bsz, int n, const tqk_staged_op* ops, i
                     int* status, void* stream);
 int tqk_tiled_adjoint(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* ops, int nops,
                       uint64_t tile_mask, int* status, void* stream);
+/* The same out of place: psi and lam are written, psi_in and lam_in read (each equal to its own
+ * output, or not overlapping any). */
+int tqk_tiled_adjoint_to(const void* psi_in, const void* lam_in, void* psi, void* lam, int64_t bsz, int n,
+                         const tqk_staged_op* ops, int nops, uint64_t tile_mask, int* status, void* stream);
 
 /* ---------------------------------------------------------------- persistent circuit batches
  * Many independent circuits of different sizes (n <= 24) in one launch.  tqk_batch_plan
@@ -525,6 +533,12 @@ int tqk_segment_forward(void* state, int64_t bsz, int n, const tqk_exec_op* ops,
 int tqk_segment_backward(const void* psi_end, void* lam, void* work, int64_t bsz, int n, const tqk_exec_op* ops,
                          int nops, int* status, const void** start, int64_t* launches, tqk_exec_hook hook,
                          void* user, void* stream);
+/* The same with the cotangent at the segment's end in lam_end, which is only read (lam_end == lam:
+ * in place); lam receives the one at the segment's start.  The first step reads lam_end itself
+ * where it can (tile passes, blocks with a stored input) and a copy of it otherwise. */
+int tqk_segment_backward_from(const void* psi_end, const void* lam_end, void* lam, void* work, int64_t bsz, int n,
+                              const tqk_exec_op* ops, int nops, int* status, const void** start,
+                              int64_t* launches, tqk_exec_hook hook, void* user, void* stream);
 
 #ifdef __cplusplus
 }

@@ -83,6 +83,10 @@ _SIGS = {
     "tqk_pauli_expval_noalloc": (_int, [_vp, _i64, _int, _u64p, _u64p, _int, _vp, _vp]),
     "tqk_segment_forward": (_int, [_vp, _i64, _int, _vp, _int, _vp, _vp, _vp, EXEC_HOOK, _vp, _vp]),
     "tqk_segment_backward": (_int, [_vp, _vp, _vp, _i64, _int, _vp, _int, _vp, _vp, _vp, EXEC_HOOK, _vp, _vp]),
+    "tqk_tiled_adjoint_to": (_int, [_vp, _vp, _vp, _vp, _i64, _int, _vp, _int, ctypes.c_uint64, _vp, _vp]),
+    "tqk_fused_adjoint_stored_to": (_int, [_vp, _vp, _vp, _i64, _int, _i32p, _vp, _i64, _vp, _vp, _vp]),
+    "tqk_segment_backward_from": (_int, [_vp, _vp, _vp, _vp, _i64, _int, _vp, _int, _vp, _vp, _vp, EXEC_HOOK, _vp,
+                                         _vp]),
     "tqk_gate_operand_size": (_int, [_int]),
     "tqk_gate_operands": (_int, [_vp, _int, _vp]),
     "tqk_param_grads": (_int, [_vp, _int, _vp]),
@@ -412,15 +416,17 @@ def segment_forward(state, n, table, nops) -> int:
     return final.value or 0
 
 
-def segment_backward(psi_end, lam, work, n, table, nops) -> int:
+def segment_backward(psi_end, lam, work, n, table, nops, lam_end=None) -> int:
     """Reverse sweep of a host table of ``ExecOp``; returns the device address where the
-    sweep's state ended (the segment's start)."""
+    sweep's state ended (the segment's start).  ``lam_end``: the cotangent at the segment's
+    end, only read (default: ``lam``, in place)."""
     start = ctypes.c_void_p()
     count = ctypes.c_int64(0)
     hook = _hook("backward", table)
-    _check(load().tqk_segment_backward(psi_end.data_ptr(), lam.data_ptr(), _ptr(work), lam.shape[0], n, table, nops,
-                                       status_word(lam.device).data_ptr(), ctypes.byref(start), ctypes.byref(count),
-                                       hook, None, _stream(lam)), launches=0)
+    _check(load().tqk_segment_backward_from(psi_end.data_ptr(), (lam if lam_end is None else lam_end).data_ptr(),
+                                            lam.data_ptr(), _ptr(work), lam.shape[0], n, table, nops,
+                                            status_word(lam.device).data_ptr(), ctypes.byref(start),
+                                            ctypes.byref(count), hook, None, _stream(lam)), launches=0)
     LAUNCHES[0] += count.value
     return start.value or 0
 

@@ -267,6 +267,7 @@ struct TcParams {
   uint8_t warp_row[8], warp_g[8], warp_lam[8];
   uint8_t c_row[4], c_g[4];
   uint8_t nat_of_k[64];      // natural pattern index of K-order index jk (cross term)
+  const float2* adj_in[2];   // ADJ: where psi and lam are read (in place: psi, lam)
 };
 
 // Warp roles (416 threads): warps 0-7 produce A images, warps 8-11 drain the tensor-
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(kThreadsWS, 1) k_tc(const TcParams p) {
     const int64_t toff = static_cast<int64_t>(p.lane_off[lane] + p.warp_off[warp]);
     const int row0 = p.lane_row[lane] + p.warp_row[warp];
     const int g0 = p.lane_g[lane] + p.warp_g[warp];
-    const float2* base = (ADJ && p.warp_lam[warp]) ? p.lam : p.psi;
+    const float2* base = ADJ ? p.adj_in[p.warp_lam[warp]] : p.psi;
     const uint32_t pf_mask = kPrefetchTiles > 0 ? line_owner_mask(p, toff) : 0u;
     for (int64_t k = 1; k < kPrefetchTiles && k < ntiles; ++k)
       prefetch_lines(p, base + tile_base(p, t_begin + k, ADJ) + toff, pf_mask);
@@ -1052,7 +1053,7 @@ bool overlaps(const void* a, const void* b, int64_t bytes) {
   return x != y && x < y + static_cast<uintptr_t>(bytes) && y < x + static_cast<uintptr_t>(bytes);
 }
 
-int adjoint_entry(const void* psi, float2* psi_out, void* lam, int64_t bsz, int n, const int32_t* wires,
+int adjoint_entry(const void* psi, float2* psi_out, const void* lam_in, void* lam, int64_t bsz, int n, const int32_t* wires,
                   const void* image_h, int64_t u_batch, double* mr_out, int* status, void* stream, const char* what) {
   int rc = check_state(psi, bsz, n, what);
   if (rc) return rc;
@@ -1062,7 +1063,14 @@ int adjoint_entry(const void* psi, float2* psi_out, void* lam, int64_t bsz, int 
   if (n < 13) return fail(TQK_UNSUPPORTED, "%s: needs n_wires >= 13 (got %d)", what, n);
   const int64_t bytes = bsz * (int64_t(8) << n);
   if (psi == lam || overlaps(psi, lam, bytes)) return fail(TQK_BAD_POINTER, "%s: psi and lam overlap", what);
+  if (lam_in != lam) {
+    if ((rc = check_state(lam_in, bsz, n, what))) return rc;
+    if (overlaps(lam_in, lam, bytes) || (psi_out != nullptr && (psi_out == lam_in || overlaps(psi_out, lam_in, bytes))))
+      return fail(TQK_BAD_POINTER, "%s: the cotangent read overlaps a state written", what);
+  }
   tc::TcParams p;
+  p.adj_in[0] = static_cast<const float2*>(psi);
+  p.adj_in[1] = static_cast<const float2*>(lam_in);
   p.psi = const_cast<float2*>(static_cast<const float2*>(psi));
   p.psi_out = psi_out;
   p.lam = static_cast<float2*>(lam);
@@ -1101,15 +1109,22 @@ int apply_entry(const void* in, void* out, int64_t bsz, int n, const int32_t* wi
 
 extern "C" int tqk_fused_adjoint(void* psi, void* lam, int64_t bsz, int n, const int32_t* wires,
                                  const void* image_h, int64_t u_batch, double* mr_out, int* status, void* stream) {
-  return adjoint_entry(psi, static_cast<float2*>(psi), lam, bsz, n, wires, image_h, u_batch, mr_out, status, stream,
+  return adjoint_entry(psi, static_cast<float2*>(psi), lam, lam, bsz, n, wires, image_h, u_batch, mr_out, status, stream,
                        "tqk_fused_adjoint");
 }
 
 extern "C" int tqk_fused_adjoint_stored(const void* psi_in, void* lam, int64_t bsz, int n, const int32_t* wires,
                                         const void* image_h, int64_t u_batch, double* mr_out, int* status,
                                         void* stream) {
-  return adjoint_entry(psi_in, nullptr, lam, bsz, n, wires, image_h, u_batch, mr_out, status, stream,
+  return adjoint_entry(psi_in, nullptr, lam, lam, bsz, n, wires, image_h, u_batch, mr_out, status, stream,
                        "tqk_fused_adjoint_stored");
+}
+
+extern "C" int tqk_fused_adjoint_stored_to(const void* psi_in, const void* lam_in, void* lam, int64_t bsz, int n,
+                                           const int32_t* wires, const void* image_h, int64_t u_batch,
+                                           double* mr_out, int* status, void* stream) {
+  return adjoint_entry(psi_in, nullptr, lam_in, lam, bsz, n, wires, image_h, u_batch, mr_out, status, stream,
+                       "tqk_fused_adjoint_stored_to");
 }
 
 extern "C" int tqk_fused_apply(void* state, int64_t bsz, int n, const int32_t* wires, const void* image,

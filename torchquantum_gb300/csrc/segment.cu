@@ -22,6 +22,12 @@ struct Cursor {
   bool owned;         // the state is the work buffer (writable)
   cudaStream_t st;
   int64_t* launches;
+  // the buffer a step that need not work in place writes
+  int target(void** out, const char* what) const {
+    if (work == nullptr) return fail(TQK_BAD_POINTER, "%s: a reverse step needs the work buffer", what);
+    *out = work;
+    return TQK_OK;
+  }
   // the state, made writable: copied into the work buffer if it is read only
   int writable(void** out, const char* what) {
     if (!owned) {
@@ -144,10 +150,18 @@ extern "C" int tqk_segment_forward(void* state, int64_t bsz, int n, const tqk_ex
 extern "C" int tqk_segment_backward(const void* psi_end, void* lam, void* work, int64_t bsz, int n,
                                     const tqk_exec_op* ops, int nops, int* status, const void** start,
                                     int64_t* launches, tqk_exec_hook hook, void* user, void* stream) {
+  return tqk_segment_backward_from(psi_end, lam, lam, work, bsz, n, ops, nops, status, start, launches, hook, user,
+                                   stream);
+}
+
+extern "C" int tqk_segment_backward_from(const void* psi_end, const void* lam_end, void* lam, void* work, int64_t bsz,
+                                         int n, const tqk_exec_op* ops, int nops, int* status, const void** start,
+                                         int64_t* launches, tqk_exec_hook hook, void* user, void* stream) {
   const char* what = "tqk_segment_backward";
   int rc = check_state(psi_end, bsz, n, what);
   if (rc) return rc;
   if ((rc = check_state(lam, bsz, n, what))) return rc;
+  if ((rc = check_state(lam_end, bsz, n, what))) return rc;
   if (work != nullptr && (rc = check_state(work, bsz, n, what))) return rc;
   if (nops < 0 || (nops > 0 && ops == nullptr)) return fail(TQK_BAD_POINTER, "%s: null op table", what);
   if (status == nullptr) return fail(TQK_BAD_POINTER, "%s: null status word", what);
@@ -162,6 +176,17 @@ extern "C" int tqk_segment_backward(const void* psi_end, void* lam, void* work, 
   cudaStream_t st = as_stream(stream);
   Cursor psi{psi_end, work, static_cast<size_t>(bsz) * (static_cast<size_t>(8) << n), false, st, &count};
   if (work == psi_end) psi.owned = true;  // the caller lets the sweep write the result in place
+  // where lam is until the first step that writes it to `lam`: a tile pass or a block with a stored
+  // input reads it there, any other step works on a copy
+  const void* lam_at = lam_end;
+  auto own_lam = [&]() -> int {
+    if (lam_at == lam) return TQK_OK;
+    if (cudaMemcpyAsync(lam, lam_at, psi.bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+      return fail(TQK_CUDA_ERROR, "%s: copy of the cotangent failed", what);
+    ++count;
+    lam_at = lam;
+    return TQK_OK;
+  };
   for (int i = nops - 1; i >= 0; --i) {
     const tqk_exec_op& op = ops[i];
     if (op.skip_reverse) break;
@@ -169,16 +194,31 @@ extern "C" int tqk_segment_backward(const void* psi_end, void* lam, void* work, 
     void* p = nullptr;
     if (op.kind == TQK_X_BLOCK_TC && op.stored != nullptr) {
       if (hook) hook(i, op.kind, 0, user);
-      rc = tqk_fused_adjoint_stored(op.stored, lam, bsz, n, w, op.image_h, op.batch, op.grad ? op.mr : nullptr,
-                                    status, stream);
+      rc = tqk_fused_adjoint_stored_to(op.stored, lam_at, lam, bsz, n, w, op.image_h, op.batch,
+                                       op.grad ? op.mr : nullptr, status, stream);
       if (rc) return rc;
+      lam_at = lam;
       if (hook) hook(i, op.kind, 1, user);
       ++count;
       psi.state = op.stored;
       psi.owned = false;
       continue;
     }
+    if (op.kind == TQK_X_TILED) {
+      if ((rc = psi.target(&p, what))) return rc;
+      if (hook) hook(i, op.kind, 0, user);
+      rc = tqk_tiled_adjoint_to(psi.state, lam_at, p, lam, bsz, n, op.staged, op.nstaged,
+                                static_cast<uint64_t>(op.batch), status, stream);
+      if (rc) return rc;
+      if (hook) hook(i, op.kind, 1, user);
+      ++count;
+      psi.state = p;
+      psi.owned = true;
+      lam_at = lam;
+      continue;
+    }
     if ((rc = psi.writable(&p, what))) return rc;
+    if ((rc = own_lam())) return rc;
     if (hook) hook(i, op.kind, 0, user);
     switch (op.kind) {
       case TQK_X_DENSE:
@@ -214,10 +254,6 @@ extern "C" int tqk_segment_backward(const void* psi_end, void* lam, void* work, 
       case TQK_X_STAGED:
         rc = tqk_staged_adjoint(p, lam, bsz, n, op.staged, op.nstaged, op.tile_bits, status, stream);
         break;
-      case TQK_X_TILED:
-        rc = tqk_tiled_adjoint(p, lam, bsz, n, op.staged, op.nstaged, static_cast<uint64_t>(op.batch), status,
-                               stream);
-        break;
       case TQK_X_BLOCK_TC: {
         double* mr = op.grad ? op.mr : nullptr;
         rc = tqk_fused_adjoint(p, lam, bsz, n, w, op.image_h, op.batch, mr, status, stream);
@@ -232,6 +268,7 @@ extern "C" int tqk_segment_backward(const void* psi_end, void* lam, void* work, 
     if (hook) hook(i, op.kind, 1, user);
     ++count;
   }
+  if ((rc = own_lam())) return rc;
   if (start) *start = psi.state;
   if (launches) *launches = count;
   return TQK_OK;

@@ -91,8 +91,10 @@ struct Sweep {
 };
 
 struct Params {
-  float2* psi;
+  float2* psi;            // tiles are stored here ..
   float2* lam;
+  const float2* psi_in;   // .. and loaded from here (in place: the same)
+  const float2* lam_in;
   int n, m;               // qubits; tile bits
   int64_t tiles;          // tiles per row
   uint64_t outer;         // index bits outside the tile
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_tiled(const __grid_constant_
   const Source src{p, fac};
   for (int64_t t = blockIdx.x; t < p.tiles; t += gridDim.x) {
     const uint64_t base = deposit(static_cast<uint64_t>(t), p.outer);
-    load_tile(p, frame(p, base), p.psi, tile);
+    load_tile(p, frame(p, base), p.psi_in, tile);
     wait_loads();  // also orders the tables
 #pragma unroll 1
     for (int s = 0; s < p.nsweeps; ++s) {
@@ -489,8 +491,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
     const uint64_t base = deposit(static_cast<uint64_t>(t), p.outer);
     {
       const Frame f = frame(p, base);
-      load_tile(p, f, p.psi, ps);
-      load_tile(p, f, p.lam, ls);
+      load_tile(p, f, p.psi_in, ps);
+      load_tile(p, f, p.lam_in, ls);
     }
     wait_loads();
 #pragma unroll 1
@@ -739,11 +741,13 @@ int fill_tiled(tiled::Params& p, int64_t bsz, int n, const tqk_staged_op* ops, i
   return TQK_OK;
 }
 
-int tiled_entry(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* ops, int nops, uint64_t tile_mask,
+int tiled_entry(const void* psi_in, const void* lam_in, void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* ops, int nops, uint64_t tile_mask,
                 int* status, bool adjoint, void* stream, const char* what) {
   int rc = check_state(psi, bsz, n, what);
   if (rc) return rc;
   if (adjoint && (rc = check_state(lam, bsz, n, what))) return rc;
+  if ((rc = check_state(psi_in, bsz, n, what))) return rc;
+  if (adjoint && (rc = check_state(lam_in, bsz, n, what))) return rc;
   const int m = __builtin_popcountll(tile_mask);
   if (n < tiled::kMinBits || (tile_mask >> n) != 0 || m != (n < tiled::kMaxBits ? n : tiled::kMaxBits) ||
       (tile_mask & 1ull) == 0)
@@ -755,6 +759,8 @@ int tiled_entry(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* o
   if (status == nullptr) return fail(TQK_BAD_POINTER, "%s: null status word", what);
   p.psi = static_cast<float2*>(psi);
   p.lam = static_cast<float2*>(lam);
+  p.psi_in = static_cast<const float2*>(psi_in);
+  p.lam_in = static_cast<const float2*>(lam_in);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -791,10 +797,25 @@ int tiled_entry(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* o
 
 extern "C" int tqk_tiled_apply(void* state, int64_t bsz, int n, const tqk_staged_op* ops, int nops, uint64_t tile_mask,
                                int* status, void* stream) {
-  return tiled_entry(state, nullptr, bsz, n, ops, nops, tile_mask, status, false, stream, "tqk_tiled_apply");
+  return tiled_entry(state, nullptr, state, nullptr, bsz, n, ops, nops, tile_mask, status, false, stream, "tqk_tiled_apply");
 }
 
 extern "C" int tqk_tiled_adjoint(void* psi, void* lam, int64_t bsz, int n, const tqk_staged_op* ops, int nops,
                                  uint64_t tile_mask, int* status, void* stream) {
-  return tiled_entry(psi, lam, bsz, n, ops, nops, tile_mask, status, true, stream, "tqk_tiled_adjoint");
+  return tiled_entry(psi, lam, psi, lam, bsz, n, ops, nops, tile_mask, status, true, stream, "tqk_tiled_adjoint");
+}
+
+extern "C" int tqk_tiled_adjoint_to(const void* psi_in, const void* lam_in, void* psi, void* lam, int64_t bsz, int n,
+                                    const tqk_staged_op* ops, int nops, uint64_t tile_mask, int* status,
+                                    void* stream) {
+  const char* what = "tqk_tiled_adjoint_to";
+  const char* a[2] = {static_cast<const char*>(psi_in), static_cast<const char*>(lam_in)};
+  const char* o[2] = {static_cast<const char*>(psi), static_cast<const char*>(lam)};
+  const int64_t bytes = n >= 0 && n < 48 && bsz > 0 ? bsz * (int64_t(8) << n) : 0;
+  for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < 2; ++j)
+      if ((i != j || a[i] != o[j]) && a[i] < o[j] + bytes && o[j] < a[i] + bytes)
+        return fail(TQK_BAD_POINTER, "%s: an input overlaps an output other than its own buffer", what);
+  if (o[0] < o[1] + bytes && o[1] < o[0] + bytes) return fail(TQK_BAD_POINTER, "%s: psi and lam overlap", what);
+  return tiled_entry(psi_in, lam_in, psi, lam, bsz, n, ops, nops, tile_mask, status, true, stream, what);
 }

@@ -130,10 +130,15 @@ class CircuitFunction(torch.autograd.Function):
         final, *stored = ctx.saved_tensors
         inputs = {id(op): t for op, t in zip(ctx.stored_ops, stored)}
         psi = StateCursor(final.detach())
-        lam = kernel_operand(grad_out.to(torch.complex64)).clone()
+        # the incoming cotangent is only read: the first segment's sweep writes lam elsewhere
+        lam_end = kernel_operand(grad_out.to(torch.complex64))
+        if lam_end.data_ptr() % 16:  # a view the kernels cannot read
+            lam_end = lam_end.clone()
+        lam = torch.empty_like(lam_end) if ctx.segments else lam_end
         per_seg = []
         for sg, cnt in zip(reversed(ctx.segments), reversed(ctx.counts)):
-            per_seg.append(sg.backward(psi, lam, cnt > 0, inputs))
+            per_seg.append(sg.backward(psi, lam, cnt > 0, inputs, lam_end))
+            lam_end = None
         grads = [g for gl in reversed(per_seg) for g in gl]
         g_init = lam if ctx.has_init else None
         return (None, None, None, g_init, *grads)

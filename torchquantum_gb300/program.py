@@ -442,19 +442,20 @@ class Segment:
 
     # -------------------------------------------------------------- backward
     def backward(self, psi: "engine.StateCursor", lam: torch.Tensor, need_grads: bool,
-                 inputs: Optional[dict] = None) -> List[Optional[torch.Tensor]]:
+                 inputs: Optional[dict] = None, lam_end: Optional[torch.Tensor] = None) -> List[Optional[torch.Tensor]]:
         """Reverse sweep over this segment (``psi`` at its end on entry, at its start on
-        return; ``lam`` updated in place); ``inputs`` maps id(block) to the block's stored
+        return; ``lam`` updated in place, or written from ``lam_end``, which is only read);
+        ``inputs`` maps id(block) to the block's stored
         input state, where the forward kept one and it is still held.  Returns grads for
         ``self.diff_inputs``."""
         _lib.nvtx_push(f"tqk.segment.backward[{len(self.exec_ops)} passes]")
         try:
-            return self._backward(psi, lam, need_grads, inputs or {})
+            return self._backward(psi, lam, need_grads, inputs or {}, lam_end)
         finally:
             _lib.nvtx_pop()
 
     def _backward(self, psi: "engine.StateCursor", lam: torch.Tensor, need_grads: bool,
-                  inputs: dict) -> List[Optional[torch.Tensor]]:
+                  inputs: dict, lam_end: Optional[torch.Tensor] = None) -> List[Optional[torch.Tensor]]:
         dev = self.device
         n = self.n
         opg = torch.zeros_like(self.op128) if (need_grads and self.natives) else None
@@ -530,11 +531,13 @@ class Segment:
             uncomputes = any(not (r.kind == _lib.X_BLOCK_TC and (r.stored or r.skip_reverse)) for r in recs)
             work = psi.state if psi.owned else (psi.work_buffer() if uncomputes else None)
             table = (_lib.ExecOp * len(recs))(*recs)
-            start = _lib.segment_backward(psi.state, lam, work, n, table, len(recs))
+            start = _lib.segment_backward(psi.state, lam, work, n, table, len(recs), lam_end)
             if work is not None and start == work.data_ptr():
                 psi.state, psi.owned = work, True
             elif start in stored_at:
                 psi.state, psi.owned = stored_at[start], False
+        elif lam_end is not None:
+            lam.copy_(lam_end)
         if zero_block is not None and zero_block[1] is not None:
             _add_zero_input_cotangent(lam, zero_block[0], zero_block[1], n)
         if cross_jobs:
