@@ -242,6 +242,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // amplitudes r = e + 8c: e = K bits 0-2 (one chunk), c = two more dimensions; its lanes
 // run over the 5 lowest-address remaining dimensions, so every load instruction is
 // coalesced whatever the target bits are.
+// Row-major; transposed (where its stores touch fewer sectors a warp); row-major with outputs 2o and
+// 2o + 1, neighbours in memory, stored together; row-major with the lanes of two neighbouring rows
+// exchanging outputs so that each stores both rows of one.
+enum { DRAIN_ROWS = 0, DRAIN_COLS = 1, DRAIN_PAIRS = 2, DRAIN_SWAP = 3 };
 struct TcParams {
   float2* psi;               // state read (APPLY) / psi (ADJ)
   float2* psi_out;           // APPLY: product destination (psi: in place); ADJ: U^H psi
@@ -257,7 +261,7 @@ struct TcParams {
   int64_t tiles;
   double* mr_out;            // ADJ: [u_batch][128][128] cross term, or null
   int* status;
-  int transposed;            // output orientation (fewer store sectors per warp)
+  int drain;                 // DRAIN_*: output orientation
   uint64_t off[64];          // amplitude offset of output pattern j'
   uint64_t col_off[128];     // amplitude offset of tile row i (ADJ: i & 63)
   uint64_t lane_off[32];     // producer mapping: offsets, tile rows and chunk indices
@@ -389,9 +393,32 @@ __device__ __forceinline__ void drain_rows(const TcParams& p, int64_t tb, uint32
     tmem_ld16(d_tmem + lanes + q * 32, *reinterpret_cast<uint32_t(*)[16]>(&v[0]));
     tmem_ld16(d_tmem + lanes + q * 32 + 16, *reinterpret_cast<uint32_t(*)[16]>(&v[16]));
     tmem_wait_ld();
+    if (p.drain == DRAIN_PAIRS) {
 #pragma unroll
-    for (int h = 0; h < 16; ++h)
-      __stcs(dst + p.off[q * 16 + h], make_float2(__uint_as_float(v[2 * h]), __uint_as_float(v[2 * h + 1])));
+      for (int h = 0; h < 16; h += 2)
+        __stcs(reinterpret_cast<float4*>(dst + p.off[q * 16 + h]),
+               make_float4(__uint_as_float(v[2 * h]), __uint_as_float(v[2 * h + 1]), __uint_as_float(v[2 * h + 2]),
+                           __uint_as_float(v[2 * h + 3])));
+    } else if (!ADJ && p.drain == DRAIN_SWAP) {
+      // off[2o + 1] = off[2o] + 2, col_off of an odd row = its even neighbour's + 1: an odd lane's
+      // output starts at off[2o] + 2 from the neighbour's place
+      const bool odd = lane & 1;
+      float2* at = dst + (odd ? 1 : 0);
+#pragma unroll
+      for (int h = 0; h < 16; h += 2) {
+        const uint32_t sx = odd ? v[2 * h] : v[2 * h + 2], sy = odd ? v[2 * h + 1] : v[2 * h + 3];
+        const float kx = __uint_as_float(odd ? v[2 * h + 2] : v[2 * h]);
+        const float ky = __uint_as_float(odd ? v[2 * h + 3] : v[2 * h + 1]);
+        const float rx = __uint_as_float(__shfl_xor_sync(0xffffffffu, sx, 1));
+        const float ry = __uint_as_float(__shfl_xor_sync(0xffffffffu, sy, 1));
+        __stcs(reinterpret_cast<float4*>(at + p.off[q * 16 + h]),
+               odd ? make_float4(rx, ry, kx, ky) : make_float4(kx, ky, rx, ry));
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 16; ++h)
+        __stcs(dst + p.off[q * 16 + h], make_float2(__uint_as_float(v[2 * h]), __uint_as_float(v[2 * h + 1])));
+    }
   }
 }
 
@@ -454,7 +481,7 @@ __global__ void __launch_bounds__(kThreadsWS, 1) k_tc(const TcParams p) {
   const uint32_t ncols_tmem = ADJ ? 512u : 256u;
   const bool want_cross = ADJ && p.mr_out != nullptr;
   const bool flush_per_row = want_cross && p.u_batch > 1;
-  const bool tr = p.transposed != 0;
+  const bool tr = p.drain == DRAIN_COLS;
 
   if (threadIdx.x < 128) sy->nat_of_k[threadIdx.x] = (threadIdx.x & 64) + p.nat_of_k[threadIdx.x & 63];
   if (threadIdx.x == 0) {
@@ -1017,7 +1044,13 @@ int tc_setup(tqk::tc::TcParams& p, int64_t bsz, int n, const int32_t* wires, boo
     }
     return cnt;
   };
-  p.transposed = distinct_sectors(p.off, 16) < distinct_sectors(p.col_off, 32) ? 1 : 0;
+  // Bit 0 or bit 1 a target and not both: either plain orientation stores half sectors twice (a
+  // 2^24-amplitude block of 16 rows: 822 to 837 us forward, 1335 in reverse).  With bit 0 a pair of
+  // outputs is 16 bytes and two rows a whole sector (650 and 1045 us); with bit 1 alone two rows are
+  // 16 bytes and the pair a sector (653 us forward; in reverse the exchange takes what it saves).
+  if (tasc[0] == 0 && tasc[1] != 1) p.drain = tc::DRAIN_PAIRS;
+  else if (!adj && tasc[0] == 1 && tasc[1] != 2) p.drain = tc::DRAIN_SWAP;
+  else p.drain = distinct_sectors(p.off, 16) < distinct_sectors(p.col_off, 32) ? tc::DRAIN_COLS : tc::DRAIN_ROWS;
   p.tiles_per_row = (1ll << (n - 6)) / (adj ? 64 : 128);
   p.tpr_log2 = n - 6 - (adj ? 6 : 7);
   p.tiles = p.tiles_per_row * bsz;
