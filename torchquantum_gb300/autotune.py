@@ -116,8 +116,9 @@ def _time_ms(fn, dev, reps: int = 3) -> float:
 def batch_candidates(max_n: int):
     from .batch import BatchConfig
 
-    cands = [BatchConfig(14, 512, 1), BatchConfig(14, 256, 1), BatchConfig(13, 256, 3), BatchConfig(13, 128, 3),
-             BatchConfig(12, 128, 3), BatchConfig(11, 128, 3)]
+    cands = [BatchConfig(14, 512, 1), BatchConfig(14, 256, 1), BatchConfig(13, 256, 3), BatchConfig(13, 256, 1),
+             BatchConfig(13, 128, 3), BatchConfig(12, 256, 1), BatchConfig(12, 128, 3), BatchConfig(11, 512, 1),
+             BatchConfig(11, 128, 3)]
     # a tile wider than every circuit only wastes shared memory
     narrow = [c for c in cands if c.tile_bits <= max(max_n, 11)]
     return narrow or cands[-1:]

@@ -41,144 +41,7 @@ struct Tabs {
 
 __device__ __forceinline__ uint32_t dep(const Tabs& t, uint32_t l) { return t.lo[l & 127] + t.hi[l >> 7]; }
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {  // a * b + c
-  return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
-}
-
-// 2x2 matrix m on local bit lb of the tile; if lc >= 0 only where local bit lc is set.
-// Two adjacent pairs (i0, i0 + 2^lb), (i0 + 1, i0 + 1 + 2^lb) per 16-byte access when
-// lb >= 1, one pair (2q, 2q + 1) per access when lb == 0.
-template <int THREADS>
-__device__ __forceinline__ void apply_1q(float2* amp, int tb, int lb, int lc, const float2* m) {
-  float2 M[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) M[e] = __ldg(m + e);
-  const uint32_t cm = lc >= 0 ? (1u << lc) : 0u;
-  float4* amp4 = reinterpret_cast<float4*>(amp);
-  if (lb == 0) {
-    for (uint32_t q = threadIdx.x; q < (1u << (tb - 1)); q += THREADS) {
-      const uint32_t i0 = q << 1;
-      if ((i0 & cm) != cm) continue;
-      const float4 v = amp4[q];
-      const float2 a0 = lo2(v), a1 = hi2(v);
-      amp4[q] = pack4(cfma(M[0], a0, cmul(M[1], a1)), cfma(M[2], a0, cmul(M[3], a1)));
-    }
-    return;
-  }
-  const uint32_t lowm = (1u << (lb - 1)) - 1u;
-  for (uint32_t q = threadIdx.x; q < (1u << (tb - 2)); q += THREADS) {
-    const uint32_t i0 = ((q >> (lb - 1)) << (lb + 1)) | ((q & lowm) << 1);
-    const uint32_t i1 = i0 | (1u << lb);
-    const bool ok0 = (i0 & cm) == cm, ok1 = ((i0 | 1u) & cm) == cm;
-    if (!ok0 && !ok1) continue;
-    const float4 va = amp4[i0 >> 1], vb = amp4[i1 >> 1];
-    float2 a0 = lo2(va), b0 = lo2(vb), a1 = hi2(va), b1 = hi2(vb);
-    if (ok0) {
-      const float2 y = cfma(M[0], a0, cmul(M[1], b0));
-      b0 = cfma(M[2], a0, cmul(M[3], b0));
-      a0 = y;
-    }
-    if (ok1) {
-      const float2 y = cfma(M[0], a1, cmul(M[1], b1));
-      b1 = cfma(M[2], a1, cmul(M[3], b1));
-      a1 = y;
-    }
-    amp4[i0 >> 1] = pack4(a0, a1);
-    amp4[i1 >> 1] = pack4(b0, b1);
-  }
-}
-
-// Negate the amplitudes whose local index l has odd parity of c0 + popc(l & lin) +
-// popc(l & (l >> 1) & quad) (CZ and CZ ladders split into tile-local terms).
-template <int THREADS>
-__device__ __forceinline__ void apply_sign(float2* amp, int tb, int c0, uint32_t lin, uint32_t quad) {
-  float4* amp4 = reinterpret_cast<float4*>(amp);
-  for (uint32_t q = threadIdx.x; q < (1u << (tb - 1)); q += THREADS) {
-    const uint32_t l0 = q << 1, l1 = l0 | 1u;
-    const int s0 = (c0 + __popc(l0 & lin) + __popc(l0 & (l0 >> 1) & quad)) & 1;
-    const int s1 = (c0 + __popc(l1 & lin) + __popc(l1 & (l1 >> 1) & quad)) & 1;
-    if (!(s0 | s1)) continue;
-    float4 v = amp4[q];
-    if (s0) v.x = -v.x, v.y = -v.y;
-    if (s1) v.z = -v.z, v.w = -v.w;
-    amp4[q] = v;
-  }
-}
-
 __device__ __forceinline__ int local_pos(uint32_t tmask, int b) { return __popc(tmask & ((1u << b) - 1u)); }
-
-// Sign terms of CZ on global bits (bh, bl): both local -> a quadratic term only when the
-// bits are adjacent in the tile (true for ladder neighbours), else handled as lin/const.
-__device__ __forceinline__ void cz_terms(uint32_t tmask, uint32_t base, int b0, int b1, int& c0, uint32_t& lin,
-                                         uint32_t& quad, uint32_t& pairs) {
-  const bool in0 = (tmask >> b0) & 1u, in1 = (tmask >> b1) & 1u;
-  if (in0 && in1) {
-    const int p0 = local_pos(tmask, b0), p1 = local_pos(tmask, b1);
-    const int lo = p0 < p1 ? p0 : p1, hi = p0 < p1 ? p1 : p0;
-    if (hi == lo + 1) quad |= 1u << lo;
-    else pairs |= (1u << lo) | (1u << hi);  // a general local pair (single CZ only)
-  } else if (in0) {
-    if ((base >> b1) & 1u) lin ^= 1u << local_pos(tmask, b0);
-  } else if (in1) {
-    if ((base >> b0) & 1u) lin ^= 1u << local_pos(tmask, b1);
-  } else {
-    c0 ^= static_cast<int>((base >> b0) & (base >> b1) & 1u);
-  }
-}
-
-template <int THREADS>
-__device__ void apply_op(const tqk_batch_op& op, float2* amp, int n, int tb, uint32_t tmask, uint32_t base,
-                         const float2* mats) {
-  switch (op.kind) {
-    case TQK_B_DENSE1: {
-      const int b = n - 1 - op.w0;
-      apply_1q<THREADS>(amp, tb, local_pos(tmask, b), -1, mats + 4 * op.mat);
-      break;
-    }
-    case TQK_B_CTRL1: {
-      const int cb = n - 1 - op.w0, b = n - 1 - op.w1;
-      const int lb = local_pos(tmask, b);
-      if ((tmask >> cb) & 1u) {
-        apply_1q<THREADS>(amp, tb, lb, local_pos(tmask, cb), mats + 4 * op.mat);
-      } else if ((base >> cb) & 1u) {  // control outside the tile: set for the whole tile
-        apply_1q<THREADS>(amp, tb, lb, -1, mats + 4 * op.mat);
-      }
-      break;
-    }
-    case TQK_B_CZ: {
-      int c0 = 0;
-      uint32_t lin = 0, quad = 0, pairs = 0;
-      cz_terms(tmask, base, n - 1 - op.w0, n - 1 - op.w1, c0, lin, quad, pairs);
-      if (pairs) {  // both bits in the tile but not adjacent: negate where both are set
-        float4* amp4 = reinterpret_cast<float4*>(amp);
-        for (uint32_t q = threadIdx.x; q < (1u << (tb - 1)); q += THREADS) {
-          const uint32_t l0 = q << 1;
-          const bool s0 = (l0 & pairs) == pairs, s1 = ((l0 | 1u) & pairs) == pairs;
-          if (!(s0 || s1)) continue;
-          float4 v = amp4[q];
-          if (s0) v.x = -v.x, v.y = -v.y;
-          if (s1) v.z = -v.z, v.w = -v.w;
-          amp4[q] = v;
-        }
-      } else if (c0 | lin | quad) {
-        apply_sign<THREADS>(amp, tb, c0, lin, quad);
-      }
-      break;
-    }
-    case TQK_B_CZ_LADDER: {
-      int c0 = 0;
-      uint32_t lin = 0, quad = 0, pairs = 0;
-      for (int w = op.w0; w < op.w1; ++w) cz_terms(tmask, base, n - 1 - w, n - 2 - w, c0, lin, quad, pairs);
-      if (c0 | lin | quad) apply_sign<THREADS>(amp, tb, c0, lin, quad);
-      break;
-    }
-    default:
-      break;
-  }
-}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -188,9 +51,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 
-// ------------------------------------------------------------------ sweeps (tiles of >= 2^10)
-// A pass's ops on a tile of at least 2^10 amplitudes run from registers (sweep.cuh): the ops
-// are taken in order, a sweep ending before the op whose target would be the fifth besides
+// ------------------------------------------------------------------ sweeps
+// A pass's ops run from registers (sweep.cuh): the ops are taken in order, a sweep ending before the op whose target would be the fifth besides
 // tile bit 0 (or after kSweepOps).  A warp of its own reads the ops ahead of the others, cuts
 // the next sweep and writes it out while they run the current one, so a sweep costs them one
 // barrier, the one after its stores.  (Reading and cutting in every warp between the barriers:
@@ -200,9 +62,10 @@ constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 // (2.5 us) and the latency of 12 warps an SM, all the registers allow.  256 circuits of n = 8..20
 // and 2..40 layers, ms: one op per crossing and barrier 11.4 (13-bit tiles, 3 CTAs of 256);
 // sweeps of 16 amplitudes a thread 8.9 (3 x 256), of 32 8.7 (3 x 128).  96 circuits of up to 13
-// qubits, one tile each: 0.58 before, 0.38 now (256 threads, 32 amplitudes).
-constexpr int kSweepMinBits = 10;  // a tile fills at least one warp
-constexpr int kMaxAmpBits = 5;     // 2^AB amplitudes per thread: AB = 5, or 4 where CTAs are many
+// qubits, one tile each: 0.58 before, 0.38 now (256 threads, 32 amplitudes).  A row of fewer
+// amplitudes than a thread holds works in a tile of that many, the rest zero: 119 circuits of 7
+// qubits and 17 layers, 81 us op by op (each op's and matrix's read before it), 73 in sweeps.
+constexpr int kMaxAmpBits = 5;  // 2^AB amplitudes per thread: AB = 5, or 4 where CTAs are many
 constexpr int kSweepOps = 8;
 
 // How a sweep's threads run an op.  Patterns: sets of a thread's registers.
@@ -351,7 +214,7 @@ struct SweepMaker {
     const int count = __ffs(~__ballot_sync(0xffffffffu, fit)) - 1;  // leading ops that fit
     uint32_t regs = __shfl_sync(0xffffffffu, tg, count > 0 ? count - 1 : 0);
     if (count == 0) regs = 0u;
-    for (int b = tb - 1; __popc(regs) < AB - 1; --b) regs |= 1u << b;  // tb >= 9: never bit 0
+    for (int b = tb - 1; __popc(regs) < AB - 1; --b) regs |= 1u << b;  // tb >= AB: never bit 0
     regs |= 1u;
     int r[AB];
     {
@@ -452,7 +315,7 @@ __device__ __forceinline__ void run_sweep(const SweepRec& rec, float2* amp, int 
   };
   const uint32_t slots = 1u << (tb - AB);  // threads' worth of amplitudes
 #pragma unroll 1
-  for (uint32_t vt = threadIdx.x; vt < slots; vt += THREADS) {  // uniform for the warp
+  for (uint32_t vt = threadIdx.x; vt < slots; vt += THREADS) {  // (part of a warp in the smallest tiles)
     const uint32_t e = rec.lane[threadIdx.x & 31] ^ rec.high[vt >> 5], tl = e & 0xffffu;
     {
       uint16_t rphys[AB - 1];
@@ -481,7 +344,6 @@ __device__ __forceinline__ void run_sweep(const SweepRec& rec, float2* amp, int 
             default: dense_rows<AB, 4, true>(m4, so.reg); break;
           }
         }
-        __syncwarp();
       } else if (code == SW_SIGN) {
         uint32_t mask = so.reg;
         if ((__popc(tl & so.lin) + __popc(tl & (tl >> 1) & so.quad)) & 1) mask = ~mask;
@@ -508,7 +370,7 @@ __device__ __noinline__ void make_sweeps(SweepRec* rec, const tqk_batch_op* ops,
   s.mats = mats;
   s.num_ops = num_ops;
   s.n = n;
-  s.tb = __popc(tmask);
+  s.tb = max(__popc(tmask), AB);
   s.tmask = tmask;
   s.base = base;
   s.start(threadIdx.x & 31);
@@ -531,9 +393,6 @@ __device__ __noinline__ void run_sweeps(const SweepRec* rec, float2* amp, int tb
     __syncthreads();
   }
 }
-
-// Shared-memory place of tile amplitude l: tiles that run in sweeps are swizzled.
-__device__ __forceinline__ uint32_t place(uint32_t l, int tb) { return tb >= kSweepMinBits ? sweep::swz(l) : l; }
 
 // An item as its CTA works on it.
 struct Work {
@@ -651,37 +510,25 @@ __global__ void __launch_bounds__(THREADS + 32, MINB)
       __syncthreads();
     }
     if (maker) {
-      if (tb >= kSweepMinBits) {
-        make_sweeps<AB>(rec, W.ops, W.num_ops, mats, W.n, W.tmask, W.base);
-      } else {
-        for (int oi = 0; oi <= W.num_ops; ++oi) __syncthreads();
-      }
+      make_sweeps<AB>(rec, W.ops, W.num_ops, mats, W.n, W.tmask, W.base);
       fetch_item(work[cur ^ 1], tab_buf[cur ^ 1], circ, ops, passes, items, n_items, states, counter, max_tb);
     } else {
       if (W.flags & kFirst) {
-        for (uint32_t l = tid; l < tsz; l += THREADS)
-          amp[place(l, tb)] = make_float2((W.base == 0u && l == 0) ? 1.f : 0.f, 0.f);
+        for (uint32_t l = tid; l < max(tsz, 1u << AB); l += THREADS)
+          amp[sweep::swz(l)] = make_float2((W.base == 0u && l == 0) ? 1.f : 0.f, 0.f);
       } else if (2u * tid < tsz) {
         // 16-byte pieces through L2 (another SM may have stored them: .cg skips this SM's L1);
         // tile bits 0-4 are address bits 0-4, so a warp's pieces are 256-byte runs
         // (both places are linear: that of tile index l + k is the sum or XOR of theirs)
         const float2* src = W.state + W.base + dep(tabs, 2u * tid);
-        const uint32_t dst = place(2u * tid, tb);
+        const uint32_t dst = sweep::swz(2u * tid);
         for (uint32_t k = 0; k < tsz; k += 2u * THREADS)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bulk::smem_addr(amp + (dst ^ place(k, tb)))),
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bulk::smem_addr(amp + (dst ^ sweep::swz(k)))),
                        "l"(src + dep(tabs, k))
                        : "memory");
         asm volatile("cp.async.wait_all;" ::: "memory");
       }
-      if (tb >= kSweepMinBits) {
-        run_sweeps<THREADS, AB>(rec, amp, tb);
-      } else {
-        __syncthreads();
-        for (int oi = 0; oi < W.num_ops; ++oi) {
-          apply_op<THREADS>(W.ops[oi], amp, W.n, tb, W.tmask, W.base, mats);
-          __syncthreads();
-        }
-      }
+      run_sweeps<THREADS, AB>(rec, amp, max(tb, AB));
       if (W.flags & kLast) {
         const int zbit = W.n - 1 - W.z_wire;
         const bool in = (W.tmask >> zbit) & 1u;
@@ -689,7 +536,7 @@ __global__ void __launch_bounds__(THREADS + 32, MINB)
         const uint32_t out = (W.base >> zbit) & 1u;
         double zacc = 0.0;
         for (uint32_t l = tid; l < tsz; l += THREADS) {
-          const float2 a = amp[place(l, tb)];
+          const float2 a = amp[sweep::swz(l)];
           const bool minus = in ? (l >> zl) & 1u : out;
           zacc = fma(static_cast<double>(a.x), static_cast<double>(minus ? -a.x : a.x), zacc);
           zacc = fma(static_cast<double>(a.y), static_cast<double>(minus ? -a.y : a.y), zacc);
@@ -699,10 +546,10 @@ __global__ void __launch_bounds__(THREADS + 32, MINB)
       }
       if (((W.flags & kLast) == 0 || write_states) && W.state != nullptr && 2u * tid < tsz) {
         float2* dst = W.state + W.base + dep(tabs, 2u * tid);
-        const uint32_t src = place(2u * tid, tb);
+        const uint32_t src = sweep::swz(2u * tid);
         for (uint32_t k = 0; k < tsz; k += 2u * THREADS)
           *reinterpret_cast<float4*>(dst + dep(tabs, k)) =
-              *reinterpret_cast<const float4*>(amp + (src ^ place(k, tb)));
+              *reinterpret_cast<const float4*>(amp + (src ^ sweep::swz(k)));
       }
       __threadfence();  // stored before the tile counts as done
     }
@@ -896,13 +743,16 @@ extern "C" int tqk_batch_run(const tqk_batch_circuit* circuits, int ncirc, const
   cudaStream_t s = as_stream(stream);
 #define TQK_BATCH_ARGS circuits, ncirc, ops, passes, items, n_items, mats, states, write_states, z_out, pass_done, \
                        t_done, counter, status, cfg.tile_bits, cfg.ctas_per_sm, s
+  // 32 amplitudes a thread where the CTAs asked for leave it the registers (8.6 ms against 8.9 with
+  // 16 for 256 circuits of 8 to 20 qubits), else 16
   switch (cfg.threads) {
     case 512:
       return launch_batch<512, 1, 4>(TQK_BATCH_ARGS);
     case 256:
       return cfg.ctas_per_sm >= 2 ? launch_batch<256, 3, 4>(TQK_BATCH_ARGS) : launch_batch<256, 1, 5>(TQK_BATCH_ARGS);
     case 128:
-      return cfg.ctas_per_sm >= 4 ? launch_batch<128, 6, 4>(TQK_BATCH_ARGS) : launch_batch<128, 3, 5>(TQK_BATCH_ARGS);
+      return cfg.ctas_per_sm >= 4 && cfg.tile_bits <= 11 ? launch_batch<128, 6, 4>(TQK_BATCH_ARGS)
+                                                         : launch_batch<128, 3, 5>(TQK_BATCH_ARGS);
     default:
       return fail(TQK_BAD_SHAPE, "%s: threads %d (128, 256 or 512)", what, cfg.threads);
   }
