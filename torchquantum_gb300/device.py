@@ -100,7 +100,7 @@ class QuantumDevice(nn.Module):
         self.method = d["method"]                # "plain" | "fused" (see fusion.py)
         self.fuse_wires = d["fuse_wires"]        # fused block width 1..6, or "auto" (autotune.choose_fusion)
         self.fused_backend = d["fused_backend"]  # "auto" | "tc" (tensor cores) | "cuda" (CUDA cores)
-        self.stage_low = d["stage_low"]          # plain method: runs of low-qubit gates share one pass
+        self.stage_low = d["stage_low"]          # plain method: gates share passes (program.tile_runs)
         # fused method: keep each tensor-core block's input state for the backward
         # ("auto": when a backward may follow and the states fit in memory)
         self.checkpoint = d["checkpoint"]

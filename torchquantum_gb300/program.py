@@ -6,7 +6,8 @@ the state is read:
 * every parameterised gate of a supported type (``NATIVE``) gets its operand built
   on the GPU by one ``tqk_gate_operands`` launch for the whole segment, reading its
   parameters in place through their strides (no per-gate torch ops);
-* the plain method then applies each op with its kernel; the fused method plans
+* the plain method then applies the ops in tile passes that gates on any wires share
+  (``tile_runs``), or each with its own kernel; the fused method plans
   blocks of up to 6 wires (``fusion.plan_blocks``; width, planner variant and kernel
   per block chosen by ``autotune.choose_fusion`` from measured pass costs when
   ``fuse_wires == "auto"``), builds every block unitary in float64 with one
