@@ -422,7 +422,7 @@ typedef struct {
 
 typedef struct {
   int32_t tile_bits;   /* 10..14: tile of 2^tile_bits amplitudes; must equal the plan's */
-  int32_t threads;     /* threads per CTA: 128, 256 or 512 */
+  int32_t threads;     /* threads per CTA: 128, 256 or 512 (a preparing warp comes on top) */
   int32_t ctas_per_sm; /* persistent CTAs per SM, 1..8 (clamped to what fits) */
   int32_t pad;
 } tqk_batch_config; /* 16 bytes; NULL = {14, 512, 1} */

@@ -134,7 +134,8 @@ def _circuit(rng, n, depth, bsz):
 @pytest.mark.parametrize("n,bsz,depth", [(9, 2, 80), (10, 5, 150), (11, 5, 80), (12, 1, 140), (13, 3, 90), (15, 2, 150),
                                          (18, 1, 60)])
 def test_tile_passes_match_gate_by_gate_and_oracle(n, bsz, depth, monkeypatch):
-    monkeypatch.setattr(P, "TILE_SHORT_ROW_AMPS", 0)  # short rows take the tiled kernels too
+    monkeypatch.setattr(P, "TILE_SHORT_ROW_AMPS", 0)  # small states take the tiled kernels too
+    monkeypatch.setattr(P, "TILE_MIN_AMPS", 0)
     import torchquantum_gb300 as tq
     import torchquantum_gb300.functional as tqf
 

@@ -304,9 +304,9 @@ __global__ void __launch_bounds__(256) k_dense_adj(const DenseParams<D> p) {
 }
 
 // ------------------------------------------------------------------ dense k, 7 wires and more
-// (3 to 6 wires: dense_tile.cu, but for small reverse steps, see dense_entry.)  One block stages gpb groups (2^k amplitudes each) in shared
-// memory, applies the matrix and writes back.  Thread idx maps to (group gi = idx % gpb,
-// row r = idx / gpb), so a warp shares its matrix row.
+// (3 to 6 wires: dense_tile.cu, but for small reverse steps, see dense_entry.)  One block stages
+// gpb groups (2^k amplitudes each) in shared memory, applies the matrix and writes back.  Thread
+// idx maps to (group gi = idx % gpb, row r = idx / gpb), so a warp shares its matrix row.
 struct DenseKParams {
   float2* state;
   float2* lam;                      // adjoint only

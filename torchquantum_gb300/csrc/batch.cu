@@ -52,9 +52,10 @@ __device__ __forceinline__ unsigned long long global_ns() {
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 
 // ------------------------------------------------------------------ sweeps
-// A pass's ops run from registers (sweep.cuh): the ops are taken in order, a sweep ending before the op whose target would be the fifth besides
-// tile bit 0 (or after kSweepOps).  A warp of its own reads the ops ahead of the others, cuts
-// the next sweep and writes it out while they run the current one, so a sweep costs them one
+// A pass's ops run from registers (sweep.cuh): the ops are taken in order, a sweep ending before
+// the op whose target would be the fifth besides tile bit 0 (or after kSweepOps; with 16
+// amplitudes a thread, the fourth).  A warp of its own reads the ops ahead of the others, cuts the
+// next sweep and writes it out while they run the current one, so a sweep costs them one
 // barrier, the one after its stores.  (Reading and cutting in every warp between the barriers:
 // 13.3 ms below.)
 // What bounds it: float32 multiply-adds (8 per amplitude and one-qubit op: 4.9 us of the 11 us a
@@ -489,7 +490,8 @@ __global__ void __launch_bounds__(THREADS + 32, MINB)
         atomicAdd(pass_done + W.pass, 1);
       }
       __syncthreads();  // the other slot's item is done with
-      if (maker) fetch_item(work[cur ^ 1], tab_buf[cur ^ 1], circ, ops, passes, items, n_items, states, counter, max_tb);
+      if (maker)
+        fetch_item(work[cur ^ 1], tab_buf[cur ^ 1], circ, ops, passes, items, n_items, states, counter, max_tb);
       __syncthreads();
       continue;
     }

@@ -1086,8 +1086,8 @@ bool overlaps(const void* a, const void* b, int64_t bytes) {
   return x != y && x < y + static_cast<uintptr_t>(bytes) && y < x + static_cast<uintptr_t>(bytes);
 }
 
-int adjoint_entry(const void* psi, float2* psi_out, const void* lam_in, void* lam, int64_t bsz, int n, const int32_t* wires,
-                  const void* image_h, int64_t u_batch, double* mr_out, int* status, void* stream, const char* what) {
+int adjoint_entry(const void* psi, float2* psi_out, const void* lam_in, void* lam, int64_t bsz, int n,
+                  const int32_t* wires, const void* image_h, int64_t u_batch, double* mr_out, int* status, void* stream, const char* what) {
   int rc = check_state(psi, bsz, n, what);
   if (rc) return rc;
   if ((rc = check_state(lam, bsz, n, what))) return rc;

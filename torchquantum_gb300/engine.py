@@ -41,7 +41,6 @@ class TapeOp:
     native = None   # the parameterised gate (program.NativeGate) the operand is built from ..
     op128 = None    # .. its complex128 operand and that operand's address
     ptr128 = 0
-    members = None  # the ops of a fused block
     const = None    # the constant gate (its template op) this is an application of
     _op128_keep = None  # complex128 operand of an op without parameters
 

@@ -389,7 +389,7 @@ class Segment:
         for i, op in enumerate(self.exec_ops):
             if isinstance(op, StagedRun):
                 recs.append(_staged_record(op, op.descs(), keep))
-            elif op.members is not None:
+            elif getattr(op, "members", None) is not None:
                 if not op.tc:
                     recs.append(_exec(_lib.X_BLOCK_DENSE, op.wires, batch=op.block_batch, operand=op.operand))
                     continue
@@ -493,7 +493,7 @@ class Segment:
                     slots.append(slot)
                 recs.append(_staged_record(op, op.descs(slots), keep))
                 continue
-            if op.members is not None:
+            if getattr(op, "members", None) is not None:
                 slot = None
                 if gu is not None and _block_needs_grad(op):
                     slot = _as_real(gu, op.u128, self.u128)
@@ -786,11 +786,14 @@ def stage_runs(ops, n: int, min_run: int = 2):
 # than this its ops must together cost at least that on their own kernels to share a pass;
 # a smaller state stays in L2, where launches cost more than bytes.
 TILE_L2_BYTES = 32 << 20
-# Rows of at most 2^12 amplitudes are one tile either way.  Up to 2^21 amplitudes in all the
-# run keeps the op-by-op kernels of staged.cu, whose order of operations its results are
-# known by: there a step is host bound (n = 10, bsz = 256, 100 gates: 162 us of 3.3 ms in
-# these kernels, 128 us in the tiled ones).  Above, the tiled kernels' rate counts.
+# Where a step is bound by the host (35 us a gate, forward and backward), the kernels of one gate
+# and the staged runs stay, whose order of operations results are known by.  Rows of at most 2^12
+# amplitudes are one tile either way: up to 2^21 amplitudes in all (n = 10, bsz = 256, 100 gates:
+# 162 us of 3.3 ms in the staged kernels, 128 us in the tiled ones).  Longer rows: below 2^20 in all
+# (60 gates with backward, ms: n = 13, bsz = 64 2.20 so and 2.11 in tile passes; n = 16, bsz = 16,
+# 2^20 amplitudes, 2.21 and 2.00; n = 18, bsz = 8, 2^21, 2.42 and 2.02).
 TILE_SHORT_ROW_AMPS = 1 << 22
+TILE_MIN_AMPS = 1 << 20
 _TILE_PLANS: dict = {}
 
 
@@ -852,9 +855,10 @@ def plan_tiles(ops, n: int, small: bool) -> List[tuple]:
 
 def tile_runs(ops, n: int, bsz: int):
     """The plain method's execution list: ``StagedRun`` passes and ops on their own kernels.
-    Short rows take ``stage_runs``; the others are cut by ``plan_tiles``, memoised on the
+    Small states take ``stage_runs``; the others are cut by ``plan_tiles``, memoised on the
     circuit's structure."""
-    if n < _lib.TILED_MIN_WIRES or (n <= _lib.STAGED_MAX_TILE_BITS and (bsz << n) < TILE_SHORT_ROW_AMPS):
+    if n < _lib.TILED_MIN_WIRES or \
+            (bsz << n) < (TILE_SHORT_ROW_AMPS if n <= _lib.STAGED_MAX_TILE_BITS else TILE_MIN_AMPS):
         return stage_runs(ops, n)
     small = (bsz << (n + 3)) <= TILE_L2_BYTES
     key = (n, small, tuple((op.kind, tuple(op.wires), len(op.controls), stageable(op, n, n)) for op in ops))
