@@ -588,7 +588,10 @@ __global__ void k_block_build(const tqk_block_desc* blocks, const tqk_block_op* 
   for (int i = 0; i <= bl.num_ops; ++i) {
     const bool last = i == bl.num_ops;  // then only the bits that no op touches are left
     const int q = i % kChunk;
-    if (!last && q == 0) stage_ops(sh, bl, ops, i, b);
+    if (!last && q == 0) {
+      __syncthreads();  // a skipped op at the end of the chunk before has no barrier after its kind is read
+      stage_ops(sh, bl, ops, i, b);
+    }
     if (!last && sh.op[q].kind < 0) continue;  // uniform for the CTA
     const int reach = last ? bl.k : sh.op[q].reach;
     while (p.reach < reach) {  // join: U <- U (x) identity on the next bit
