@@ -919,7 +919,7 @@ int dense_entry(void* state, void* lam, int64_t bsz, int n, const int32_t* contr
   if (nc > 0) return fail(TQK_UNSUPPORTED, "%s: controlled gates take 1 or 2 targets", what);
   // 3 to 6 wires: tiles (dense_tile.cu), but for a reverse step with a cotangent on a small
   // state, which fits a few CTAs: k = 3, 4, 5 at 2^15 / 2^16 amplitudes took 10-11, 12-14 and
-  // 22-23 us op by op, 16, 20 and 27 us in tiles; at 2^21 it is 138, 142, 111 against 39, 50, 66.
+  // 22-23 us op by op, 16, 20 and 27 us in tiles; at 2^21 it is 138, 142, 111 against 39, 55, 77.
   const bool small_reverse = adjoint && grad != nullptr && kt <= 5 && (bsz << n) <= (1ll << 18);
   if (kt >= kTileMinWires && kt <= kTileMaxWires && !small_reverse) {
     DenseTileArgs a{ps, ps, pl, pl, bsz, n, kt, s.tb, pm, pi, mat_batch, grad, false};

@@ -9,8 +9,8 @@
 // (k_dense_k, k_dense_k_adj in apply.cu) every complex multiply-add takes two shared loads, in
 // reverse one from global memory.  n = 22, bsz = 8 (S = 268 MB), k = 3 / 4 / 5 / 6, us: forward
 // 707 / 677 / 783 / 1100 before, 140 / 173 / 237 / 382 here (float32 pipe alone 29 / 58 / 116 /
-// 232, 2 S of HBM 79); reverse with cotangent 2091 / 2096 / 1525 / 2635 before, 614 / 735 / 964 /
-// 1409 here.
+// 232, 2 S of HBM 79); reverse with cotangent 2091 / 2096 / 1525 / 2635 before, 603 / 772 / 896 /
+// 1558 here.
 // Each output's sum runs over c in ascending order with one fused multiply-add per product,
 // so states are the same bit for bit as there.
 //
@@ -18,8 +18,10 @@
 // the tile's address bits to (row, column).  The reverse step holds the psi and lam tiles:
 // psi <- U^H psi (or U^-1 psi, or the gate's kept input as it is), the cotangent
 // sum lam_in psi_out^H, lam <- U^H lam.  A thread's part of the cotangent is 4 x 4 entries
-// over a share of the columns: float32 sums of at most 32 columns, those summed in float32
-// over kChunks of them, then a float64 atomic per entry.
+// over a share of the columns: float32 sums of at most 32 columns, as in the kernels above, then
+// pairs of float32 values (sum and error) over the warp's threads and the CTA's tiles, and a
+// float64 atomic per entry at the end.  Pairs cost 5 to 10 % of the step (plain float32 over 256
+// columns and the warp: 614 / 735 / 964 / 1409 us, but errors of that many additions).
 #include <stdint.h>
 
 #include <atomic>
@@ -31,7 +33,7 @@ namespace dtile {
 
 constexpr int kMaxThreads = 256;
 constexpr int kTileBits = 12;
-constexpr int kChunks = 8;   // cotangent sums of 32 columns added up before they go to float64
+constexpr int kChunk = 32;   // columns a thread's cotangent sums take before they go to pairs of float32
 constexpr int kCopies = 16;  // amplitudes a thread copies at most (a tile of 16 per thread)
 
 struct Params {
@@ -171,6 +173,59 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_fwd(const __grid_constant__ 
   }
 }
 
+// ------------------------------------------------------------------ cotangent sums
+// Beyond kChunk columns sums are pairs of float32 values: hi the running sum, lo the sum of its
+// rounding errors, found exactly (Knuth's two-sum).  float64 additions, one warp's in 16 cycles
+// an SM, would take as long as the products they follow.
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float s = __fadd_rn(a, b), v = __fsub_rn(s, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v));
+  return s;
+}
+// The value (an infinite sum has no finite error).  Conversions are float64 operations too: a sum
+// without error takes one instead of three.
+__device__ __forceinline__ double pair_value(float hi, float lo) {
+  double v = static_cast<double>(hi);
+  if (lo != 0.f && isfinite(lo)) v += static_cast<double>(lo);
+  return v;
+}
+
+// Halving steps of a fold: 2^H threads of a warp share a block of entries.
+template <int K>
+constexpr int kHalvings = K == 3 ? 5 : (K == 4 ? 4 : (K == 5 ? 2 : 0));
+
+// tot summed over the 2^H threads by halves (each step hands half of the values over) and added to
+// the thread's 32 >> H pairs; tot becomes zero.
+template <int H>
+__device__ __forceinline__ void fold(float (&tot)[32], float (&hi)[32 >> H], float (&lo)[32 >> H], int gs) {
+  float e[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) e[i] = 0.f;
+#pragma unroll
+  for (int h = 16, o = (1 << H) >> 1; o > 0; h >>= 1, o >>= 1) {
+    const bool up = (gs & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const float send = up ? tot[i] : tot[i + h], keep = up ? tot[i + h] : tot[i];
+      float err;
+      tot[i] = two_sum(keep, __shfl_xor_sync(0xffffffffu, send, o), err);
+      if (h < 16) {
+        const float es = up ? e[i] : e[i + h], ek = up ? e[i + h] : e[i];
+        err += ek + __shfl_xor_sync(0xffffffffu, es, o);
+      }
+      e[i] = err;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < (32 >> H); ++i) {
+    float err;
+    hi[i] = two_sum(hi[i], tot[i], err);
+    lo[i] += err + e[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) tot[i] = 0.f;
+}
+
 enum { PSI_UH = 0, PSI_INV = 1, PSI_KEPT = 2 };
 
 template <int K, int PSI, bool GRAD>
@@ -186,14 +241,16 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
   const int64_t row = blockIdx.y;
   load_plain<K>(p.mat + row * p.mat_stride, w);       // (U^H)[r][c] = conj U[c][r]
   if (PSI == PSI_INV) load_transposed<K>(p.uinv + row * p.mat_stride, wi);
-  float tot[GRAD ? 32 : 1];
+  // cotangent blocks of 4 x 4 entries, the columns shared out over `split` threads per block
+  constexpr int kBlocks = D * D / 16, H = kHalvings<K>, NV = GRAD ? 32 >> H : 1;
+  const int split = static_cast<int>(blockDim.x) / kBlocks;  // a power of two, 2^H at least with a cotangent
+  const int gb = static_cast<int>(threadIdx.x) / split, gs = static_cast<int>(threadIdx.x) % split;
+  float tot[GRAD ? 32 : 1], hi[NV], lo[NV];
 #pragma unroll
   for (int e = 0; e < (GRAD ? 32 : 1); ++e) tot[e] = 0.f;
-  int chunks = 0;
-  // cotangent blocks of 4 x 4 entries, the columns shared out over `split` threads per block
-  constexpr int kBlocks = D * D / 16;
-  const int split = static_cast<int>(blockDim.x) / kBlocks;  // a power of two
-  const int gb = static_cast<int>(threadIdx.x) / split, gs = static_cast<int>(threadIdx.x) % split;
+#pragma unroll
+  for (int e = 0; e < NV; ++e) hi[e] = lo[e] = 0.f;
+  int summed = 0;  // columns in tot
   // entries (gr + D/4 i, gc + D/4 j): neighbouring threads read neighbouring rows
   constexpr int Q = D / 4;
   const int gr = gb / Q, gc = gb % Q;
@@ -213,17 +270,13 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
       __syncthreads();
       cp.store(p, p.state + base, ps);
     }
-    if (GRAD) {  // += sum over the thread's columns (pairs 2 gs, 2 gs + 2 split, ...) of lam conj(psi)
+    if constexpr (GRAD) {  // += sum over the thread's columns (pairs 2 gs, 2 gs + 2 split, ...) of lam conj(psi)
       const int cols = 1 << p.m;
-      for (int cb = 2 * gs; cb < cols; cb += 32 * split) {
-        float2 s[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) s[i][j] = make_float2(0.f, 0.f);
-        const int ce = min(cols, cb + 32 * split);
 #pragma unroll 1
-        for (int c = cb; c < ce; c += 2 * split) {
+      for (int cb = 0; cb < cols; cb += kChunk * split) {
+        const int ce = min(cols, cb + kChunk * split);
+#pragma unroll 1
+        for (int c = cb + 2 * gs; c < ce; c += 2 * split) {
           float4 l[4], y[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -234,46 +287,19 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
 #pragma unroll
           for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = cfma_bconj(hi2(l[i]), hi2(y[j]), cfma_bconj(lo2(l[i]), lo2(y[j]), s[i][j]));
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            tot[2 * (4 * i + j)] += s[i][j].x;
-            tot[2 * (4 * i + j) + 1] += s[i][j].y;
-          }
-        ++chunks;
-      }
-      // the same for every thread: all take as many columns while there are several tiles
-      if (chunks >= kChunks || t + gridDim.x >= p.tiles) {
-        // The sums so far into float64: over the threads of a block of entries in this warp by
-        // halves (each step hands half of the values over), then one atomic per value left.
-        int o = (split < 32 ? split : 32) >> 1, first = 0, left = 32;
-#pragma unroll
-        for (int h = 16; h >= 1; h >>= 1) {
-          if (o > 0) {
-            const bool up = (gs & o) != 0;
-#pragma unroll
-            for (int i = 0; i < h; ++i) {
-              const float send = up ? tot[i] : tot[i + h], keep = up ? tot[i + h] : tot[i];
-              tot[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            for (int j = 0; j < 4; ++j) {
+              float2 v = make_float2(tot[2 * (4 * i + j)], tot[2 * (4 * i + j) + 1]);
+              v = cfma_bconj(hi2(l[i]), hi2(y[j]), cfma_bconj(lo2(l[i]), lo2(y[j]), v));
+              tot[2 * (4 * i + j)] = v.x;
+              tot[2 * (4 * i + j) + 1] = v.y;
             }
-            if (up) first += h;
-            left = h;
-            o >>= 1;
-          }
         }
-        double* gd = p.grad + row * p.grad_stride + 2 * (gr * D + gc);
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (i < left) {
-            const int e = (first + i) >> 1;
-            atomicAdd(gd + 2 * (Q * (e >> 2) * D + Q * (e & 3)) + ((first + i) & 1), static_cast<double>(tot[i]));
-          }
-#pragma unroll
-        for (int e = 0; e < 32; ++e) tot[e] = 0.f;
-        chunks = 0;
+        // the same for every thread: a thread's columns of a tile are 2^k or fewer
+        summed += max(2, (ce - cb) / split);
+        if (K >= 5 || summed >= kChunk || t + gridDim.x >= p.tiles) {
+          fold<H>(tot, hi, lo, gs);
+          summed = 0;
+        }
       }
     }
     float2 acc[4][4];
@@ -283,6 +309,18 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
     __syncthreads();
     cp.store(p, p.lam + base, ls);
     __syncthreads();
+  }
+  if constexpr (GRAD) {  // one atomic per value of the thread's
+    double* gd = p.grad + row * p.grad_stride + 2 * (gr * D + gc);
+    int first = 0;
+#pragma unroll
+    for (int h = 16, o = (1 << H) >> 1; o > 0; h >>= 1, o >>= 1)
+      if (gs & o) first += h;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int e = (first + i) >> 1;
+      atomicAdd(gd + 2 * (Q * (e >> 2) * D + Q * (e & 3)) + ((first + i) & 1), pair_value(hi[i], lo[i]));
+    }
   }
 }
 
@@ -296,12 +334,12 @@ int column_bits(const DenseTileArgs& a, bool grad) {
   return m;
 }
 
-// Threads of a CTA: 16 amplitudes each, at least a warp; the cotangent needs one per 4 x 4
-// block of its entries.
+// Threads of a CTA: 16 amplitudes each, at least a warp; the cotangent needs 2^H per 4 x 4 block of
+// its entries.
 int threads_of(int k, int m, bool grad) {
   int t = 1 << (k + m < 9 ? 5 : k + m - 4);
-  if (grad && t < (1 << (2 * k)) / 16) t = (1 << (2 * k)) / 16;
-  return t;
+  const int least = k == 3 ? 4 << kHalvings<3> : (k == 4 ? 16 << kHalvings<4> : kMaxThreads);
+  return grad && t < least ? least : t;
 }
 
 // Row stride of a tile: padded so that the rows that neighbouring threads read start in
