@@ -8,9 +8,9 @@
 // float32 pipe is the bound, and HBM where k is small.  With one output per thread and step
 // (k_dense_k, k_dense_k_adj in apply.cu) every complex multiply-add takes two shared loads, in
 // reverse one from global memory.  n = 22, bsz = 8 (S = 268 MB), k = 3 / 4 / 5 / 6, us: forward
-// 707 / 677 / 783 / 1100 before, 140 / 173 / 237 / 382 here (float32 pipe alone 29 / 58 / 116 /
-// 232, 2 S of HBM 79); reverse with cotangent 2091 / 2096 / 1525 / 2635 before, 603 / 772 / 896 /
-// 1558 here.
+// 707 / 677 / 783 / 1100 before, 146 / 178 / 251 / 397 here (float32 pipe alone 29 / 58 / 116 /
+// 232, 2 S of HBM 79); reverse with cotangent 2091 / 2096 / 1525 / 2635 before, 589 / 773 / 902 /
+// 1563 here.
 // Each output's sum runs over c in ascending order with one fused multiply-add per product,
 // so states are the same bit for bit as there.
 //
@@ -20,8 +20,8 @@
 // sum lam_in psi_out^H, lam <- U^H lam.  A thread's part of the cotangent is 4 x 4 entries
 // over a share of the columns: float32 sums of at most 32 columns, as in the kernels above, then
 // pairs of float32 values (sum and error) over the warp's threads and the CTA's tiles, and a
-// float64 atomic per entry at the end.  Pairs cost 5 to 10 % of the step (plain float32 over 256
-// columns and the warp: 614 / 735 / 964 / 1409 us, but errors of that many additions).
+// float64 atomic per entry at the end.  (Plain float32 over 256 columns and the warp took 614 / 735 /
+// 964 / 1409 us, with the errors of that many additions.)
 #include <stdint.h>
 
 #include <atomic>
@@ -43,7 +43,8 @@ struct Params {
   float2* lam;
   int n, m;                  // qubits; column bits of a tile
   int ld;                    // row stride of a tile in shared memory (even: 16-byte pairs)
-  int64_t tiles;             // tiles per row
+  int tiles_log;             // tiles per row: 2^tiles_log
+  int64_t items;             // tiles of all rows (below 2^31)
   uint64_t outer;            // index bits outside the tile
   int bits;                  // address bits of a tile: k + m
   uint8_t pos[kTileBits];    // index bit of the tile's address bit j (ascending)
@@ -92,6 +93,27 @@ struct Copy {
       if (i < count) dst[off + p.coff[i]] = tile[at + p.cstep[i]];
   }
 };
+
+// Work: the tiles of all rows.  With one matrix for all rows the CTAs take them in turn (neighbouring
+// tiles at the same time), with a matrix a row an even share of neighbouring ones each.
+// (CTAs of one row each, rounded down to whole rows, left up to half of the places for CTAs empty:
+// n = 16, k = 5 reverse with cotangent, 153 / 305 rows 513 / 829 us, now 296 / 535.)
+// I: 32 bits forward, 64 in reverse, as the registers come out (n = 22, bsz = 8: k = 6 forward 394
+// us, 417 with 64; kept input, k = 3 reverse 299 us, 341 with 32).
+template <typename I>
+struct Items {
+  I it, end;
+  uint32_t step;
+};
+template <typename I>
+__device__ __forceinline__ Items<I> items_of(const Params& p) {
+  if (p.mat_stride == 0) return {static_cast<I>(blockIdx.x), static_cast<I>(p.items), gridDim.x};
+  return {static_cast<I>(p.items * blockIdx.x / gridDim.x), static_cast<I>(p.items * (blockIdx.x + 1) / gridDim.x), 1u};
+}
+template <typename I>
+__device__ __forceinline__ uint64_t item_base(const Params& p, I it) {
+  return (static_cast<uint64_t>(it >> p.tiles_log) << p.n) + deposit(it & ((I(1) << p.tiles_log) - I(1)), p.outer);
+}
 
 // mt[c * D + r] = M[r][c]
 template <int K>
@@ -157,19 +179,23 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_fwd(const __grid_constant__ 
   float2* x = w + D * D;
   const Copy cp(p);
   const Block b = block_of<K>(p);
-  const int64_t row = blockIdx.y;
-  load_transposed<K>(p.mat + row * p.mat_stride, w);
-  for (int64_t t = blockIdx.x; t < p.tiles; t += gridDim.x) {
-    const uint64_t base = (static_cast<uint64_t>(row) << p.n) + deposit(static_cast<uint64_t>(t), p.outer);
-    cp.load(p, p.in + base, x);
-    __syncthreads();
-    float2 acc[4][4];
-    if (b.active) product<K, false>(p.ld, b, w, x, acc);
-    __syncthreads();
-    if (b.active) put_block(p.ld, b, acc, x);
-    __syncthreads();
-    cp.store(p, p.state + base, x);
-    __syncthreads();
+  auto todo = items_of<uint32_t>(p);
+  while (todo.it < todo.end) {
+    // the items that share a matrix
+    const uint32_t end = p.mat_stride == 0 ? todo.end : min(todo.end, ((todo.it >> p.tiles_log) + 1u) << p.tiles_log);
+    load_transposed<K>(p.mat + (todo.it >> p.tiles_log) * p.mat_stride, w);
+    for (; todo.it < end; todo.it += todo.step) {
+      const uint64_t base = item_base(p, todo.it);
+      cp.load(p, p.in + base, x);
+      __syncthreads();
+      float2 acc[4][4];
+      if (b.active) product<K, false>(p.ld, b, w, x, acc);
+      __syncthreads();
+      if (b.active) put_block(p.ld, b, acc, x);
+      __syncthreads();
+      cp.store(p, p.state + base, x);
+      __syncthreads();
+    }
   }
 }
 
@@ -238,9 +264,6 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
   float2* ls = ps + D * p.ld;
   const Copy cp(p);
   const Block b = block_of<K>(p);
-  const int64_t row = blockIdx.y;
-  load_plain<K>(p.mat + row * p.mat_stride, w);       // (U^H)[r][c] = conj U[c][r]
-  if (PSI == PSI_INV) load_transposed<K>(p.uinv + row * p.mat_stride, wi);
   // cotangent blocks of 4 x 4 entries, the columns shared out over `split` threads per block
   constexpr int kBlocks = D * D / 16, H = kHalvings<K>, NV = GRAD ? 32 >> H : 1;
   const int split = static_cast<int>(blockDim.x) / kBlocks;  // a power of two, 2^H at least with a cotangent
@@ -254,8 +277,20 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
   // entries (gr + D/4 i, gc + D/4 j): neighbouring threads read neighbouring rows
   constexpr int Q = D / 4;
   const int gr = gb / Q, gc = gb % Q;
-  for (int64_t t = blockIdx.x; t < p.tiles; t += gridDim.x) {
-    const uint64_t base = (static_cast<uint64_t>(row) << p.n) + deposit(static_cast<uint64_t>(t), p.outer);
+  auto todo = items_of<int64_t>(p);
+  // one loop over items and matrices (a loop of its own for each matrix's items spills: kept input,
+  // k = 3, n = 22, bsz = 8 373 us, this 299)
+  int64_t row = -1;
+  for (; todo.it < todo.end; todo.it += todo.step) {
+    const int64_t was = row;
+    row = todo.it >> p.tiles_log;
+    if (was < 0 || (row != was && p.mat_stride != 0)) {
+      load_plain<K>(p.mat + row * p.mat_stride, w);  // (U^H)[r][c] = conj U[c][r]
+      if (PSI == PSI_INV) load_transposed<K>(p.uinv + row * p.mat_stride, wi);
+    }
+    // the last item of its matrix
+    const bool last = todo.it + todo.step >= todo.end || (p.grad_stride != 0 && (todo.it + 1) >> p.tiles_log != row);
+    const uint64_t base = item_base(p, todo.it);
     if (PSI != PSI_KEPT || GRAD) cp.load(p, (PSI == PSI_KEPT ? p.in : p.state) + base, ps);
     cp.load(p, p.lam_in + base, ls);
     __syncthreads();
@@ -296,7 +331,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
         }
         // the same for every thread: a thread's columns of a tile are 2^k or fewer
         summed += max(2, (ce - cb) / split);
-        if (K >= 5 || summed >= kChunk || t + gridDim.x >= p.tiles) {
+        if (K >= 5 || summed >= kChunk || last) {
           fold<H>(tot, hi, lo, gs);
           summed = 0;
         }
@@ -308,19 +343,22 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_adj(const __grid_constant__ 
     if (b.active) put_block(p.ld, b, acc, ls);
     __syncthreads();
     cp.store(p, p.lam + base, ls);
-    __syncthreads();
-  }
-  if constexpr (GRAD) {  // one atomic per value of the thread's
-    double* gd = p.grad + row * p.grad_stride + 2 * (gr * D + gc);
-    int first = 0;
+    if constexpr (GRAD) {
+      if (last) {  // one atomic per value of the thread's
+        double* gd = p.grad + row * p.grad_stride + 2 * (gr * D + gc);
+        int first = 0;
 #pragma unroll
-    for (int h = 16, o = (1 << H) >> 1; o > 0; h >>= 1, o >>= 1)
-      if (gs & o) first += h;
+        for (int h = 16, o = (1 << H) >> 1; o > 0; h >>= 1, o >>= 1)
+          if (gs & o) first += h;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int e = (first + i) >> 1;
-      atomicAdd(gd + 2 * (Q * (e >> 2) * D + Q * (e & 3)) + ((first + i) & 1), pair_value(hi[i], lo[i]));
+        for (int i = 0; i < NV; ++i) {
+          const int e = (first + i) >> 1;
+          atomicAdd(gd + 2 * (Q * (e >> 2) * D + Q * (e & 3)) + ((first + i) & 1), pair_value(hi[i], lo[i]));
+          hi[i] = lo[i] = 0.f;
+        }
+      }
     }
+    __syncthreads();
   }
 }
 
@@ -358,7 +396,8 @@ void fill(Params& p, const DenseTileArgs& a, int m, int threads) {
   p.m = m;
   p.ld = row_stride(a.k, p.m);
   p.bits = a.k + p.m;
-  p.tiles = 1ll << (a.n - p.bits);
+  p.tiles_log = a.n - p.bits;
+  p.items = a.bsz << p.tiles_log;
   uint64_t tgt = 0, used = 0;
   for (int j = 0; j < a.k; ++j) tgt |= 1ull << a.tbits[j];
   int bit = 0, cols = 0;
@@ -399,7 +438,7 @@ int reserve(const void* kern, std::atomic<uint64_t>& done, int dev, size_t bytes
 }
 
 template <typename Kernel>
-int launch(Kernel kern, std::atomic<uint64_t>& done, const Params& p, int64_t bsz, int threads, size_t smem, size_t top,
+int launch(Kernel kern, std::atomic<uint64_t>& done, const Params& p, int threads, size_t smem, size_t top,
            const char* what, cudaStream_t st) {
   int dev = 0, sms = 0, fit = 0;
   cudaGetDevice(&dev);
@@ -407,11 +446,9 @@ int launch(Kernel kern, std::atomic<uint64_t>& done, const Params& p, int64_t bs
   int rc = reserve(reinterpret_cast<const void*>(kern), done, dev, top);
   if (rc) return rc;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, smem) != cudaSuccess || fit < 1) fit = 1;
-  // resident CTAs only: each loads its matrix (and flushes its cotangent) once
-  int64_t gx = static_cast<int64_t>(sms) * fit / bsz;
-  if (gx > p.tiles) gx = p.tiles;
-  if (gx < 1) gx = 1;
-  kern<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(bsz), 1), threads, smem, st>>>(p);
+  // resident CTAs only: each loads its matrices (and flushes their cotangents) once
+  const int64_t slots = static_cast<int64_t>(sms) * fit;
+  kern<<<static_cast<unsigned>(slots < p.items ? slots : p.items), threads, smem, st>>>(p);
   return launch_status(what);
 }
 
@@ -422,7 +459,7 @@ int launch_fwd(const DenseTileArgs& a, cudaStream_t st) {
   Params p;
   fill(p, a, m, threads);
   constexpr size_t mat = sizeof(float2) << (2 * K);
-  return launch(k_fwd<K>, done, p, a.bsz, threads, mat + tile_bytes(K, p.m), mat + tile_bytes(K, kTileBits - K),
+  return launch(k_fwd<K>, done, p, threads, mat + tile_bytes(K, p.m), mat + tile_bytes(K, kTileBits - K),
                 "dense k-wire gate", st);
 }
 
@@ -433,7 +470,7 @@ int launch_adj(const DenseTileArgs& a, cudaStream_t st) {
   Params p;
   fill(p, a, m, threads);
   constexpr size_t mat = (PSI == PSI_INV ? 2 : 1) * (sizeof(float2) << (2 * K));
-  return launch(k_adj<K, PSI, GRAD>, done, p, a.bsz, threads, mat + 2 * tile_bytes(K, p.m),
+  return launch(k_adj<K, PSI, GRAD>, done, p, threads, mat + 2 * tile_bytes(K, p.m),
                 mat + 2 * tile_bytes(K, kTileBits - K), "adjoint dense k-wire gate", st);
 }
 
