@@ -59,13 +59,14 @@ __device__ __forceinline__ pair make(float lo, float hi) {
     static __device__ __forceinline__ void flip(pair s) {                                                         \
       asm volatile("xor.b64 t" P "%0, t" P "%0, %1;" ::"n"(Q), "l"(s));                                            \
     }                                                                                                             \
-    /* (Q, U) <- real 2x2 */                                                                                      \
+    /* (Q, U) <- real 2x2.  Here and below an output's products with its own input come last: in gates near  \
+       the identity they are the large ones, and only the last addition rounds at their size */                 \
     template <int Q, int U>                                                                                       \
     static __device__ __forceinline__ void real2(const Factor (&m)[4]) {                                          \
       asm volatile(                                                                                               \
           "{\n .reg .b64 t, u;\n"                                                                                 \
-          " mul.rn.f32x2 t, %2, t" P "%0;\n mul.rn.f32x2 u, %4, t" P "%0;\n"                                       \
-          " fma.rn.f32x2 t" P "%0, %3, t" P "%1, t;\n fma.rn.f32x2 t" P "%1, %5, t" P "%1, u;\n}" ::"n"(Q),       \
+          " mul.rn.f32x2 t, %3, t" P "%1;\n mul.rn.f32x2 u, %4, t" P "%0;\n"                                       \
+          " fma.rn.f32x2 t" P "%0, %2, t" P "%0, t;\n fma.rn.f32x2 t" P "%1, %5, t" P "%1, u;\n}" ::"n"(Q),       \
           "n"(U), "l"(m[0].r), "l"(m[1].r), "l"(m[2].r), "l"(m[3].r));                                            \
     }                                                                                                             \
     /* (Q, U) <- complex 2x2: the imaginary products of both inputs first */                                      \
@@ -74,12 +75,12 @@ __device__ __forceinline__ pair make(float lo, float hi) {
       asm volatile(                                                                                               \
           "{\n .reg .f32 x, y, z, w, ny, nw, p, q;\n .reg .b64 t, u;\n"                                            \
           " mov.b64 {x, y}, t" P "%0;\n mov.b64 {z, w}, t" P "%1;\n neg.f32 ny, y;\n neg.f32 nw, w;\n"             \
-          " mul.rn.f32 p, %6, ny;\n mul.rn.f32 q, %6, x;\n"                                                        \
-          " fma.rn.f32 p, %7, nw, p;\n fma.rn.f32 q, %7, z, q;\n mov.b64 t, {p, q};\n"                             \
+          " mul.rn.f32 p, %7, nw;\n mul.rn.f32 q, %7, z;\n"                                                        \
+          " fma.rn.f32 p, %6, ny, p;\n fma.rn.f32 q, %6, x, q;\n mov.b64 t, {p, q};\n"                             \
           " mul.rn.f32 p, %8, ny;\n mul.rn.f32 q, %8, x;\n"                                                        \
           " fma.rn.f32 p, %9, nw, p;\n fma.rn.f32 q, %9, z, q;\n mov.b64 u, {p, q};\n"                             \
-          " fma.rn.f32x2 t, %2, t" P "%0, t;\n fma.rn.f32x2 u, %4, t" P "%0, u;\n"                                 \
-          " fma.rn.f32x2 t" P "%0, %3, t" P "%1, t;\n fma.rn.f32x2 t" P "%1, %5, t" P "%1, u;\n}" ::"n"(Q),       \
+          " fma.rn.f32x2 u, %4, t" P "%0, u;\n fma.rn.f32x2 t, %3, t" P "%1, t;\n"                                 \
+          " fma.rn.f32x2 t" P "%1, %5, t" P "%1, u;\n fma.rn.f32x2 t" P "%0, %2, t" P "%0, t;\n}" ::"n"(Q),       \
           "n"(U), "l"(m[0].r), "l"(m[1].r), "l"(m[2].r), "l"(m[3].r), "f"(m[0].i), "f"(m[1].i), "f"(m[2].i),      \
           "f"(m[3].i));                                                                                           \
     }                                                                                                             \
