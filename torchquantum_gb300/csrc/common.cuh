@@ -59,6 +59,23 @@ __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); 
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 __device__ __forceinline__ float4 pack4(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
 
+// ------------------------------------------------------------------ pairs of float32
+// Sums that float32 alone would not hold are pairs: hi the running sum, lo the sum of its rounding
+// errors, found exactly (Knuth's two-sum).  float64 additions, one warp's in 16 cycles an SM, would
+// take as long as the products they follow.
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float s = __fadd_rn(a, b), v = __fsub_rn(s, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v));
+  return s;
+}
+// The value (an infinite sum has no finite error).  Conversions are float64 operations too: a sum
+// without error takes one instead of three.
+__device__ __forceinline__ double pair_value(float hi, float lo) {
+  double v = static_cast<double>(hi);
+  if (lo != 0.f && isfinite(lo)) v += static_cast<double>(lo);
+  return v;
+}
+
 // ------------------------------------------------------------------ block reductions
 // Sum NV float accumulators of every thread of the block into NV doubles, then
 // atomically add them to dst[0..NV) (one atomic per value per block).  Warp level in

@@ -200,22 +200,6 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_fwd(const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------ cotangent sums
-// Beyond kChunk columns sums are pairs of float32 values: hi the running sum, lo the sum of its
-// rounding errors, found exactly (Knuth's two-sum).  float64 additions, one warp's in 16 cycles
-// an SM, would take as long as the products they follow.
-__device__ __forceinline__ float two_sum(float a, float b, float& err) {
-  const float s = __fadd_rn(a, b), v = __fsub_rn(s, a);
-  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v));
-  return s;
-}
-// The value (an infinite sum has no finite error).  Conversions are float64 operations too: a sum
-// without error takes one instead of three.
-__device__ __forceinline__ double pair_value(float hi, float lo) {
-  double v = static_cast<double>(hi);
-  if (lo != 0.f && isfinite(lo)) v += static_cast<double>(lo);
-  return v;
-}
-
 // Halving steps of a fold: 2^H threads of a warp share a block of entries.
 template <int K>
 constexpr int kHalvings = K == 3 ? 5 : (K == 4 ? 4 : (K == 5 ? 2 : 0));

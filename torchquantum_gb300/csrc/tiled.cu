@@ -19,9 +19,10 @@
 //   What bounds it: issue slots, then the float32 pipe.  A dense op is 8 multiply-adds per
 //   amplitude forward (6 issue slots, f32x2.cuh) and 24 in reverse with its cotangent; its
 //   factors are read once per thread from a table in shared memory, and a crossing (2
-//   instructions per amplitude) is shared by all ops of a sweep.  Measured per dense op at
-//   n = 22, bsz = 8: 12.2 us forward and 36 us in reverse (float32 pipe alone: 7.2 and 22);
-//   one op per shared-memory crossing (staged.cu): 24 and 70 us.
+//   instructions per amplitude) is shared by all ops of a sweep.  Measured per op of 120
+//   RX, RY and RZ at n = 22, bsz = 8: 11.9 us forward and 39 us in reverse (36.5 with plain
+//   float32 sums over the warp; float32 pipe alone: 7.2 and 22 a dense op); one op per
+//   shared-memory crossing (staged.cu): 24 and 70 us.
 //   Registers: 16 amplitudes are 32 registers forward, 64 for the reverse pass's psi and
 //   lam, so 256 threads fit 3 and 2 CTAs per SM, whose loads, sweeps and stores overlap.
 //   (32 amplitudes per thread: 3 % faster forward, 10 % slower in reverse; 4 CTAs of 64
@@ -29,7 +30,9 @@
 //
 // The reverse pass holds the psi and lam tiles of the same amplitudes and walks the run
 // backwards: psi <- U^H psi, lam <- U^H lam and, for ops with a cotangent slot,
-// sum lam_in conj(psi_out): float32 over a thread's amplitudes and a warp, float64 beyond.
+// sum lam_in conj(psi_out): float32 over a thread's amplitudes and eight threads (64 terms, as in
+// the kernels of one gate), pairs of float32 (sum and error) over the warps and tiles, float64
+// where the CTAs' sums meet.
 #include <stdint.h>
 
 #include <atomic>
@@ -451,21 +454,31 @@ __device__ __forceinline__ void apply_adj(int j, int go, const Source& src, uint
   }
 }
 
-// Sum v[0..8) over the warp: afterwards lane L holds the sum of value (L >> 2).
-__device__ __forceinline__ float warp_sum8(float (&v)[8], int lane) {
+// Sum v[0..8) over the warp: afterwards lane L holds the sum of value (L >> 2) as a pair (sum, error):
+// plain float32 over eight threads, exact beyond (16: a thread's part is of 16 terms, not 8: over four).
+__device__ __forceinline__ float warp_sum8(float (&v)[8], bool of16, int lane, float& err) {
 #pragma unroll
-  for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+  for (int h = 4, o = 16; h >= 2; h >>= 1, o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (i >= h) break;
+    for (int i = 0; i < h; ++i) {
       const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  float s = v[0];
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  const bool up = (lane & 4) != 0;
+  float s = up ? v[1] : v[0], r = __shfl_xor_sync(0xffffffffu, up ? v[0] : v[1], 4), e;
+  if (of16) {  // uniform
+    s = two_sum(s, r, err);
+    err += __shfl_xor_sync(0xffffffffu, err, 2);
+    s = two_sum(s, __shfl_xor_sync(0xffffffffu, s, 2), e);
+    err += e;
+  } else {
+    s += r;
+    s = two_sum(s, __shfl_xor_sync(0xffffffffu, s, 2), err);
+  }
+  s = two_sum(s, __shfl_xor_sync(0xffffffffu, s, 1), e);
+  err += __shfl_xor_sync(0xffffffffu, err, 1) + e;
   return s;
 }
 
@@ -475,17 +488,17 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
   float2* ps = reinterpret_cast<float2*>(sm4);
   float2* ls = ps + (1u << p.m);
   float4* fac = reinterpret_cast<float4*>(ls + (1u << p.m));
-  // a tile's warp sums in gtile [ngrad][warps][8], their float64 sums over warps and tiles
-  // in gacc [ngrad][8]
+  // a tile's warp sums in gtile [ngrad][warps][8 sums, 8 errors], their sums over warps and tiles
+  // in gacc [ngrad][8], pairs too
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int nacc = p.ngrad * 8;
-  double* gacc = reinterpret_cast<double*>(fac + p.nops * 4);
+  float2* gacc = reinterpret_cast<float2*>(fac + p.nops * 4);
   float* gtile = reinterpret_cast<float*>(gacc + nacc);
-  Decoded* dec = reinterpret_cast<Decoded*>(gtile + nacc * warps);
+  Decoded* dec = reinterpret_cast<Decoded*>(gtile + 2 * nacc * warps);
   uint32_t* tab = reinterpret_cast<uint32_t*>(dec + p.nops);
   build_tables(p, tab);
   build_ops<true>(p, fac, dec);
-  for (int i = threadIdx.x; i < nacc; i += blockDim.x) gacc[i] = 0.0;
+  for (int i = threadIdx.x; i < nacc; i += blockDim.x) gacc[i] = make_float2(0.f, 0.f);
   const Source src{p, fac};
   for (int64_t t = blockIdx.x; t < p.tiles; t += gridDim.x) {
     const uint64_t base = deposit(static_cast<uint64_t>(t), p.outer);
@@ -505,9 +518,9 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
 #pragma unroll 1
       for (int j = sw.first + sw.count - 1; j >= sw.first; --j) {
         const Decoded d = dec[j];
-        float* gw = gtile + (d.gidx * warps + warp) * 8;
+        float* gw = gtile + (d.gidx * warps + warp) * 16;
         if ((base & d.omask) != d.oval) {  // uniform for the tile
-          if (d.gidx >= 0 && lane < 8) gw[lane] = 0.f;
+          if (d.gidx >= 0 && lane < 16) gw[lane] = 0.f;
           continue;
         }
         const bool on = (tl & d.tmask) == d.tval;
@@ -524,8 +537,12 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
           v[2 * k.value + 1] = g.y;
         });
         __syncwarp();
-        const float sum = warp_sum8(v, lane);
-        if ((lane & 3) == 0) gw[lane >> 2] = sum;
+        float err;
+        const float sum = warp_sum8(v, d.go >= GO_SCALE, lane, err);
+        if ((lane & 3) == 0) {
+          gw[lane >> 2] = sum;
+          gw[8 + (lane >> 2)] = err;
+        }
       }
       const uint32_t tp = thread_offset(tab, s) >> 16;
       store_regs<f2::Psi>(sw.rphys, ps, tp);
@@ -538,9 +555,14 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
       store_tile(p, f, p.lam, ls);
     }
     for (int i = threadIdx.x; i < nacc; i += blockDim.x) {
-      double s = 0.0;
-      for (int w = 0; w < warps; ++w) s += static_cast<double>(gtile[((i >> 3) * warps + w) * 8 + (i & 7)]);
-      gacc[i] += s;
+      float2 g = gacc[i];
+      for (int w = 0; w < warps; ++w) {
+        const float* gw = gtile + ((i >> 3) * warps + w) * 16 + (i & 7);
+        float e;
+        g.x = two_sum(g.x, gw[0], e);
+        g.y += gw[8] + e;
+      }
+      gacc[i] = g;
     }
     __syncthreads();
   }
@@ -548,7 +570,10 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
   for (int i = threadIdx.x; i < p.nops * 8; i += blockDim.x) {
     const SOp& o = p.ops[i >> 3];
     const int v = i & 7;
-    if (o.gidx >= 0 && v < 2 * o.nent) atomicAdd(o.grad + blockIdx.y * o.grad_stride + v, gacc[o.gidx * 8 + v]);
+    if (o.gidx >= 0 && v < 2 * o.nent) {
+      const float2 g = gacc[o.gidx * 8 + v];
+      atomicAdd(o.grad + blockIdx.y * o.grad_stride + v, pair_value(g.x, g.y));
+    }
   }
 }
 
@@ -768,14 +793,14 @@ int tiled_entry(const void* psi_in, const void* lam_in, void* psi, void* lam, in
   const size_t tile = sizeof(float2) << m;
   const size_t tables = nops * (4 * sizeof(float4) + sizeof(tiled::Decoded)) +
                         static_cast<size_t>(p.nsweeps) * tiled::kTabEntries * sizeof(uint32_t);
-  const size_t acc = static_cast<size_t>(p.ngrad) * 8 * (sizeof(double) + threads / 32 * sizeof(float));
+  const size_t acc = static_cast<size_t>(p.ngrad) * 8 * (sizeof(float2) + threads / 32 * 2 * sizeof(float));
   const size_t smem = adjoint ? 2 * tile + acc + tables : tile + tables;
   auto kern = adjoint ? tiled::k_tiled_adj : tiled::k_tiled;
   static std::atomic<uint64_t> configured[2];  // devices whose attribute is set
   const uint64_t bit = 1ull << (dev & 63);
   if (!(configured[adjoint].load() & bit)) {
     constexpr size_t top = 2 * (sizeof(float2) << tiled::kMaxBits) +
-                           TQK_STAGED_MAX_OPS * (8 * (sizeof(double) + tiled::kMaxWarps * sizeof(float)) +
+                           TQK_STAGED_MAX_OPS * (8 * (sizeof(float2) + tiled::kMaxWarps * 2 * sizeof(float)) +
                                                  4 * sizeof(float4) + sizeof(tiled::Decoded) +
                                                  tiled::kTabEntries * sizeof(uint32_t));
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(top)) != cudaSuccess)
