@@ -8,8 +8,8 @@
 // xmasks are grouped and each group is one coset pass (k_coset): the row is cut into
 // cosets of the span of the group's xmasks, staged in shared memory (16-byte cp.async copies), so
 // all partners are read on chip and DRAM reads the state once per group.  Each thread
-// accumulates in float32, blocks reduce in float64 and write one partial per (row,
-// block or coset, string) to scratch; a second kernel adds the partials in a fixed
+// accumulates in float32, blocks reduce in float64 (k_coset: in pairs of float32) and write
+// one float64 partial per (row, block or coset, string) to scratch; a second kernel adds the partials in a fixed
 // order, so results are bitwise reproducible run to run.  The backward seed
 // sum_s c_s P_s psi (k_coset<true>) uses the same coset passes.
 #include <atomic>
@@ -258,14 +258,15 @@ __global__ void __launch_bounds__(kFinishThreads) k_expval_finish(const double* 
 // iteration finished reading, and arrives on that stage's full mbarrier once they land;
 // then all wait for the current stage.  A thread owns eight amplitude pairs of a full stage.
 // Expvals: it keeps them in registers and visits each string's partners in the stage (from one
-// side only where it can), float32 sums over its pairs and its warp; the CTA reduces in float64
-// and writes one partial per (coset, string); the partials are summed per row in a fixed order
-// (k_expval_finish).  Backward seed: it forms sum_s c_s (P_s psi)_u for its pairs and stores
+// side only where it can), float32 sums over its pairs and eight threads (64 visits), pairs of
+// float32 (sum and error) over the CTA, float64 in its one partial per (coset, string); the
+// partials are summed per row in a fixed order (k_expval_finish).  Backward seed: it forms sum_s c_s (P_s psi)_u for its pairs and stores
 // them to the output row, added to what earlier groups left there, which it reads before it
 // waits for the stage.
 // What bounds it: DRAM moves a 64 KB stage in 2800 cycles an SM, the strings' partner reads take
 // 2500 to 4600 of shared memory and about as many issue cycles; they overlap in part.  n = 22,
-// 4 rows, 24 strings: expvals 201 -> 152 us (three groups; 60 at the DRAM rate), seed 369 -> 244 us
+// 4 rows, 24 strings: expvals 201 -> 160 us (three groups; 60 at the DRAM rate; 152 with the CTA's sums
+// in plain float32), seed 369 -> 244 us
 // (158 at the DRAM rate); before, each warp took a segment of the strings' visits (two stage
 // reads, a shift, a population count and a flip each), the seed read the earlier groups' output
 // after its sums, and every thread divided for its coset.
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(kCosetThreads, 1) k_coset(const CosetParams p)
   __shared__ CosetString strings[kMaxStringsPerPass];
   // expvals, by iteration parity: halves of the warps' lanes, sums of half a string's
   __shared__ __align__(16) float half_sum[SEED ? 1 : 2][kMaxStringsPerPass][kCosetThreads / 2];
-  __shared__ float red[2][kCosetWarps];
+  __shared__ float2 red[2][kCosetWarps];
   __shared__ int quit;
   static_assert(kCosetWarps == 2 * kMaxStringsPerPass, "two warps add a string's sums");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -562,8 +563,8 @@ __global__ void __launch_bounds__(kCosetThreads, 1) k_coset(const CosetParams p)
   // the previous iteration's partials: its sums meet in red after the barrier that follows
   auto put_partial = [&](int64_t item, int parity) {
     if (!SEED && static_cast<int>(threadIdx.x) < p.ns) {
-      const double sum = static_cast<double>(red[parity][2 * threadIdx.x]) +
-                         static_cast<double>(red[parity][2 * threadIdx.x + 1]);
+      const float2 a = red[parity][2 * threadIdx.x], b = red[parity][2 * threadIdx.x + 1];
+      const double sum = pair_value(a.x, a.y) + pair_value(b.x, b.y);
       p.partial[item * kMaxStringsPerPass + threadIdx.x] =
           (*vquit == 0) ? sum : __longlong_as_double(0x7ff8000000000000ll);
     }
@@ -646,10 +647,14 @@ __global__ void __launch_bounds__(kCosetThreads, 1) k_coset(const CosetParams p)
       if (it > 0) put_partial(item - gridDim.x, (it - 1) & 1);
       // warps 2 s and 2 s + 1: half of string s's sums each
       const float4 h = *reinterpret_cast<const float4*>(&half_sum[SEED ? 0 : it & 1][warp >> 1][128 * (warp & 1) + 4 * lane]);
-      float a = (h.x + h.y) + (h.z + h.w);
+      float a = (h.x + h.y) + (h.z + h.w), err = 0.f;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane == 0) red[it & 1][warp] = a;
+      for (int o = 16; o > 0; o >>= 1) {
+        float e;
+        a = two_sum(a, __shfl_xor_sync(0xffffffffu, a, o), e);
+        err += __shfl_xor_sync(0xffffffffu, err, o) + e;
+      }
+      if (lane == 0) red[it & 1][warp] = make_float2(a, err);
     }
 #pragma unroll
     for (int k = 0; k < kCosetStages - 1; ++k) reps[k] = reps[k + 1];
