@@ -160,11 +160,19 @@ def _u64(vals: Sequence[int]):
     return (ctypes.c_uint64 * max(1, len(vals)))(*vals)
 
 
-_raw_stream = torch._C._cuda_getCurrentRawStream  # without building a Stream object
+# The current stream's handle without building a Stream object (2 us a launch), where torch has the call
+# (torch built without CUDA does not).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _dstream(device) -> int:
+    if _raw_stream is None or not isinstance(device, torch.device) or device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
 
 
 def _stream(t: torch.Tensor) -> int:
-    return _raw_stream(t.device.index)
+    return _dstream(t.device)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -554,11 +562,6 @@ def cross_to_complex(mr: torch.Tensor) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------ gate programs
-def _dstream(device) -> int:
-    index = device.index
-    return _raw_stream(torch.cuda.current_device() if index is None else index)
-
-
 def gate_operands(table, ngates, device):
     _check(load().tqk_gate_operands(table.data_ptr(), ngates, _dstream(device)))
 

@@ -55,6 +55,11 @@ def _check(rc: int) -> None:
         raise RuntimeError(_load().tqk_last_error().decode(errors="replace"))
 
 
+def _stream(device: torch.device) -> int:
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # without building a Stream object, where torch has it
+    return torch.cuda.current_stream(device).cuda_stream if raw is None else raw(device.index)
+
+
 def _wires(wires) -> List[int]:
     return [int(wires)] if isinstance(wires, int) else [int(w) for w in wires]
 
@@ -85,7 +90,7 @@ class _ApplyUnitary(torch.autograd.Function):
         m = mat.detach().to(x.device, torch.complex64)
         m3 = (m if m.dim() == 3 else m.unsqueeze(0)).resolve_conj().resolve_neg().contiguous()
         w = (ctypes.c_int32 * k)(*wires)
-        stream = torch._C._cuda_getCurrentRawStream(x.device.index)
+        stream = _stream(x.device)
         if _out_of_place(x, bsz, n, k):
             out = torch.empty_like(x)
             _check(lib.tqk_apply_matrix_to(x.data_ptr(), out.data_ptr(), bsz, n, w, k, m3.data_ptr(), m3.shape[0],
@@ -107,7 +112,7 @@ class _ApplyUnitary(torch.autograd.Function):
         need_mat = ctx.needs_input_grad[1]
         grad = torch.zeros(m3.shape[0] * d * d * 2, dtype=torch.float64, device=x.device) if need_mat else None
         w = (ctypes.c_int32 * k)(*ctx.wires)
-        stream = torch._C._cuda_getCurrentRawStream(x.device.index)
+        stream = _stream(x.device)
         if _out_of_place(x, bsz, n, k):
             g = _readable(grad_out, bsz)
             lam = torch.empty_like(g)
