@@ -422,7 +422,8 @@ typedef struct {
 
 typedef struct {
   int32_t tile_bits;   /* 10..14: tile of 2^tile_bits amplitudes; must equal the plan's */
-  int32_t threads;     /* threads per CTA: 128, 256 or 512 (a preparing warp comes on top) */
+  int32_t threads;     /* threads per CTA: 128, 256 or 512 (a preparing warp comes on top;
+                          128 with 4 CTAs per SM or more and tiles of 2^10 or 2^11: 32 or 64) */
   int32_t ctas_per_sm; /* persistent CTAs per SM, 1..8 (clamped to what fits) */
   int32_t pad;
 } tqk_batch_config; /* 16 bytes; NULL = {14, 512, 1} */

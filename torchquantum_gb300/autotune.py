@@ -119,6 +119,8 @@ def batch_candidates(max_n: int):
     cands = [BatchConfig(14, 512, 1), BatchConfig(14, 256, 1), BatchConfig(13, 256, 3), BatchConfig(13, 256, 1),
              BatchConfig(13, 128, 3), BatchConfig(12, 256, 1), BatchConfig(12, 128, 3), BatchConfig(11, 512, 1),
              BatchConfig(11, 128, 3)]
+    if max_n <= 11:  # many small circuits: as many CTAs as an SM takes (1500 of 8 qubits: 188 us, 389 with three)
+        cands += [BatchConfig(11, 128, 8), BatchConfig(10, 128, 8)]
     # a tile wider than every circuit only wastes shared memory
     narrow = [c for c in cands if c.tile_bits <= max(max_n, 11)]
     return narrow or cands[-1:]
@@ -128,7 +130,7 @@ def tune_batch(cb, dev: torch.device, return_states: bool = False):
     """Best ``BatchConfig`` for ``cb`` on ``dev`` (measured, cached)."""
     from .batch import BatchConfig
 
-    key = f"batch|{gpu_key(dev)}|{','.join(map(str, cb.signature()))}|{int(return_states)}|sweeps"
+    key = f"batch|{gpu_key(dev)}|{','.join(map(str, cb.signature()))}|{int(return_states)}|sweeps2"
     hit = lookup(key)
     if hit is not None:
         return BatchConfig(**hit["config"])

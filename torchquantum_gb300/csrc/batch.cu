@@ -753,8 +753,12 @@ extern "C" int tqk_batch_run(const tqk_batch_circuit* circuits, int ncirc, const
     case 256:
       return cfg.ctas_per_sm >= 2 ? launch_batch<256, 3, 4>(TQK_BATCH_ARGS) : launch_batch<256, 1, 5>(TQK_BATCH_ARGS);
     case 128:
-      return cfg.ctas_per_sm >= 4 && cfg.tile_bits <= 11 ? launch_batch<128, 6, 4>(TQK_BATCH_ARGS)
-                                                         : launch_batch<128, 3, 5>(TQK_BATCH_ARGS);
+      // many CTAs of small tiles: a tile of 2^9 amplitudes is 32 threads' worth, and more threads a CTA only
+      // keep CTAs off the SM (us, 128 threads of 32 amplitudes and 3 CTAs / of 16 and 6 / these 8: 2000
+      // circuits of 5 qubits 184 / 137 / 106; 1000 of 10 378 / - / 215)
+      if (cfg.ctas_per_sm >= 4 && cfg.tile_bits == 10) return launch_batch<32, 8, 4>(TQK_BATCH_ARGS);
+      if (cfg.ctas_per_sm >= 4 && cfg.tile_bits == 11) return launch_batch<64, 8, 4>(TQK_BATCH_ARGS);
+      return launch_batch<128, 3, 5>(TQK_BATCH_ARGS);
     default:
       return fail(TQK_BAD_SHAPE, "%s: threads %d (128, 256 or 512)", what, cfg.threads);
   }
