@@ -7,7 +7,7 @@
 //   k_tile_sums  one warp per tile of 2^tb amplitudes: the tile's probability (float64);
 //   k_tile_scan  one block per row: inclusive prefix sums of the tile probabilities;
 //   k_draw       one warp per (row, shot): search over the tile prefixes, then the running
-//                sum over the chosen tile's amplitudes;
+//                sum over the chosen tile's amplitudes (rows of less than a tile: k_draw_row);
 //   k_parity     one block per (row, string): the share of even minus odd parities of the
 //                outcomes on a string's sites.
 // Uniforms come from the caller (a seeded torch generator), so draws are reproducible.
@@ -115,19 +115,6 @@ __device__ __noinline__ int draw_in_tile(const float2* src, double before, doubl
   return __reduce_max_sync(0xffffffffu, some);  // rounding left target at the tile's end: the last one not zero
 }
 
-// The same in a row of fewer amplitudes.
-__device__ __noinline__ int draw_in_row(const float2* src, int count, double before, double target) {
-  double acc = before;
-  int last_nonzero = 0;
-  for (int j = 0; j < count; ++j) {
-    const double p = prob(src[j]);
-    if (p > 0.0) last_nonzero = j;
-    acc += p;
-    if (acc > target) return j;
-  }
-  return last_nonzero;
-}
-
 // The outcome from sums in R (a lane's 8 neighbouring amplitudes, then the warp's), or -1 where
 // the target t (from the tile's start) is not farther than the margin from both of the
 // outcome's ends.  float32: at most 16 roundings of sums up to the tile's and t's own; `walk`
@@ -193,18 +180,57 @@ __global__ void __launch_bounds__(256) k_draw(const float2* state, int n, int tb
     }
     const double before = lo > 0 ? pre[lo - 1] : 0.0;
     const float2* src = state + (b << n) + (lo << tb);
-    int pick = -1;
-    if (tb == kTileBits) {
-      float4 v[4];
+    float4 v[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = ld4(src + 8 * lane + 2 * k);
-      const double t = target - before, walk = 1e-12 * total;
-      pick = sure_draw<float>(v, static_cast<float>(t), static_cast<float>(walk));
-      if (pick < 0) pick = sure_draw<double>(v, t, walk);
-    }
-    if (pick < 0)
-      pick = tb == kTileBits ? draw_in_tile(src, before, target) : draw_in_row(src, 1 << tb, before, target);
+    for (int k = 0; k < 4; ++k) v[k] = ld4(src + 8 * lane + 2 * k);
+    const double t = target - before, walk = 1e-12 * total;
+    int pick = sure_draw<float>(v, static_cast<float>(t), static_cast<float>(walk));
+    if (pick < 0) pick = sure_draw<double>(v, t, walk);
+    if (pick < 0) pick = draw_in_tile(src, before, target);
     if (lane == 0) out[b * shots + s] = (lo << tb) + pick;
+  }
+}
+
+// Rows of less than a tile: a block walks its row once, amplitude by amplitude in float64, and its
+// threads search the running sums, a shot each (the sums do not decrease, so the first that
+// exceeds the target is the walk's stop; where they end in NaN the walk itself decides).
+// What bounds it: the walk's chain of additions, paid once a block.  6 qubits, 32 rows, 65536
+// shots: 1722 us with a walk a thread, 28212 with a warp per shot, which leaves 31 lanes without
+// work, 66 here.
+__global__ void __launch_bounds__(256) k_draw_row(const float2* state, int n, const double* total_of,
+                                                  const double* uniforms, int64_t shots, int64_t* out) {
+  __shared__ double p[1 << (kTileBits - 1)], sum[1 << (kTileBits - 1)];
+  __shared__ int last_nonzero;
+  const int64_t b = blockIdx.y;
+  const int count = 1 << n, tid = threadIdx.x;
+  if (tid < count) p[tid] = prob(state[(b << n) + tid]);
+  __syncthreads();
+  if (tid == 0) {
+    double acc = 0.0;
+    int last = 0;
+    for (int j = 0; j < count; ++j) {
+      if (p[j] > 0.0) last = j;
+      acc += p[j];
+      sum[j] = acc;
+    }
+    last_nonzero = last;
+  }
+  __syncthreads();
+  const double total = total_of[b];
+  const bool whole = sum[count - 1] == sum[count - 1];
+  for (int64_t s = (int64_t)blockIdx.x * 256 + tid; s < shots; s += (int64_t)gridDim.x * 256) {
+    const double target = uniforms[b * shots + s] * total;
+    int lo = 0, hi = count;
+    if (whole) {
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sum[mid] > target) hi = mid;
+        else lo = mid + 1;
+      }
+    } else {
+      while (lo < count && !(sum[lo] > target)) ++lo;
+    }
+    out[b * shots + s] = lo < count ? lo : last_nonzero;  // rounding left target at the end: the last one not zero
   }
 }
 
@@ -261,6 +287,13 @@ extern "C" int tqk_sample(const void* state, int64_t bsz, int n, const double* u
   cudaStream_t s = as_stream(stream);
   sample::k_tile_sums<<<dim3((unsigned)((ntiles + 7) / 8), (unsigned)bsz), 256, 0, s>>>(st, n, tb, ntiles, pre);
   sample::k_tile_scan<<<(unsigned)bsz, 1024, 0, s>>>(pre, ntiles);
+  if (tb < sample::kTileBits) {
+    int64_t blocks = (shots + 255) / 256, most = 8 * 152 / bsz;  // several shots a thread once the GPU is full
+    if (most < 1) most = 1;
+    if (blocks > most) blocks = most;
+    sample::k_draw_row<<<dim3((unsigned)blocks, (unsigned)bsz), 256, 0, s>>>(st, n, pre, uniforms, shots, out);
+    return launch_status(what);
+  }
   const int64_t blocks = (shots + sample::kDrawWarps - 1) / sample::kDrawWarps;
   sample::k_draw<<<dim3((unsigned)(blocks < (1 << 20) ? blocks : (1 << 20)), (unsigned)bsz),
                    32 * sample::kDrawWarps, 0, s>>>(st, n, tb, ntiles, pre,
