@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(256) k_dense_adj(const DenseParams<D> p) {
 }
 
 // ------------------------------------------------------------------ dense k, 7 wires and more
-// (3 to 6 wires: dense_tile.cu, but for small reverse steps, see dense_entry.)  One block stages
+// (3 to 6 wires: dense_tile.cu, but for small states, see output_by_output.)  One block stages
 // gpb groups (2^k amplitudes each) in shared memory, applies the matrix and writes back.  Thread
 // idx maps to (group gi = idx % gpb, row r = idx / gpb), so a warp shares its matrix row.
 struct DenseKParams {
@@ -320,6 +320,7 @@ struct DenseKParams {
   double* grad;                     // adjoint: [batch][D][D] complex128 or null
   int64_t grad_stride;
   int gpb;                          // groups per block
+  int mat_in_smem;
 };
 
 __device__ __forceinline__ uint64_t dk_offset(const DenseKParams& p, int r) {
@@ -331,7 +332,7 @@ __device__ __forceinline__ uint64_t dk_offset(const DenseKParams& p, int r) {
 
 constexpr int kDkMaxOut = 16;
 
-// smem: [tile gpb*(D+1)] (tile rows padded by one amplitude)
+// smem: [mat D*D if staged][tile gpb*(D+1)] (tile rows padded by one amplitude)
 __global__ void __launch_bounds__(256) k_dense_k(const DenseKParams p) {
   extern __shared__ float2 sm[];
   const int D = 1 << p.k;
@@ -339,8 +340,11 @@ __global__ void __launch_bounds__(256) k_dense_k(const DenseKParams p) {
   const int64_t b = blockIdx.y;
   const int64_t gbase = (int64_t)blockIdx.x * p.gpb;
   float2* row = p.state + (b << p.n);
-  const float2* M = p.mat + b * p.mat_stride;
-  float2* tile = sm;
+  const float2* Mg = p.mat + b * p.mat_stride;
+  float2* tile = sm + (p.mat_in_smem ? D * D : 0);
+  if (p.mat_in_smem)
+    for (int i = threadIdx.x; i < D * D; i += blockDim.x) sm[i] = Mg[i];
+  const float2* M = p.mat_in_smem ? sm : Mg;
   const int total = p.gpb * D;
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
     const int gi = idx % p.gpb, r = idx / p.gpb;
@@ -868,7 +872,8 @@ int launch_dense_k(const GateSetup& s, float2* state, float2* lam, const float2*
   if (gpb > p.groups) gpb = (int)p.groups;
   p.gpb = gpb;
   const size_t tile = (size_t)gpb * (D + 1) * sizeof(float2);
-  const size_t smem = adjoint ? 2 * tile : tile;
+  p.mat_in_smem = !adjoint && s.kt <= 5;  // (of 6 wires: 32 KB a block, 10.5 us against 8.4 at 2^12 amplitudes)
+  const size_t smem = adjoint ? 2 * tile : tile + (p.mat_in_smem ? (size_t)D * D * sizeof(float2) : 0);
   if (smem > 200 * 1024) return fail(TQK_TOO_MANY_QUBITS, "dense gate: k=%d too wide", s.kt);
   static bool attr_set = false;
   if (!attr_set) {
@@ -898,6 +903,20 @@ int setup_targets(GateSetup& s, int n, int64_t bsz, const int32_t* targets, int 
   return TQK_OK;
 }
 
+// Gates on 3 to 6 wires that k_dense_k takes (in place; k wires, 2^c groups of 2^k amplitudes a row, amps in
+// all): small states, whose few tiles leave most SMs without work, and rows of a few groups, whose tiles
+// have fewer columns than a thread's 4 x 4 block.  Measured, us, k_dense_k / tiles: forward n = 8, 2^12
+// amplitudes, k = 4 / 5 / 6 6.3 / 6.3 / 8.4 against 6.6 / 8.6 / 14.8, but n = 12, k = 5 / 6 12.5 / 27 against 8.6 /
+// 15 and at 2^18 amplitudes 15 / 27 against 11 / 21; reverse without a cotangent n = 6, k = 6 8.5 against 20 at
+// 2^12, 205 against 652 at 2^21; with a cotangent k = 3, 4, 5 at 2^16 12 to 21 against 16 to 27, k = 6 n = 8
+// 19 against 37 at 2^15, 39 against 62 the other way at n = 18 and 2^19.
+bool output_by_output(int k, int c, int64_t amps, bool adjoint, bool grad) {
+  if (!adjoint) return amps <= (1ll << 15) && (k == 3 || c <= 3);
+  if (!grad) return c <= 2 || (amps <= (1ll << 16) && (k == 3 || c <= 3 || k + c <= 8));
+  if (k == 6) return c <= 4 && amps <= (c < 2 ? 1ll << 16 : 1ll << 18);
+  return amps <= (1ll << 18) || (k == 5 && c <= 3);
+}
+
 int dense_entry(void* state, void* lam, int64_t bsz, int n, const int32_t* controls, int nc,
                 const int32_t* targets, int kt, const void* mat, int64_t mat_batch, const void* uinv,
                 double* grad, bool adjoint, void* stream, const char* what) {
@@ -917,11 +936,8 @@ int dense_entry(void* state, void* lam, int64_t bsz, int n, const int32_t* contr
   if (kt == 1) return launch_dense<2>(s, ps, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
   if (kt == 2) return launch_dense<4>(s, ps, ps, pl, pm, mat_batch, pi, grad, adjoint, st);
   if (nc > 0) return fail(TQK_UNSUPPORTED, "%s: controlled gates take 1 or 2 targets", what);
-  // 3 to 6 wires: tiles (dense_tile.cu), but for a reverse step with a cotangent on a small
-  // state, which fits a few CTAs: k = 3, 4, 5 at 2^15 / 2^16 amplitudes took 10-11, 12-14 and
-  // 22-23 us op by op, 16, 20 and 27 us in tiles; at 2^21 it is 138, 142, 111 against 39, 55, 77.
-  const bool small_reverse = adjoint && grad != nullptr && kt <= 5 && (bsz << n) <= (1ll << 18);
-  if (kt >= kTileMinWires && kt <= kTileMaxWires && !small_reverse) {
+  // 3 to 6 wires: tiles (dense_tile.cu), but for small states
+  if (kt >= kTileMinWires && kt <= kTileMaxWires && !output_by_output(kt, n - kt, bsz << n, adjoint, grad != nullptr)) {
     DenseTileArgs a{ps, ps, pl, pl, bsz, n, kt, s.tb, pm, pi, mat_batch, grad, false};
     return adjoint ? launch_dense_tile_adj(a, st) : launch_dense_tile(a, st);
   }
