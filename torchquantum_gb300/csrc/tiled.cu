@@ -99,9 +99,13 @@ struct Params {
   const float2* psi_in;   // .. and loaded from here (in place: the same)
   const float2* lam_in;
   int n, m;               // qubits; tile bits
-  int64_t tiles;          // tiles per row
+  int tiles_log;          // tiles per row: 2^tiles_log
+  int per_row;            // some op has an operand for each row
+  uint32_t items;         // tiles of all rows
+  uint32_t row_ctas;      // CTAs of each row, or 0: an even share of the items each
   uint64_t outer;         // index bits outside the tile
   int nsweeps, nops, ngrad;
+  uint8_t grad_op[TQK_STAGED_MAX_OPS];  // op of each accumulator
   uint8_t tb[kMaxBits];   // index bit of tile-local bit j (ascending)
   int64_t ioff[kAmps / 2];  // offset within the tile of copy piece group i
   Sweep sweeps[TQK_STAGED_MAX_OPS];
@@ -120,6 +124,27 @@ __device__ __forceinline__ uint64_t deposit(uint64_t t, uint64_t mask) {
   return r;
 }
 
+// Work: the tiles of all rows.  With operands that all rows share the CTAs take them in turn.  Else a
+// CTA should work out its tables for few rows: while whole CTAs a row leave at most a sixteenth of the
+// places empty, each row's CTAs take its tiles in turn; at more rows a CTA gets an even share of
+// neighbouring tiles.  (Whole CTAs a row at any number of rows: 14 wires, 305 rows, two U3 22 us forward
+// and 63 in reverse, now 18 and 52; shares at any number: 40 gates at 22 wires and 8 rows 2477 us a
+// step, 2453 so.)
+struct Items {
+  uint32_t it, end, step;
+};
+__device__ __forceinline__ Items items_of(const Params& p) {
+  const uint32_t c = blockIdx.x;
+  if (!p.per_row) return {c, p.items, gridDim.x};
+  if (p.row_ctas > 0) {
+    const uint32_t row = c / p.row_ctas;
+    return {(row << p.tiles_log) + c % p.row_ctas, (row + 1) << p.tiles_log, p.row_ctas};
+  }
+  const uint64_t n = p.items;
+  return {static_cast<uint32_t>(n * c / gridDim.x), static_cast<uint32_t>(n * (c + 1) / gridDim.x), 1u};
+}
+__device__ __forceinline__ uint32_t tile_of(const Params& p, uint32_t it) { return it & ((1u << p.tiles_log) - 1u); }
+
 // A thread's part of the tile copies, worked out anew for each copy: held across the op
 // loop its addresses would take registers from the amplitudes.
 struct Frame {
@@ -127,11 +152,11 @@ struct Frame {
   uint32_t lphys;  // its offset in the tile
 };
 
-__device__ __forceinline__ Frame frame(const Params& p, uint64_t base) {
+__device__ __forceinline__ Frame frame(const Params& p, uint32_t row, uint64_t base) {
   uint32_t l = threadIdx.x << 1;
   asm volatile("" : "+r"(l));  // not a loop invariant to the compiler
   Frame f;
-  f.off = (static_cast<int64_t>(blockIdx.y) << p.n) + static_cast<int64_t>(base);
+  f.off = (static_cast<int64_t>(row) << p.n) + static_cast<int64_t>(base);
   for (int j = 1; j < p.m; ++j)
     if ((l >> j) & 1u) f.off += 1ll << p.tb[j];
   f.lphys = swz(l);
@@ -186,11 +211,10 @@ struct Decoded {
   uint64_t omask, oval;
 };
 
-// Decoded ops and their factors for the CTA's row: fac[op][entry] = (re, re, im, -), of U
+// Decoded ops and their factors for a row: fac[op][entry] = (re, re, im, -), of U
 // or (ADJ) of U^H.
 template <bool ADJ>
-__device__ __forceinline__ void build_ops(const Params& p, float4* fac, Decoded* dec) {
-  const int64_t row = blockIdx.y;
+__device__ __forceinline__ void build_ops(const Params& p, int64_t row, float4* fac, Decoded* dec) {
   for (int j = threadIdx.x; j < p.nops; j += blockDim.x) {
     const SOp& o = p.ops[j];
     int go = o.go;
@@ -330,11 +354,14 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_tiled(const __grid_constant_
   Decoded* dec = reinterpret_cast<Decoded*>(fac + p.nops * 4);
   uint32_t* tab = reinterpret_cast<uint32_t*>(dec + p.nops);
   build_tables(p, tab);
-  build_ops<false>(p, fac, dec);
   const Source src{p, fac};
-  for (int64_t t = blockIdx.x; t < p.tiles; t += gridDim.x) {
-    const uint64_t base = deposit(static_cast<uint64_t>(t), p.outer);
-    load_tile(p, frame(p, base), p.psi_in, tile);
+  bool fresh = true;
+  for (Items w = items_of(p); w.it < w.end; w.it += w.step) {
+    const uint32_t row = w.it >> p.tiles_log;
+    const uint64_t base = deposit(tile_of(p, w.it), p.outer);
+    if (fresh) build_ops<false>(p, row, fac, dec);
+    fresh = p.per_row && (w.it + w.step) >> p.tiles_log != row;
+    load_tile(p, frame(p, row, base), p.psi_in, tile);
     wait_loads();  // also orders the tables
 #pragma unroll 1
     for (int s = 0; s < p.nsweeps; ++s) {
@@ -351,7 +378,7 @@ __global__ void __launch_bounds__(kMaxThreads, 3) k_tiled(const __grid_constant_
       store_regs<f2::Psi>(sw.rphys, tile, thread_offset(tab, s) >> 16);
       __syncthreads();
     }
-    store_tile(p, frame(p, base), p.psi, tile);
+    store_tile(p, frame(p, row, base), p.psi, tile);
     __syncthreads();
   }
 }
@@ -497,13 +524,16 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
   Decoded* dec = reinterpret_cast<Decoded*>(gtile + 2 * nacc * warps);
   uint32_t* tab = reinterpret_cast<uint32_t*>(dec + p.nops);
   build_tables(p, tab);
-  build_ops<true>(p, fac, dec);
   for (int i = threadIdx.x; i < nacc; i += blockDim.x) gacc[i] = make_float2(0.f, 0.f);
   const Source src{p, fac};
-  for (int64_t t = blockIdx.x; t < p.tiles; t += gridDim.x) {
-    const uint64_t base = deposit(static_cast<uint64_t>(t), p.outer);
+  bool fresh = true;
+  for (Items w = items_of(p); w.it < w.end; w.it += w.step) {
+    const uint32_t row = w.it >> p.tiles_log;
+    const uint64_t base = deposit(tile_of(p, w.it), p.outer);
+    if (fresh) build_ops<true>(p, row, fac, dec);
+    fresh = p.per_row && (w.it + w.step) >> p.tiles_log != row;  // the next item is another row's
     {
-      const Frame f = frame(p, base);
+      const Frame f = frame(p, row, base);
       load_tile(p, f, p.psi_in, ps);
       load_tile(p, f, p.lam_in, ls);
     }
@@ -550,7 +580,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
       __syncthreads();
     }
     {
-      const Frame f = frame(p, base);
+      const Frame f = frame(p, row, base);
       store_tile(p, f, p.psi, ps);
       store_tile(p, f, p.lam, ls);
     }
@@ -562,18 +592,14 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tiled_adj(const __grid_const
         g.x = two_sum(g.x, gw[0], e);
         g.y += gw[8] + e;
       }
+      if (fresh || w.it + w.step >= w.end) {  // the sums so far, one atomic per value
+        const SOp& o = p.ops[p.grad_op[i >> 3]];
+        if ((i & 7) < 2 * o.nent) atomicAdd(o.grad + row * o.grad_stride + (i & 7), pair_value(g.x, g.y));
+        g = make_float2(0.f, 0.f);
+      }
       gacc[i] = g;
     }
     __syncthreads();
-  }
-  // one atomic per value per op with a cotangent slot
-  for (int i = threadIdx.x; i < p.nops * 8; i += blockDim.x) {
-    const SOp& o = p.ops[i >> 3];
-    const int v = i & 7;
-    if (o.gidx >= 0 && v < 2 * o.nent) {
-      const float2 g = gacc[o.gidx * 8 + v];
-      atomicAdd(o.grad + blockIdx.y * o.grad_stride + v, pair_value(g.x, g.y));
-    }
   }
 }
 
@@ -639,7 +665,9 @@ int fill_tiled(tiled::Params& p, int64_t bsz, int n, const tqk_staged_op* ops, i
   p.n = n;
   p.m = m;
   p.nops = nops;
-  p.tiles = 1ll << (n - m);
+  p.tiles_log = n - m;
+  p.items = static_cast<uint32_t>(bsz << (n - m));
+  p.per_row = 0;
   p.outer = ((1ull << n) - 1ull) & ~tile_mask;
   int local[64];  // tile-local bit of an index bit, or -1
   for (int b = 0, j = 0; b < 64; ++b) {
@@ -712,8 +740,10 @@ int fill_tiled(tiled::Params& p, int64_t bsz, int n, const tqk_staged_op* ops, i
       o = tiled::SOp{};
       o.operand = static_cast<const float2*>(src.operand);
       o.grad = adjoint && src.kind != TQK_S_X ? src.grad : nullptr;
-      o.gidx = o.grad ? p.ngrad++ : -1;
-      const bool per_row = src.batch > 1;
+      o.gidx = o.grad ? p.ngrad : -1;
+      if (o.grad) p.grad_op[p.ngrad++] = static_cast<uint8_t>(i);
+      const bool per_row = src.batch > 1 && src.kind != TQK_S_X;
+      p.per_row |= per_row;
       const bool targeted = src.kind == TQK_S_DENSE1 || src.kind == TQK_S_X;
       for (int w = 0; w < 2; ++w) o.dslot[w] = o.dbit[w] = o.obit[w] = -1;
       if (src.kind == TQK_S_DIAG) {
@@ -809,12 +839,12 @@ int tiled_entry(const void* psi_in, const void* lam_in, void* psi, void* lam, in
   }
   int fit = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, smem) != cudaSuccess || fit < 1) fit = 1;
-  // CTAs that fill the GPU once, rounded down so that all are resident: each builds its
-  // tables once and loops over tiles of its row
-  int64_t gx = static_cast<int64_t>(sms) * fit / bsz;
-  if (gx > p.tiles) gx = p.tiles;
-  if (gx < 1) gx = 1;
-  kern<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(bsz), 1), threads, smem, as_stream(stream)>>>(p);
+  const uint32_t slots = static_cast<uint32_t>(sms) * fit;  // CTAs that fill the GPU once
+  uint32_t grid = slots < p.items ? slots : p.items;
+  p.row_ctas = grid / static_cast<uint32_t>(bsz);
+  if (grid - p.row_ctas * static_cast<uint32_t>(bsz) > grid / 16) p.row_ctas = 0;
+  if (p.per_row && p.row_ctas > 0) grid = p.row_ctas * static_cast<uint32_t>(bsz);
+  kern<<<grid, threads, smem, as_stream(stream)>>>(p);
   return launch_status(what);
 }
 
