@@ -30,18 +30,15 @@ def _walk(ops, n, small):
                     continue
             blocked |= wires or (1 << n) - 1
             rest.append(i)
-        if not take:
+        if len(take) < 2 or not (small or sum(P._pass_share(ops[i]) for i in take) >= P.TILE_MIN_SHARE):
             out.append(([pending[0]], 0))
             pending = pending[1:]
             continue
-        if len(take) < 2 or not (small or sum(P._pass_share(ops[i]) for i in take) >= 1.0):
-            out.extend(([i], 0) for i in take)
-        else:
-            for b in range(n):
-                if free and not (mask >> b) & 1:
-                    mask |= 1 << b
-                    free -= 1
-            out.append((take, mask))
+        for b in range(n):
+            if free and not (mask >> b) & 1:
+                mask |= 1 << b
+                free -= 1
+        out.append((take, mask))
         pending = rest
     return out
 
@@ -94,3 +91,16 @@ def test_time_grows_with_the_ops(kinds, tail):
         return min(runs)
 
     assert best(8000) <= 8 * best(2000)  # four times the ops; the walk takes sixteen times as long
+
+
+def test_light_ops_wait_for_company():
+    one = torch.eye(2, dtype=torch.complex64)[None]
+    u3 = lambda w: engine.TapeOp("dense", [w], operand=one)  # noqa: E731
+    swap = lambda a, b: engine.TapeOp("swap", [a, b], targets=[a, b])  # noqa: E731
+    crx = lambda c, t: engine.TapeOp("ctrl", [c, t], controls=[c], targets=[t], operand=one)  # noqa: E731
+    # two half passes gain nothing ..
+    assert [m for _, m in P.plan_tiles([crx(0, 1), crx(2, 3)], 20, False)] == [0, 0]
+    assert [len(i) for i, _ in P.plan_tiles([crx(0, 1), crx(2, 3), crx(4, 5)], 20, False)] == [3]
+    # .. and an op that comes free alone waits for the next
+    plan = P.plan_tiles([swap(0, 1), swap(2, 3), u3(0), u3(2)], 20, False)
+    assert [i for i, _ in plan] == [[0], [1], [2, 3]] and [bool(m) for _, m in plan] == [False, False, True]

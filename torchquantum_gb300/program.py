@@ -783,10 +783,17 @@ def stage_runs(ops, n: int, min_run: int = 2):
     return out
 
 
-# A tile pass moves the state once (2 S bytes forward, 4 S in reverse).  On a state larger
-# than this its ops must together cost at least that on their own kernels to share a pass;
-# a smaller state stays in L2, where launches cost more than bytes.
-TILE_L2_BYTES = 32 << 20
+# A tile pass moves the state once (2 S bytes forward, 4 S in reverse) whatever its ops are; an op on its
+# own kernel moves its share of that.  Ops share a pass when their shares add up to more than the pass
+# costs: TILE_MIN_SHARE, or TILE_L2_SHARE on states that stay in L2, where a pass is bound by its
+# instructions (us forward + reverse, tile pass / own kernels: 268 MB two CRX 377 / 314, three 416 / 440, U3
+# and CNOT 350 / 365; 32 MB three CRX 66 / 58, four 73 / 85, U3 and CNOT 53 / 49).  States up to
+# TILE_SMALL_BYTES always share: launches cost more than bytes there (8 MB: two CRX 18 / 26; 16 MB: two
+# gates with the rest of a step 86 / 106).
+TILE_MIN_SHARE = 1.2
+TILE_L2_SHARE = 1.75
+TILE_L2_BYTES = 64 << 20
+TILE_SMALL_BYTES = 16 << 20
 # Where a step is bound by the host (35 us a gate, forward and backward), the kernels of one gate
 # and the staged runs stay, whose order of operations results are known by.  Rows of at most 2^12
 # amplitudes are one tile either way: up to 2^21 amplitudes in all (n = 10, bsz = 256, 100 gates:
@@ -807,13 +814,15 @@ def _pass_share(op) -> float:
     return 1.0
 
 
-def plan_tiles(ops, n: int, small: bool) -> List[tuple]:
+def plan_tiles(ops, n: int, small: bool, share: float = TILE_MIN_SHARE) -> List[tuple]:
     """Cut the ops into passes: (op indices, tile mask), mask 0 for an op on its own kernel.
 
     A pass starts from the lowest four index bits (whole 128-byte lines) and walks the
     pending ops in order: an op joins when no wire of it was touched by an op left out and
     its target (if any) is or fits among the tile's bits; ops on disjoint wires commute, so
-    the passes apply an equivalent order.  Free bits are filled from the lowest.
+    the passes apply an equivalent order.  Free bits are filled from the lowest.  Unless
+    ``small``, the ops of a pass move the state ``share`` times at least on their own kernels; where
+    they would not, the first pending op runs on its own and the others wait.
 
     The ops of a wire leave in order, so each wire has a queue, and a pass looks at the queues'
     fronts only: every op left out closes a wire for the pass, which takes at most
@@ -840,7 +849,7 @@ def plan_tiles(ops, n: int, small: bool) -> List[tuple]:
         mask, free, blocked, take = 15, tb - 4, 0, []
         heap = [q[f] for q, f in zip(queues, front) if f < len(q)]
         heapq.heapify(heap)
-        first, last = heap[0], -1
+        first, last, fronts = heap[0], -1, list(front)
         while heap and len(take) < _lib.STAGED_MAX_OPS:
             i = heapq.heappop(heap)
             if i == last:  # at the front of another wire's queue too
@@ -861,20 +870,18 @@ def plan_tiles(ops, n: int, small: bool) -> List[tuple]:
                         heapq.heappush(heap, j)
                     continue
             blocked |= wires
-        if not take:  # the first op is not one a tile pass can hold
-            out.append(([first], 0))
+        if len(take) < 2 or not (small or sum(_pass_share(ops[i]) for i in take) >= share):
+            front = fronts  # the others may join ops that are not free yet
             leave(first)
+            out.append(([first], 0))
             left -= 1
             continue
         left -= len(take)
-        if len(take) < 2 or not (small or sum(_pass_share(ops[i]) for i in take) >= 1.0):
-            out.extend(([i], 0) for i in take)
-        else:
-            for b in range(n):
-                if free and not (mask >> b) & 1:
-                    mask |= 1 << b
-                    free -= 1
-            out.append((take, mask))
+        for b in range(n):
+            if free and not (mask >> b) & 1:
+                mask |= 1 << b
+                free -= 1
+        out.append((take, mask))
     return out
 
 
@@ -885,13 +892,14 @@ def tile_runs(ops, n: int, bsz: int):
     if n < _lib.TILED_MIN_WIRES or \
             (bsz << n) < (TILE_SHORT_ROW_AMPS if n <= _lib.STAGED_MAX_TILE_BITS else TILE_MIN_AMPS):
         return stage_runs(ops, n)
-    small = (bsz << (n + 3)) <= TILE_L2_BYTES
-    key = (n, small, tuple((op.kind, tuple(op.wires), len(op.controls), stageable(op, n, n)) for op in ops))
+    small = (bsz << (n + 3)) <= TILE_SMALL_BYTES
+    share = TILE_L2_SHARE if (bsz << (n + 3)) <= TILE_L2_BYTES else TILE_MIN_SHARE
+    key = (n, small, share, tuple((op.kind, tuple(op.wires), len(op.controls), stageable(op, n, n)) for op in ops))
     plan = _TILE_PLANS.get(key)
     if plan is None:
         if len(_TILE_PLANS) > 256:
             _TILE_PLANS.clear()
-        plan = plan_tiles(ops, n, small)
+        plan = plan_tiles(ops, n, small, share)
         _TILE_PLANS[key] = plan
     return [StagedRun([ops[i] for i in idx], mask) if mask else ops[idx[0]] for idx, mask in plan]
 
