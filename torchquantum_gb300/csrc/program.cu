@@ -332,6 +332,8 @@ __device__ __forceinline__ bool op_ok(const tqk_block_op& op, int k) {
 }
 
 constexpr int kChunk = 32;  // ops read at a time
+constexpr int kBuildPlaces = 152;
+constexpr int kBuildEntryBits = 9;  // entries of a block that a CTA of the build holds
 
 struct ShOp {
   const double2* opnd;
@@ -570,6 +572,16 @@ __device__ void build_op(C2* U, const Part& p, const ShOp& op, const C2* m) {
   }
 }
 
+// Column bits that the CTAs of a block share out: all that are offered while the blocks (and rows of those
+// with a batch) are fewer than the SMs; beyond, a CTA keeps as many columns as its shared memory holds (2^9
+// entries), since the reading and ordering of the ops is paid in each CTA.  (Always 8 CTAs a block: 100 blocks
+// of 64 rows, 6 ops, k = 3 / 4 / 5 / 6 847 / 844 / 870 / 1023 us, so 132 / 140 / 286 / 1008; one CTA of 256 threads and
+// all columns, whatever the width: 321 / 349 / 778 / 3000.)
+__device__ __forceinline__ int columns_shared(const tqk_block_desc& bl) {
+  const int64_t ctas = static_cast<int64_t>(gridDim.x) * (bl.batch > 1 ? bl.batch : 1);
+  return ctas < kBuildPlaces ? bl.k : max(0, bl.k - min(4, kBuildEntryBits - bl.k));
+}
+
 __global__ void k_block_build(const tqk_block_desc* blocks, const tqk_block_op* ops, int split) {
   extern __shared__ double2 smem_u[];
   __shared__ Stage<C2> sh;
@@ -578,7 +590,7 @@ __global__ void k_block_build(const tqk_block_desc* blocks, const tqk_block_op* 
   const int64_t b = blockIdx.y;
   const int z = blockIdx.z;
   if (b >= bl.batch || !block_ok(bl)) return;
-  split = min(split, bl.k);
+  split = min(split, columns_shared(bl));
   if (z >> split) return;
   const int tid = threadIdx.x, nth = blockDim.x, whole = bl.k - split;  // bits with all columns
   Part p{1 << whole, 0, 0};
@@ -881,7 +893,8 @@ extern "C" int tqk_param_grads(const tqk_gate_desc* gates, int ngates, void* str
 // split; reverse 147 + 156 against 152 + 206).  The reverse sums at most 8
 // float32 terms a thread (64 rows x 16 columns over 64 threads, one target).  Idle CTAs (rows
 // of a block without a batch, narrow blocks) leave at once.
-constexpr int kBuildSplit = 3, kBuildThreads = 128;
+constexpr int kBuildSplit = 3, kBuildThreads = 128;  // (6-wire blocks: 2^12 entries)
+static_assert(12 - kBuildSplit == prog::kBuildEntryBits, "a CTA's share of a 6-wire block");
 constexpr int kUnbuildSplit = 2, kUnbuildThreads = 64;
 
 extern "C" int tqk_block_build(const tqk_block_desc* blocks, int nblocks, int max_batch, const tqk_block_op* ops,
@@ -889,7 +902,7 @@ extern "C" int tqk_block_build(const tqk_block_desc* blocks, int nblocks, int ma
   if (nblocks <= 0) return TQK_OK;
   if (!blocks || !ops) return fail(TQK_BAD_POINTER, "tqk_block_build: null pointer");
   if (max_batch < 1 || max_batch > 65535) return fail(TQK_BAD_SHAPE, "tqk_block_build: batch %d", max_batch);
-  const size_t smem = (64 * 64 >> kBuildSplit) * sizeof(double2);
+  const size_t smem = sizeof(double2) << prog::kBuildEntryBits;
   dim3 grid(nblocks, max_batch, 1 << kBuildSplit);
   prog::k_block_build<<<grid, kBuildThreads, smem, as_stream(stream)>>>(blocks, ops, kBuildSplit);
   return launch_status("tqk_block_build");
