@@ -163,7 +163,7 @@ def pass_costs(n: int, bsz: int, dev: torch.device, tc_ok: bool) -> dict:
     ``tc_ok``; adj_stored: the reverse step that reads the block's stored input).  Probes
     use min(bsz, rows that fit 2^27 amplitudes) rows and are scaled to bsz (the kernels
     stream rows independently)."""
-    key = f"fusion3|{gpu_key(dev)}|n{n}|b{bsz}|tc{int(tc_ok)}|tiles"
+    key = f"fusion3|{gpu_key(dev)}|n{n}|b{bsz}|tc{int(tc_ok)}|tiles2"
     hit = lookup(key)
     if hit is not None:
         return hit
