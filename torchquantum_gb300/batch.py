@@ -41,7 +41,8 @@ _X = np.array([[0, 1], [1, 0]], dtype=np.complex128)
 class BatchConfig:
     """Launch shape of a circuit batch: shared-memory tile of 2^tile_bits amplitudes
     (circuits with n <= tile_bits run in one tile), threads per CTA (a warp that prepares
-    their work comes on top) and persistent CTAs per SM.  Chosen by ``autotune.tune_batch`` or given explicitly."""
+    their work comes on top; 128 become 32 or 64 with tiles of 2^10 or 2^11 and 4 CTAs per SM or
+    more) and persistent CTAs per SM.  Chosen by ``autotune.tune_batch`` or given explicitly."""
     tile_bits: int = TILE_BITS
     threads: int = 512
     ctas_per_sm: int = 1

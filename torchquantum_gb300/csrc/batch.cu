@@ -62,10 +62,11 @@ constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 // 2^13-amplitude item of 18 such ops takes an SM), the two shared-memory crossings of a sweep
 // (2.5 us) and the latency of 12 warps an SM, all the registers allow.  256 circuits of n = 8..20
 // and 2..40 layers, ms: one op per crossing and barrier 11.4 (13-bit tiles, 3 CTAs of 256);
-// sweeps of 16 amplitudes a thread 8.9 (3 x 256), of 32 8.7 (3 x 128).  96 circuits of up to 13
+// sweeps of 16 amplitudes a thread 8.9 (3 x 256), of 32 8.4 (3 x 128).  96 circuits of up to 13
 // qubits, one tile each: 0.58 before, 0.38 now (256 threads, 32 amplitudes).  A row of fewer
 // amplitudes than a thread holds works in a tile of that many, the rest zero: 119 circuits of 7
-// qubits and 17 layers, 81 us op by op (each op's and matrix's read before it), 73 in sweeps.
+// qubits and 17 layers, launch included, 112 us op by op (each op's and matrix's read before it), 88 in
+// sweeps.
 constexpr int kMaxAmpBits = 5;  // 2^AB amplitudes per thread: AB = 5, or 4 where CTAs are many
 constexpr int kSweepOps = 8;
 
@@ -745,7 +746,7 @@ extern "C" int tqk_batch_run(const tqk_batch_circuit* circuits, int ncirc, const
   cudaStream_t s = as_stream(stream);
 #define TQK_BATCH_ARGS circuits, ncirc, ops, passes, items, n_items, mats, states, write_states, z_out, pass_done, \
                        t_done, counter, status, cfg.tile_bits, cfg.ctas_per_sm, s
-  // 32 amplitudes a thread where the CTAs asked for leave it the registers (8.6 ms against 8.9 with
+  // 32 amplitudes a thread where the CTAs asked for leave it the registers (8.4 ms against 8.9 with
   // 16 for 256 circuits of 8 to 20 qubits), else 16
   switch (cfg.threads) {
     case 512:

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_expval_finish(const double* 
 // waits for the stage.
 // What bounds it: DRAM moves a 64 KB stage in 2800 cycles an SM, the strings' partner reads take
 // 2500 to 4600 of shared memory and about as many issue cycles; they overlap in part.  n = 22,
-// 4 rows, 24 strings: expvals 201 -> 160 us (three groups; 60 at the DRAM rate; 152 with the CTA's sums
+// 4 rows, 24 strings: expvals 201 -> 159 us (three groups; 60 at the DRAM rate; 152 with the CTA's sums
 // in plain float32), seed 369 -> 244 us
 // (158 at the DRAM rate); before, each warp took a segment of the strings' visits (two stage
 // reads, a shift, a population count and a flip each), the seed read the earlier groups' output
