@@ -39,3 +39,14 @@ def test_a_stream_of_no_cuda_device_is_refused_as_by_torch():
 
     with pytest.raises((ValueError, RuntimeError, AssertionError)):
         _lib._stream(torch.zeros(1))
+
+
+def test_coset_groups_given_out_are_the_callers_own():
+    from torchquantum_gb300 import _lib
+
+    masks = [1 << 19, 3, 5, 1 << 7, 1 << 18, 9, 17, 33, 65]
+    groups = _lib.coset_groups(masks, 20)
+    passes = _lib.expval_passes(masks, 20)
+    groups[0][0].clear()
+    groups.pop()
+    assert _lib.expval_passes(masks, 20) == passes and _lib.coset_groups(masks, 20)[0][0]

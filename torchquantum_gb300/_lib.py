@@ -249,7 +249,7 @@ def coset_groups(xmasks, n: int):
     strings in order, a group growing while it holds at most 8 strings and its X-masks'
     parts above the lowest c bits span at most T - c dimensions for c = min(4, T),
     T = min(n, 13).  Returns [(string indices, c, rank)] with the widest such c."""
-    return _coset_groups(tuple(xmasks), n)
+    return [(list(g), c, r) for g, c, r in _coset_groups(tuple(xmasks), n)]  # the memo's own stay as they are
 
 
 @functools.lru_cache(maxsize=256)
@@ -278,7 +278,7 @@ def expval_passes(xmasks, n: int = 64) -> int:
     """Passes tqk_pauli_expval makes: with several X-masks one coset pass per group
     (``coset_groups``); with one X-mask for all strings, one pass per 8 strings."""
     if len(set(xmasks)) > 1:
-        return len(coset_groups(list(xmasks), n))
+        return len(_coset_groups(tuple(xmasks), n))
     return (len(xmasks) + 7) // 8
 
 
@@ -301,7 +301,7 @@ def pauli_apply_sum(state, n, xmasks, zmasks, coef):
     out = torch.empty_like(state)
     _check(load().tqk_pauli_apply_sum(state.data_ptr(), state.shape[0], n, _u64(xmasks), _u64(zmasks), len(xmasks),
                                       coef.data_ptr(), out.data_ptr(), status_word(state.device).data_ptr(),
-                                      _stream(state)), launches=len(coset_groups(list(xmasks), n)))
+                                      _stream(state)), launches=len(_coset_groups(tuple(xmasks), n)))
     return out
 
 
